@@ -73,4 +73,32 @@ int check_gemm_args(int m, int n, int k, const float* alpha, const void* A, int 
 
 inline int div_up(int a, int b) { return (a + b - 1) / b; }
 
+// Launch a kernel that begins with grid_wait() (ptx.cuh), so that its CTAs may
+// be placed as soon as those of its predecessor in the stream have ended:
+// back to back, a kernel then costs its own time plus about 1 us, where an
+// ordinary launch costs about 2.2 us and is rounded up to the next multiple of
+// 2.05 us (measured on a B200 with kernels of 1 to 14 us).  Reads and writes
+// stay ordered: nothing in global memory is touched before grid_wait()
+// returns.  No kernel lets its successor start earlier than that
+// (griddepcontrol.launch_dependents): CTAs placed while a grid of about one
+// CTA per SM still runs crowd the SMs that are idle or empty first (768^3 on
+// 64 x 64 tiles: 35 us per GEMM instead of 24.7 with the release at the
+// epilogue, 24 x 4096 x 4096 on 32 x 32 tiles 62 instead of 42 with it at the
+// start).
+template <class... P, class... A>
+inline cudaError_t launch_chained(void (*kernel)(P...), int grid, int threads, size_t smem,
+                                  cudaStream_t stream, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 }  // namespace sgb

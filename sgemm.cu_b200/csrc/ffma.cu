@@ -219,6 +219,7 @@ constexpr int kPackThreads = 256;
 constexpr int kPackUnroll = 8;
 
 __global__ void __launch_bounds__(kPackThreads) pack_rows_kernel(const PackJob a, const PackJob b) {
+    grid_wait();
     const int total = a.rows + b.rows;
     for (int r = blockIdx.x; r < total; r += gridDim.x) {
         const bool in_a = r < a.rows;
@@ -263,7 +264,7 @@ static void pack(const PackJob& a, const PackJob& b, cudaStream_t s) {
     const int total = a.rows + b.rows;
     const int sms = device_info().sm_count > 0 ? device_info().sm_count : 148;
     const int grid = std::max(1, std::min(total, sms * 8));
-    pack_rows_kernel<<<grid, kPackThreads, 0, s>>>(a, b);
+    launch_chained(pack_rows_kernel, grid, kPackThreads, 0, s, a, b);
 }
 
 }  // namespace ffma
@@ -355,8 +356,8 @@ int plain_launch_acc(int cfg, int m, int n, int k, float alpha, const float* A, 
     }
     occupancy(cfg);  // sets the dynamic shared-memory attribute once per device
     const int grid = p.tiles_m * p.tiles_n;
-    cd.kernel<<<grid, cd.threads, cd.smem, stream>>>(tmA, tmB, p);
-    return cuda_status(cudaGetLastError());
+    return cuda_status(
+        launch_chained(cd.kernel, grid, cd.threads, cd.smem, stream, tmA, tmB, p));
 }
 
 }  // namespace sgb

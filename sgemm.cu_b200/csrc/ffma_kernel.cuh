@@ -555,6 +555,7 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
             fence_barrier_init();
         }
         __syncthreads();  // the only CTA-wide barrier: barriers initialised
+        grid_wait();
         if (warp == C::WM * C::WN) {
             // ------------------------------------------------ TMA producer --
             if (lane == 0 && nk > 0) {
@@ -616,6 +617,7 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
         return;
     }
 
+    grid_wait();
     const int wm = warp / C::WN, wn = warp % C::WN;
     int lm, ln;
     lane_coords(lane, lm, ln);

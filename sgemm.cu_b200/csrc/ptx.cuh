@@ -94,6 +94,15 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
     return mbar_wait_for(bar, parity, kWaitLimitNs);
 }
 
+// -------------------------------------------------- programmatic launch --
+
+// Wait until the kernels before this one in the stream have completed and
+// their memory operations are visible; returns at once when the launch had no
+// programmatic dependency.  Comes before a kernel's first global access.
+__device__ __forceinline__ void grid_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // ---------------------------------------------------------------------- TMA --
 
 __device__ __forceinline__ void tma_prefetch_desc(const void* tmap) {
