@@ -13,118 +13,132 @@ namespace sgb {
 namespace ffma {
 
 // Compiled configurations (the public config id is the position in kConfigs).
-//   tile      warps  thread tile  stages  loader   resident CTAs/SM
-using C0 = Cfg<128, 256, 4, 2, 16, 4, kLoaderTma, 1>;        // 8 warps, 192 KB smem, 1/SM
-using C1 = Cfg<128, 128, 4, 2, 8, 3, kLoaderTma, 2>;         // 8 warps,  96 KB, 2/SM
-using C2 = Cfg<128, 128, 4, 1, 16, 3, kLoaderTma, 2>;        // 4 warps,  96 KB, 2/SM
-using C3 = Cfg<64, 128, 2, 2, 8, 4, kLoaderTma, 2>;          // 4 warps,  96 KB, 2/SM
-using C4 = Cfg<64, 64, 2, 1, 8, 4, kLoaderTma, 3>;           // 2 warps,  64 KB, 3/SM
-using C5 = Cfg<64, 128, 2, 2, 8, 3, kLoaderTma, 3>;          // 4 warps,  72 KB, 3/SM
-using C6 = Cfg<128, 64, 4, 1, 8, 3, kLoaderTma, 3>;          // 4 warps,  72 KB, 3/SM
-// Small tiles with 8 x 4 threads, for problems that leave most SMs idle with
-// the tiles above (shared memory limits them to 3 and 4 CTAs/SM).
-using S0 = Cfg<64, 64, 2, 2, 4, 4, kLoaderTma, 4>;         // 4 warps,  64 KB
-using S1 = Cfg<32, 64, 1, 2, 4, 4, kLoaderTma, 6>;         // 2 warps,  48 KB
+//   tile  warps m x n  columns  stages  loader  CTAs/SM  rows  transposed A
+//
+// Large tiles read A transposed (compute_stage_kmajor).  B200, TFLOP/s at
+// beta 0, against the same tiles on A [row][k]: 128 x 64 at 4096^3 66.3 from
+// 58.8 and at 8192^3 (beta 0.5) 67.3 from 59.6 (90% of the FP32 peak from 80),
+// 28 x 256 at 2048^3 59.1 from 57.6, all with the transpose in the time.
+using C0 = Cfg<128, 256, 4, 2, 16, 4, kLoaderTma, 1, 8, true>;
+using C1 = Cfg<128, 128, 4, 2, 8, 3, kLoaderTma, 1, 8, true>;
+using C2 = Cfg<128, 128, 4, 1, 16, 3, kLoaderTma, 1, 8, true>;
+using C3 = Cfg<64, 128, 2, 2, 8, 4, kLoaderTma, 2, 8, true>;
+using C4 = Cfg<64, 64, 2, 1, 8, 4, kLoaderTma, 3, 8, true>;
+using C5 = Cfg<64, 128, 2, 2, 8, 3, kLoaderTma, 3, 8, true>;
+using C6 = Cfg<128, 64, 4, 1, 8, 3, kLoaderTma, 3, 8, true>;
+using S0 = Cfg<64, 64, 2, 2, 4, 4, kLoaderTma, 3>;
+using S1 = Cfg<32, 64, 1, 2, 4, 4, kLoaderTma, 4>;
 using C8 = Cfg<128, 256, 4, 2, 16, 4, kLoaderAsync4, 1>;
 using C9 = Cfg<128, 128, 4, 2, 8, 3, kLoaderAsync4, 2>;
 using C11 = Cfg<64, 128, 2, 2, 8, 4, kLoaderAsync4, 2>;
 using C12 = Cfg<64, 64, 2, 1, 8, 4, kLoaderAsync4, 3>;
 using C14 = Cfg<128, 64, 4, 1, 8, 3, kLoaderAsync4, 3>;
-// The 128 x 64 tile with twice the warps (8 x 4 threads): for problems that
-// are a single partial wave, where each busy SM holds one tile and four warps
-// cannot hide the shared-memory and barrier latency.
-using W0 = Cfg<128, 64, 4, 2, 4, 3, kLoaderTma, 3>;        // 8 warps,  72 KB
-using W1 = Cfg<128, 64, 4, 2, 4, 4, kLoaderTma, 2>;        // 8 warps,  96 KB
-// The best large tile with a producer warp (per-stage empty mbarriers, no CTA
-// barrier in the main loop).
-using P0 = Cfg<128, 64, 4, 1, 8, 3, kLoaderTma, 3, 8, 1>;  // 4+1 warps, 72 KB
-using P1 = Cfg<128, 64, 4, 1, 8, 4, kLoaderTma, 2, 8, 1>;  // 4+1 warps, 96 KB
-// A 28 x 256 tile of four warps side by side, 7 x 8 outputs per thread, with a
-// producer warp: a 1024 x 1024 output is 37 x 4 = 148 tiles, one per SM, each
-// thread doing 56 FMAs per k step where the 128 x 64 tile (128 tiles, 20 SMs
-// idle) does 64.  With 4 stages one CTA fits an SM; with 3, two do (2048^3:
-// 592 tiles, two full waves of eight compute warps per SM).
-using T0 = Cfg<28, 256, 1, 4, 8, 4, kLoaderTma, 1, 8, 1, 7>;  // 4+1 warps, 145 KB, 1/SM
-using T3 = Cfg<28, 256, 1, 4, 8, 3, kLoaderTma, 2, 8, 1, 7>;  // 4+1 warps, 109 KB, 2/SM
+using W0 = Cfg<128, 64, 4, 2, 4, 3, kLoaderTma, 2, 8, true>;
+using W1 = Cfg<128, 64, 4, 2, 4, 4, kLoaderTma, 2, 8, true>;
+using P0 = Cfg<128, 64, 4, 1, 8, 3, kLoaderTma, 3, 8, true>;
+using P1 = Cfg<128, 64, 4, 1, 8, 4, kLoaderTma, 2, 8, true>;
+// 28 x 256 tiles, 7 x 8 outputs per thread: a 1024 x 1024 output is 37 x 4 =
+// 148 tiles, one per SM, each thread doing 56 FMAs per k step where the
+// 128 x 64 tile (128 tiles, 20 SMs idle) does 64; two CTAs fit an SM with 3
+// stages (2048^3: 592 tiles, two full waves).  The one-CTA form keeps A
+// [row][k]: at 1024^3 the transpose costs more than it gives (47.8 against
+// 41.6 us).
+using T0 = Cfg<28, 256, 1, 4, 8, 4, kLoaderTma, 1, 7>;
+using T3 = Cfg<28, 256, 1, 4, 8, 3, kLoaderTma, 2, 7, true>;
+// Small threads (4 x 2 and 4 x 4 outputs) for outputs too few to give every
+// scheduler an 8-row one: a few rows against a wide B, and squares below
+// ~900.  A 24 x 4096 x 4096 GEMM, whose 64 tiles of 32 x 64 left 84 SMs idle at
+// 57 cycles per k step (117.5 us), takes 42 us on 128 tiles of 32 x 32 (19
+// cycles); 64 rows 59 us from 118, 512^3 8.9 from 16.2.  Deep rings: these
+// stream B from HBM, 4-8 KB per stage.  What bounds them is issue (one warp per
+// scheduler, every instruction taking two cycles) and, from two CTAs per SM,
+// shared-memory loads (a wavefront carries two floats per lane).
+using K1 = Cfg<16, 32, 1, 2, 2, 12, kLoaderTma, 2, 4>;
+using K2 = Cfg<32, 32, 2, 2, 2, 10, kLoaderTma, 2, 4>;
+using K3 = Cfg<32, 64, 2, 2, 4, 8, kLoaderTma, 2, 4>;
+using K4 = Cfg<16, 128, 1, 4, 4, 6, kLoaderTma, 2, 4>;
+using K6 = Cfg<64, 64, 4, 2, 4, 6, kLoaderTma, 2, 4>;
+using K8 = Cfg<32, 128, 2, 4, 4, 5, kLoaderTma, 2, 4>;
+using Q3 = Cfg<32, 64, 2, 2, 4, 8, kLoaderTma, 2, 4, true>;
+using Q7 = Cfg<64, 64, 2, 2, 4, 6, kLoaderTma, 2, 8, true>;
+using A2 = Cfg<32, 32, 2, 2, 2, 4, kLoaderAsync4, 2, 4>;
+using A3 = Cfg<32, 64, 2, 2, 4, 4, kLoaderAsync4, 2, 4>;
+
+// What a launch costs, in microseconds on a B200 at 1965 MHz: with c CTAs on the
+// busiest SM a k step takes u c + v cycles, and each of the c rounds w for its
+// prologue and epilogue.  u / (BM BN / 128) is the reciprocal of the tile's
+// share of the FP32 peak when the SM is full; v is what too few warps leave
+// idle.
+struct Cost {
+    float u, v, w;
+};
 
 struct ConfigDesc {
     const char* name;
     int bm, bn, threads, smem, loader;
-    float efficiency;  // relative per-SM throughput when the grid fills the GPU
-    // relative throughput used instead when the whole problem is one partial
-    // wave with a single CTA on the busiest SM (a lone CTA per SM); 0: the
-    // configuration's full-wave efficiency
-    float lone;
+    bool km;    // reads A transposed
+    int a_box;  // rows of an A box (slots when transposed)
+    Cost cost;
     void (*kernel)(const CUtensorMap, const CUtensorMap, const Params);
 };
 
 template <class C>
-constexpr ConfigDesc describe(const char* name, float eff, float lone = 0.0f) {
-    return ConfigDesc{name, C::BM, C::BN, C::THREADS, C::SMEM_BYTES, C::LOADER, eff, lone,
-                      &ffma_gemm_kernel<C>};
+constexpr ConfigDesc describe(const char* name, float u, float v, float w) {
+    return ConfigDesc{name, C::BM, C::BN, C::THREADS, C::SMEM_BYTES, C::LOADER, C::KM,
+                      C::A_BOX, Cost{u, v, w}, &ffma_gemm_kernel<C>};
 }
 
-// Efficiencies: relative per-SM throughput of a full wave, normalised to the
-// best configuration of the same loader (TMA: tma_128x64_w4_t8x8_s3;
-// cp.async: cpa_128x256_w8_t8x16_s4).  The large tiles were measured at
-// 8192^3 / 16384^3 (the 8 x 16-thread tiles at 4096^3, where their longer
-// fill and drain costs them most); the small and mid tiles and the
-// partial-wave fractions in plain_select were then fitted to B200 sweeps of
-// 256..16384 cubes and of 1000, 3001, 5003 and 8191: the model's pick is
-// within 0.2% of the fastest measured configuration at every one of those
-// sizes.  The 8-warp 128 x 64 tiles and the producer-warp tiles were measured
-// later (B200, interleaved timing at 1000..8192): the 4-stage producer tile
-// ties the 3-stage tile within 0.2% from 4096^3 up and is 3.4% (1024^3) to
-// 5.6% (1000^3) faster when the problem is one partial wave with a lone CTA
-// per SM and beta = 0; the 8-warp tiles are slower everywhere.  The model
-// gives the 4-stage producer tile its measured lone-CTA throughput (1.045 of
-// the 3-stage tile's) and a full-wave figure that keeps multi-wave problems
-// on the tiles that measured best there: at 2048^3 its two CTAs per SM fit the
-// 512 tiles in two waves, yet the 64 x 64 tile is 1.6-2.2% faster.  The
-// 28 x 256 tiles were measured the same way at 768..12288.  The 4-stage one
-// (one CTA per SM) is 9-11% faster than the previous pick at 1000^3 and
-// 1024^3 and 8-9% at 896^3 (both betas) and slower elsewhere; 0.80
-// reproduces those picks.  The 3-stage one (two CTAs per SM) is 10-12%
-// faster at 2048^3, 1.4-1.9% at 3072^3 and 6144^3, within 0.5% at 4096^3,
-// 8192^3 and 12288^3, 3% slower at 1280^3 and 2560^3 and far slower at
-// 1536^3 (330 tiles: a third, near-empty wave); 0.99 picks it at 2048^3,
-// 4096^3 and 6144^3 and leaves 8192^3 on the 128 x 64 tile, and its lone
-// figure, 0.95, keeps 896..1024 on the 4-stage tile, 1-3% faster there.
-// (Measured and dropped: 6 stages, 1-3% slower than 4; eight 7 x 4-thread
-// warps, 2-5% slower at beta = 0; 32-row rasterisation bands, no change.)
+// u, v, w fitted per configuration to B200 timings of grids of 148 c CTAs,
+// c = 1..8, at k = 1024 and 3072 (the slope gives u c + v, the rest w).
 static const ConfigDesc kConfigs[] = {
-    describe<C0>("tma_128x256_w8_t8x16_s4", 0.840f),   describe<C1>("tma_128x128_w8_t8x8_s3", 0.900f),
-    describe<C2>("tma_128x128_w4_t8x16_s3", 0.875f),   describe<C3>("tma_64x128_w4_t8x8_s4", 0.920f),
-    describe<C4>("tma_64x64_w2_t8x8_s4", 0.700f),      describe<C5>("tma_64x128_w4_t8x8_s3", 0.994f),
-    describe<C6>("tma_128x64_w4_t8x8_s3", 1.000f),     describe<S0>("tma_64x64_w4_t8x4_s4", 0.860f),
-    describe<S1>("tma_32x64_w2_t8x4_s4", 0.700f),      describe<C8>("cpa_128x256_w8_t8x16_s4", 1.000f),
-    describe<C9>("cpa_128x128_w8_t8x8_s3", 0.920f),    describe<C11>("cpa_64x128_w4_t8x8_s4", 0.810f),
-    describe<C12>("cpa_64x64_w2_t8x8_s4", 0.630f),     describe<C14>("cpa_128x64_w4_t8x8_s3", 0.890f),
-    describe<W0>("tma_128x64_w8_t8x4_s3", 0.850f),     describe<W1>("tma_128x64_w8_t8x4_s4", 0.900f),
-    describe<P0>("tma_128x64_w4p_t8x8_s3", 0.900f),    describe<P1>("tma_128x64_w4p_t8x8_s4", 0.900f, 1.045f),
-    describe<T0>("tma_28x256_w4p_t7x8_s4", 0.800f),    describe<T3>("tma_28x256_w4p_t7x8_s3", 0.990f, 0.950f),
+    describe<C0>("tma_128x256_w8_t8x16_s4", 321.6f, 1.6f, 3.6f),
+    describe<C1>("tma_128x128_w8_t8x8_s3", 142.2f, 1.3f, 2.9f),
+    describe<C2>("tma_128x128_w4_t8x16_s3", 147.4f, 0.6f, 3.0f),
+    describe<C3>("tma_64x128_w4_t8x8_s4", 70.2f, 5.5f, 0.8f),
+    describe<C4>("tma_64x64_w2_t8x8_s4", 52.0f, 30.0f, 0.8f),
+    describe<C5>("tma_64x128_w4_t8x8_s3", 69.4f, 7.3f, 0.8f),
+    describe<C6>("tma_128x64_w4_t8x8_s3", 69.2f, 7.3f, 0.8f),
+    describe<S0>("tma_64x64_w4_t8x4_s4", 40.7f, 7.0f, 0.5f),
+    describe<S1>("tma_32x64_w2_t8x4_s4", 24.0f, 36.0f, 0.5f),
+    describe<C8>("cpa_128x256_w8_t8x16_s4", 425.5f, 1.0f, 3.3f),
+    describe<C9>("cpa_128x128_w8_t8x8_s3", 225.0f, 12.0f, 1.7f),
+    describe<C11>("cpa_64x128_w4_t8x8_s4", 131.0f, 18.0f, 1.2f),
+    describe<C12>("cpa_64x64_w2_t8x8_s4", 77.0f, 75.0f, 0.8f),
+    describe<C14>("cpa_128x64_w4_t8x8_s3", 118.5f, 27.0f, 1.2f),
+    describe<W0>("tma_128x64_w8_t8x4_s3", 75.4f, 1.5f, 0.8f),
+    describe<W1>("tma_128x64_w8_t8x4_s4", 75.4f, 1.8f, 0.8f),
+    describe<P0>("tma_128x64_w4p_t8x8_s3", 69.2f, 7.4f, 0.8f),
+    describe<P1>("tma_128x64_w4p_t8x8_s4", 70.3f, 6.5f, 0.8f),
+    describe<T0>("tma_28x256_w4p_t7x8_s4", 74.5f, 1.0f, 2.4f),
+    describe<T3>("tma_28x256_w4p_t7x8_s3", 64.6f, 9.5f, 0.9f),
+    describe<K1>("tma_16x32_w2_t4x2", 9.4f, 7.0f, 0.3f),
+    describe<K2>("tma_32x32_w4_t4x2", 13.5f, 5.0f, 0.4f),
+    describe<K3>("tma_32x64_w4_t4x4", 21.7f, 5.4f, 0.5f),
+    describe<K4>("tma_16x128_w4_t4x4", 22.0f, 6.6f, 0.6f),
+    describe<K6>("tma_64x64_w8_t4x4", 41.8f, 1.7f, 0.7f),
+    describe<K8>("tma_32x128_w8_t4x4", 41.9f, 1.7f, 0.7f),
+    describe<Q3>("tma_32x64_w4_t4x4_at", 19.5f, 6.0f, 0.6f),
+    describe<Q7>("tma_64x64_w4_t8x4_at", 37.8f, 8.6f, 0.6f),
+    describe<A2>("cpa_32x32_w4_t4x2_s4", 26.0f, 16.0f, 0.5f),
+    describe<A3>("cpa_32x64_w4_t4x4_s4", 41.5f, 22.0f, 0.5f),
 };
 constexpr int kNumConfigs = sizeof(kConfigs) / sizeof(kConfigs[0]);
 
-static int occupancy(int cfg) {
-    static int occ[64][kNumConfigs];
+// The kernel's shared-memory attribute, once per device.
+static cudaError_t set_smem_attribute(int cfg) {
     static bool have[64][kNumConfigs];
     static std::mutex mu;
     const DeviceInfo& d = device_info();
-    if (d.device < 0 || d.device >= 64) return 1;
+    if (d.device < 0 || d.device >= 64) return cudaErrorInvalidDevice;
     std::lock_guard<std::mutex> lock(mu);
     if (!have[d.device][cfg]) {
-        const ConfigDesc& c = kConfigs[cfg];
-        int o = 0;
-        cudaFuncSetAttribute(c.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, c.smem);
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, c.kernel, c.threads, c.smem) !=
-                cudaSuccess ||
-            o < 1)
-            o = 1;
-        occ[d.device][cfg] = o;
+        const cudaError_t e =
+            cudaFuncSetAttribute(kConfigs[cfg].kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 kConfigs[cfg].smem);
+        if (e != cudaSuccess) return e;
         have[d.device][cfg] = true;
     }
-    return occ[d.device][cfg];
+    return cudaSuccess;
 }
 
 static bool tma_ok(const float* A, int lda, const float* B, int ldb) {
@@ -145,26 +159,22 @@ int plain_config_tile(int cfg, int* bm, int* bn) {
     return SGEMM_B200_OK;
 }
 
-// Pick the configuration with the smallest modelled time.  A configuration
-// with `occ` resident CTAs per SM runs tiles in waves of SMs x occ; one CTA of
-// a full wave takes t = occ * BM * BN / efficiency (per-SM throughput shared
-// by occ CTAs).  The last, partial wave leaves r = ceil(remainder / SMs) < occ
-// CTAs on the busiest SM, which then runs at a fraction e(r) of its full
-// throughput (fewer warps to hide latency), so that wave takes
-// t * (r / occ) / e(r).  e(1) = 0.70, e(2) = e(3) = 0.90 were fitted to the
-// same B200 measurements as the efficiencies.  One exception, also measured:
-// when the whole problem is that one partial wave with a single CTA per SM
-// and C is not read (beta == 0), e(1) = 0.82 -- the lone CTA's epilogue then
-// only writes, and nothing else on the SM waits for it (1000^3 and 1024^3 at
-// beta = 0 run 3.6-4.5% faster on the 128 x 64 tile than on 64 x 64, while at
-// beta = 0.5 the 64 x 64 tile is 3% faster).
-static double partial_wave_cost(int r, int occ, bool alone, bool reads_c) {
-    if (r >= occ) return 1.0;
-    const double e = r == 1 ? (alone && !reads_c ? 0.82 : 0.70) : 0.90;
-    return (double(r) / occ) / e;
+// Modelled time of a problem on a configuration, in microseconds.  Tiles go to
+// whichever SM is free, so the busiest SM runs ceil(tiles / SMs) of them, and
+// once there are many the ends no longer line up.  A configuration that reads A
+// transposed also pays for the transpose (its launch, and its bytes at the rate
+// it runs at).
+static double modelled_us(const ffma::ConfigDesc& cd, int m, int n, int k, int sms, bool reads_c) {
+    const double per_sm = double(div_up(m, cd.bm)) * div_up(n, cd.bn) / sms;
+    const double c = per_sm > 8 ? per_sm + 0.5 : std::ceil(per_sm);
+    const double t = c * cd.cost.w * (reads_c ? 1.6 : 1.0) +
+                     double(k) * (cd.cost.u * c + cd.cost.v) / 1965.0;
+    return cd.km ? t + 3.0 + 8.0 * double(m) * k / 4.5e6 : t;
 }
 
-static int select_for_loader(int m, int n, int k, int loader, bool reads_c) {
+// The configuration with the smallest modelled time (the first of equals).
+// `scratch`: configurations that read A transposed may be taken.
+static int select_for_loader(int m, int n, int k, int loader, bool reads_c, bool scratch = true) {
     using namespace ffma;
     const DeviceInfo& d = device_info();
     const int sms = d.sm_count > 0 ? d.sm_count : 148;
@@ -172,26 +182,22 @@ static int select_for_loader(int m, int n, int k, int loader, bool reads_c) {
     double best_t = 1e300;
     for (int c = 0; c < kNumConfigs; ++c) {
         const ConfigDesc& cd = kConfigs[c];
-        if (cd.loader != loader) continue;
-        const int occ = occupancy(c);
-        const double tiles = double(div_up(m, cd.bm)) * div_up(n, cd.bn);
-        const double slots = double(sms) * occ;
-        const double full = std::floor(tiles / slots);
-        const double rem = tiles - full * slots;
-        double waves = full;
-        const int r = rem > 0 ? static_cast<int>(std::ceil(rem / sms)) : 0;
-        if (rem > 0) waves += partial_wave_cost(r, occ, full == 0, reads_c);
-        // a lone CTA per SM runs one warp per scheduler: latency, not the FMA
-        // pipe, limits it, and the producer-warp tile hides more of it
-        const double eff = (full == 0 && r == 1 && cd.lone > 0) ? cd.lone : cd.efficiency;
-        const double t = waves * occ * double(cd.bm) * cd.bn / eff;
-        if (best < 0 || t < best_t * 0.999) {
+        if (cd.loader != loader || (cd.km && !scratch)) continue;
+        const double t = modelled_us(cd, m, n, k, sms, reads_c);
+        if (best < 0 || t < best_t) {
             best_t = t;
             best = c;
         }
     }
-    (void)k;
     return best;
+}
+
+// The same among the configurations that need no scratch: the operands in place.
+static int select_in_place(int m, int n, int k, const float* A, int lda, const float* B, int ldb,
+                           bool reads_c) {
+    using namespace ffma;
+    const int loader = (k == 0 || tma_ok(A, lda, B, ldb)) ? kLoaderTma : kLoaderAsync4;
+    return select_for_loader(m, n, k, loader, reads_c, false);
 }
 
 int plain_select(int m, int n, int k, const float* A, int lda, const float* B, int ldb,
@@ -203,25 +209,96 @@ int plain_select(int m, int n, int k, const float* A, int lda, const float* B, i
 
 namespace ffma {
 
-// Row copy into a 16-byte-aligned pitch (the pack step for strides TMA cannot
-// describe), for up to two matrices in one launch: block b copies rows b,
-// b + gridDim.x, ... of A's rows followed by B's; within a row the threads
-// take consecutive columns (coalesced), eight loads in flight per thread
-// before their stores.  HBM-bound; the padding columns are not written (the
-// TMA kernel reads only the first `cols` of each row).
+// Operand preparation, one launch for both operands: A transposed for the
+// configurations that read it [k][slot], and row copies into a 16-byte-aligned
+// pitch for strides TMA cannot describe.
 struct PackJob {
     const float* src;
     float* dst;
     int rows, cols, ld_src, ld_dst;
 };
 
+// A [m x lda] -> [k][ld]: row r at slot r, or, for 7-row threads, in groups of
+// 28 rows per 32 slots whose last 12 rows sit 3 to 4 slots (Cfg::SLOTS).
+struct TransposeJob {
+    const float* src;
+    float* dst;
+    int m, k, ld_src, ld_dst;
+    int sevens;  // 7-row slots
+    int vec;     // 16-byte aligned rows: float4 loads
+    int blocks;  // blocks of the launch that work on it (0: none)
+};
+
 constexpr int kPackThreads = 256;
 constexpr int kPackUnroll = 8;
+constexpr int kTrTile = 64;  // transposed by 64 x 64 tiles
 
-__global__ void __launch_bounds__(kPackThreads) pack_rows_kernel(const PackJob a, const PackJob b) {
+__device__ __forceinline__ int slot_of(int row, int sevens) {
+    if (!sevens) return row;
+    const int q = row % 28;
+    return row / 28 * 32 + (q < 16 ? q : 16 + (q - 16) / 3 * 4 + (q - 16) % 3);
+}
+
+__device__ __forceinline__ void transpose_tiles(const TransposeJob& j, float (&tile)[kTrTile][kTrTile + 1]) {
+    const int tk = (j.k + kTrTile - 1) / kTrTile, tiles = tk * ((j.m + kTrTile - 1) / kTrTile);
+    const int c4 = threadIdx.x % 16, r0 = threadIdx.x / 16;  // 16 float4 columns x 16 rows
+    for (int t = blockIdx.x; t < tiles; t += j.blocks) {
+        const int k0 = t % tk * kTrTile, m0 = t / tk * kTrTile;
+        float4 v[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int row = m0 + r0 + 16 * i, k = k0 + 4 * c4;
+            v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (row >= j.m) continue;
+            const float* p = j.src + (int64_t)row * j.ld_src + k;
+            if (j.vec && k + 3 < j.k) {
+                v[i] = *reinterpret_cast<const float4*>(p);
+            } else {
+                if (k < j.k) v[i].x = p[0];
+                if (k + 1 < j.k) v[i].y = p[1];
+                if (k + 2 < j.k) v[i].z = p[2];
+                if (k + 3 < j.k) v[i].w = p[3];
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int r = r0 + 16 * i;
+            tile[4 * c4][r] = v[i].x;
+            tile[4 * c4 + 1][r] = v[i].y;
+            tile[4 * c4 + 2][r] = v[i].z;
+            tile[4 * c4 + 3][r] = v[i].w;
+        }
+        __syncthreads();
+        const int row = m0 + threadIdx.x % 64;
+        const int slot = slot_of(row, j.sevens);
+        if (row < j.m) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                const int kk = threadIdx.x / 64 + 4 * i;
+                if (k0 + kk < j.k)
+                    j.dst[(int64_t)(k0 + kk) * j.ld_dst + slot] = tile[kk][threadIdx.x % 64];
+            }
+        }
+        __syncthreads();  // the next tile overwrites `tile`
+    }
+}
+
+// Blocks of the transpose, then blocks that copy rows: block r of those copies
+// rows r, r + their count, ... of a's rows followed by b's (a job with no rows
+// is skipped); within a row the threads take consecutive columns (coalesced),
+// eight loads in flight per thread before their stores.  The padding columns
+// are not written (the TMA kernel reads only the first `cols` of each row).
+// HBM-bound.
+__global__ void __launch_bounds__(kPackThreads)
+    prepare_kernel(const TransposeJob t, const PackJob a, const PackJob b) {
+    __shared__ float tile[kTrTile][kTrTile + 1];
     grid_wait();
+    if ((int)blockIdx.x < t.blocks) {
+        transpose_tiles(t, tile);
+        return;
+    }
     const int total = a.rows + b.rows;
-    for (int r = blockIdx.x; r < total; r += gridDim.x) {
+    for (int r = blockIdx.x - t.blocks; r < total; r += gridDim.x - t.blocks) {
         const bool in_a = r < a.rows;
         const int row = in_a ? r : r - a.rows;
         const int cols = in_a ? a.cols : b.cols;
@@ -245,9 +322,11 @@ __global__ void __launch_bounds__(kPackThreads) pack_rows_kernel(const PackJob a
     }
 }
 
-// Work (m*n*k) above which copying unaligned operands to aligned rows and
-// running the TMA kernel beats the 4-byte cp.async loader.
-constexpr double kPackMinWork = 134217728.0;  // 512^3
+// Work (m*n*k) above which copying unaligned operands to aligned rows (one
+// more launch, about 3 us) and running the TMA kernel beats the 4-byte
+// cp.async loader: on a B200 317^3 takes 10.0 us on the small cp.async tiles
+// and 321^3 9.4 us copied; 401^3 37.6 us on the large ones, 10.1 us copied.
+constexpr double kPackMinWork = 32.0e6;  // 317^3
 
 // Operands the plain path copies to aligned rows before its TMA kernel:
 // bit 0 A, bit 1 B; 0 when the kernel reads them in place.
@@ -258,69 +337,28 @@ static int pack_mask(int m, int n, int k, const float* A, int lda, const float* 
     return (pa ? 1 : 0) | (pb ? 2 : 0);
 }
 
-// One launch for both operands (a job with rows == 0 is skipped): eight
-// blocks per SM, each looping over rows.
-static void pack(const PackJob& a, const PackJob& b, cudaStream_t s) {
-    const int total = a.rows + b.rows;
+// One launch for the jobs given (at least one): about eight blocks per SM,
+// shared between transpose and copies in proportion to their size.
+static cudaError_t prepare(TransposeJob t, const PackJob& a, const PackJob& b, cudaStream_t s) {
     const int sms = device_info().sm_count > 0 ? device_info().sm_count : 148;
-    const int grid = std::max(1, std::min(total, sms * 8));
-    launch_chained(pack_rows_kernel, grid, kPackThreads, 0, s, a, b);
+    const int tiles = t.dst ? div_up(t.m, kTrTile) * div_up(t.k, kTrTile) : 0;
+    const double wt = t.dst ? double(t.m) * t.k : 0.0;
+    const double wp = double(a.rows) * a.cols + double(b.rows) * b.cols;
+    const int want = sms * 8, rows = a.rows + b.rows;
+    t.blocks = std::min(tiles, std::max(1, int(want * (wt / (wt + wp)))));
+    const int copies = std::min(rows, std::max(1, want - t.blocks));
+    return launch_chained(prepare_kernel, t.blocks + copies, kPackThreads, 0, s, t, a, b);
 }
 
 }  // namespace ffma
 
-int plain_launch(int cfg, int m, int n, int k, float alpha, const float* A, int lda,
-                 const float* B, int ldb, float beta, float* C, int ldc, cudaStream_t stream) {
-    return plain_launch_acc(cfg, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, nullptr, nullptr,
-                            0, stream);
-}
-
-int plain_launch_acc(int cfg, int m, int n, int k, float alpha, const float* A, int lda,
-                     const float* B, int ldb, float beta, float* C, int ldc, const float* acc_in,
-                     float* acc_out, int ld_acc, cudaStream_t stream) {
+// One launch of configuration cfg on operands it can read in place: A is the
+// transposed copy (pitch lda) for a configuration that reads it so.
+static int launch_config(int cfg, int m, int n, int k, float alpha, const float* A, int lda,
+                         const float* B, int ldb, float beta, float* C, int ldc,
+                         const float* acc_in, float* acc_out, int ld_acc, cudaStream_t stream) {
     using namespace ffma;
-    if (m == 0 || n == 0) return SGEMM_B200_OK;
-    if (!device_is_sm100()) return SGEMM_B200_ERR_UNSUPPORTED;
-    if ((acc_in || acc_out) &&
-        (ld_acc < n || ld_acc % 4 != 0 || reinterpret_cast<uintptr_t>(acc_in) % 16 != 0 ||
-         reinterpret_cast<uintptr_t>(acc_out) % 16 != 0))
-        return SGEMM_B200_ERR_INVALID_ARG;
-    // carried accumulators: the caller keeps its operands TMA-aligned (no pack step)
-    const int mask = (cfg < 0 && !acc_in && !acc_out) ? pack_mask(m, n, k, A, lda, B, ldb) : 0;
-    if (mask) {
-        // Unaligned strides on a large problem: copy the offending operand(s) to
-        // 16-byte-aligned rows (stream-ordered scratch from the library pool)
-        // and run the TMA kernel.  Same arithmetic, same bits.
-        cudaMemPool_t pool = library_pool();
-        if (pool) {
-            const bool pa = (mask & 1) != 0, pb = (mask & 2) != 0;
-            const int lda2 = pa ? (k + 3) / 4 * 4 : lda, ldb2 = pb ? (n + 3) / 4 * 4 : ldb;
-            float *A2 = nullptr, *B2 = nullptr;
-            cudaError_t e = cudaSuccess;
-            if (pa) e = cudaMallocFromPoolAsync(&A2, sizeof(float) * (size_t)m * lda2, pool, stream);
-            if (e == cudaSuccess && pb)
-                e = cudaMallocFromPoolAsync(&B2, sizeof(float) * (size_t)k * ldb2, pool, stream);
-            if (e == cudaSuccess) {
-                const PackJob ja = pa ? PackJob{A, A2, m, k, lda, lda2} : PackJob{};
-                const PackJob jb = pb ? PackJob{B, B2, k, n, ldb, ldb2} : PackJob{};
-                pack(ja, jb, stream);
-                const int s = plain_launch(-1, m, n, k, alpha, pa ? A2 : A, lda2, pb ? B2 : B,
-                                           ldb2, beta, C, ldc, stream);
-                if (A2) cudaFreeAsync(A2, stream);
-                if (B2) cudaFreeAsync(B2, stream);
-                return s;
-            }
-            if (A2) cudaFreeAsync(A2, stream);
-            if (B2) cudaFreeAsync(B2, stream);
-            cudaGetLastError();  // fall through to the cp.async loader
-        }
-    }
-    if (cfg < 0) cfg = plain_select(m, n, k, A, lda, B, ldb, beta != 0.0f);
-    if (cfg >= kNumConfigs) return SGEMM_B200_ERR_INVALID_ARG;
     const ConfigDesc& cd = kConfigs[cfg];
-    if (cd.loader == kLoaderTma && k > 0 && !tma_ok(A, lda, B, ldb))
-        return SGEMM_B200_ERR_INVALID_ARG;
-
     Params p;
     p.op.m = m;
     p.op.n = n;
@@ -346,18 +384,109 @@ int plain_launch_acc(int cfg, int m, int n, int k, float alpha, const float* A, 
     std::memset(&tmA, 0, sizeof(tmA));
     std::memset(&tmB, 0, sizeof(tmB));
     if (cd.loader == kLoaderTma && k > 0) {
-        if (!encode_tensor_map_2d(&tmA, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, A, (uint64_t)k,
-                                  (uint64_t)m, (uint64_t)lda * 4, 32, cd.bm,
-                                  CU_TENSOR_MAP_SWIZZLE_128B) ||
+        const bool okA =
+            cd.km ? encode_tensor_map_2d(&tmA, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, A,
+                                         (uint64_t)(cd.bm == 28 ? lda : m), (uint64_t)k,
+                                         (uint64_t)lda * 4, cd.a_box, 32,
+                                         CU_TENSOR_MAP_SWIZZLE_NONE)
+                  : encode_tensor_map_2d(&tmA, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, A, (uint64_t)k,
+                                         (uint64_t)m, (uint64_t)lda * 4, 32, cd.a_box,
+                                         CU_TENSOR_MAP_SWIZZLE_128B);
+        if (!okA ||
             !encode_tensor_map_2d(&tmB, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, B, (uint64_t)n,
                                   (uint64_t)k, (uint64_t)ldb * 4, cd.bn, 32,
                                   CU_TENSOR_MAP_SWIZZLE_NONE))
             return SGEMM_B200_ERR_CUDA;
     }
-    occupancy(cfg);  // sets the dynamic shared-memory attribute once per device
+    const cudaError_t e = set_smem_attribute(cfg);
+    if (e != cudaSuccess) return cuda_status(e);
     const int grid = p.tiles_m * p.tiles_n;
-    return cuda_status(
-        launch_chained(cd.kernel, grid, cd.threads, cd.smem, stream, tmA, tmB, p));
+    return cuda_status(launch_chained(cd.kernel, grid, cd.threads, cd.smem, stream, tmA, tmB,
+                                      p));
+}
+
+
+int plain_launch(int cfg, int m, int n, int k, float alpha, const float* A, int lda,
+                 const float* B, int ldb, float beta, float* C, int ldc, cudaStream_t stream) {
+    return plain_launch_acc(cfg, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, nullptr, nullptr,
+                            0, stream);
+}
+
+int plain_launch_acc(int cfg, int m, int n, int k, float alpha, const float* A, int lda,
+                     const float* B, int ldb, float beta, float* C, int ldc, const float* acc_in,
+                     float* acc_out, int ld_acc, cudaStream_t stream) {
+    using namespace ffma;
+    if (m == 0 || n == 0) return SGEMM_B200_OK;
+    if (!device_is_sm100()) return SGEMM_B200_ERR_UNSUPPORTED;
+    if ((acc_in || acc_out) &&
+        (ld_acc < n || ld_acc % 4 != 0 || reinterpret_cast<uintptr_t>(acc_in) % 16 != 0 ||
+         reinterpret_cast<uintptr_t>(acc_out) % 16 != 0))
+        return SGEMM_B200_ERR_INVALID_ARG;
+    // carried accumulators: the caller keeps its operands TMA-aligned (no pack step)
+    const int mask = (cfg < 0 && !acc_in && !acc_out) ? pack_mask(m, n, k, A, lda, B, ldb) : 0;
+    const bool chosen = cfg < 0;
+    if (chosen)
+        cfg = mask ? select_for_loader(m, n, k, kLoaderTma, beta != 0.0f)
+                   : plain_select(m, n, k, A, lda, B, ldb, beta != 0.0f);
+    if (cfg >= kNumConfigs) return SGEMM_B200_ERR_INVALID_ARG;
+    if (!mask && kConfigs[cfg].loader == kLoaderTma && k > 0 && !tma_ok(A, lda, B, ldb))
+        return SGEMM_B200_ERR_INVALID_ARG;
+
+    // Scratch from the library pool, stream-ordered: A transposed for a
+    // configuration that reads it so, or operands with strides TMA cannot
+    // describe copied to aligned rows.  Same arithmetic, same bits.
+    float *A2 = nullptr, *B2 = nullptr;
+    const bool km = kConfigs[cfg].km && k > 0;
+    if (km || mask) {
+        const bool sevens = kConfigs[cfg].bm == 28;
+        const bool pa = !km && (mask & 1) != 0, pb = (mask & 2) != 0;
+        const int lda2 = km ? (sevens ? div_up(m, 28) * 32 : (m + 3) / 4 * 4)
+                            : (k + 3) / 4 * 4;
+        const int ldb2 = pb ? (n + 3) / 4 * 4 : ldb;
+        const size_t a_bytes = km ? sizeof(float) * (size_t)k * lda2
+                                  : pa ? sizeof(float) * (size_t)m * lda2 : 0;
+        cudaMemPool_t pool = library_pool();
+        cudaError_t e = pool ? cudaSuccess : cudaErrorMemoryAllocation;
+        if (e == cudaSuccess && a_bytes) e = cudaMallocFromPoolAsync(&A2, a_bytes, pool, stream);
+        if (e == cudaSuccess && pb)
+            e = cudaMallocFromPoolAsync(&B2, sizeof(float) * (size_t)k * ldb2, pool, stream);
+        if (e != cudaSuccess) {
+            // no scratch: the best configuration that reads the operands in place
+            if (A2) cudaFreeAsync(A2, stream);
+            if (B2) cudaFreeAsync(B2, stream);
+            cudaGetLastError();
+            if (!chosen) return cuda_status(e);
+            return plain_launch_acc(select_in_place(m, n, k, A, lda, B, ldb, beta != 0.0f), m, n, k,
+                                    alpha, A, lda, B, ldb, beta, C, ldc, acc_in, acc_out, ld_acc,
+                                    stream);
+        }
+        TransposeJob jt = {};
+        PackJob ja = {}, jb = {};
+        if (km)
+            jt = TransposeJob{A, A2, m, k, lda, lda2, sevens,
+                              lda % 4 == 0 && reinterpret_cast<uintptr_t>(A) % 16 == 0, 0};
+        if (pa) ja = PackJob{A, A2, m, k, lda, lda2};
+        if (pb) jb = PackJob{B, B2, k, n, ldb, ldb2};
+        e = prepare(jt, ja, jb, stream);
+        if (e != cudaSuccess) {
+            if (A2) cudaFreeAsync(A2, stream);
+            if (B2) cudaFreeAsync(B2, stream);
+            return cuda_status(e);
+        }
+        if (A2) {
+            A = A2;
+            lda = lda2;
+        }
+        if (B2) {
+            B = B2;
+            ldb = ldb2;
+        }
+    }
+    const int st = launch_config(cfg, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, acc_in, acc_out,
+                                 ld_acc, stream);
+    if (A2) cudaFreeAsync(A2, stream);
+    if (B2) cudaFreeAsync(B2, stream);
+    return st;
 }
 
 }  // namespace sgb

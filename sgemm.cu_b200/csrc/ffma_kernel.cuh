@@ -12,15 +12,17 @@
 //
 // B200 design (not the reference's):
 //  - CTA tile BM x BN with a 32-deep k block, STAGES-deep ring of stages in
-//    shared memory filled by TMA (one elected thread, mbarrier completion) or,
-//    for strides that TMA cannot describe (lda/ldb not a multiple of 4),
+//    shared memory filled by a producer warp's TMA copies (mbarrier completion)
+//    or, for strides that TMA cannot describe (lda/ldb not a multiple of 4),
 //    by 4-byte cp.async with zero fill;
-//  - A is kept k-contiguous ([m][32] rows of 128 B) with the 128-byte XOR
-//    swizzle TMA applies, so a thread reads 4 k-values of one row with one
-//    conflict-free 128-bit shared load (instead of transposing A in smem);
-//  - B is kept [32][BN]; each 128-bit load is broadcast to the 4 lanes that
-//    share a column group (warp-level operand broadcast);
-//  - thread tile TM (m, 8 or 7) x TN (n); lanes 4 (m) x 8 (n); warps WM x WN;
+//  - large tiles read A transposed to [k][row] (a pass before the kernel), so
+//    the rows a k step multiplies arrive in consecutive registers; the others
+//    keep A k-contiguous ([m][32] rows of 128 B) with the 128-byte XOR swizzle
+//    TMA applies, so a thread reads 4 k-values of one row with one conflict-free
+//    128-bit shared load;
+//  - B is kept [32][BN]; each load is broadcast to the 4 lanes that share a
+//    column group (warp-level operand broadcast);
+//  - thread tile TM (m; 8, 7 or 4) x TN (n); lanes 4 (m) x 8 (n); warps WM x WN;
 //  - the FMAs are packed (fma.rn.f32x2, two columns of a row per
 //    instruction): the FP32 pipe, not instruction issue, becomes the limit;
 //  - epilogue straight from registers with float4 stores: for a fixed
@@ -37,27 +39,33 @@ namespace ffma {
 enum Loader { kLoaderTma = 0, kLoaderAsync4 = 1 };
 
 template <int BM_, int BN_, int WM_, int WN_, int TN_, int STAGES_, int LOADER_, int MINB_ = 1,
-          int K4U_ = 8, int PRODUCER_ = 0, int TM_ = 8>
+          int TM_ = 8, bool KM_ = false>
 struct Cfg {
     static constexpr int BM = BM_, BN = BN_, WM = WM_, WN = WN_, TN = TN_, STAGES = STAGES_;
     static constexpr int LOADER = LOADER_;
     static constexpr int MINB = MINB_;  // resident CTAs per SM the register budget targets
-    static constexpr int K4U = K4U_;    // unroll of the 8 four-deep k steps of a k block
-    // PRODUCER: one extra warp issues the TMA loads, and the compute warps free
-    // each stage through a per-stage "empty" mbarrier instead of a CTA barrier.
-    static constexpr int PRODUCER = PRODUCER_;
-    static constexpr int BK = 32;  // one 128-byte row of A per k block
-    // rows per thread: 8, or 7 for the tile whose 28 rows split a 1024-row
-    // problem into one CTA per SM
+    static constexpr bool TMA = LOADER_ == 0;
+    // KM: A comes transposed, [k][slot] (compute_stage_kmajor; the launcher
+    // transposes it first); otherwise A stays [row][k] (compute_stage).
+    static constexpr bool KM = KM_;
+    static_assert(TMA || !KM, "transposed A comes through TMA");
+    static constexpr int BK = 32;       // one 128-byte row of A per k block
+    // rows per thread: 8; 7 for the tile whose 28 rows split a 1024-row problem
+    // into one CTA per SM; 4 for tiles a few rows tall
     static constexpr int TM = TM_;
     static constexpr int WROWS = 4 * TM;  // rows of a warp's tile (4 lanes x TM)
     static constexpr int COMPUTE_THREADS = 32 * WM * WN;
-    static constexpr int THREADS = COMPUTE_THREADS + (PRODUCER ? 32 : 0);
-    static_assert(!PRODUCER || LOADER_ == 0, "the producer warp issues TMA loads");
+    static constexpr int THREADS = COMPUTE_THREADS + (TMA ? 32 : 0);  // + the producer warp
     static_assert(BM == WM * WROWS, "4 lanes x TM rows per warp along m");
     static_assert(BN == WN * 8 * TN, "8 lanes x TN columns per warp along n");
-    static_assert(TN % 4 == 0, "columns come in float4 groups");
-    static constexpr int A_TX = BM * BK * 4;  // bytes one A box brings
+    static constexpr int V = TN < 4 ? TN : 4;  // columns come in groups of V, 8 V apart
+    static_assert(TN % V == 0 && (V == 2 || V == 4), "vector column groups");
+    // Slots of a warp's rows in transposed A: its rows in order, but 7-row
+    // threads' last 3 rows padded to 4 (rows 16 + 3 lm + {0, 1, 2} at slot
+    // 16 + 4 lm), so that a thread's rows of a k are two 128-bit loads.
+    static constexpr int SLOTS = TM == 7 ? 32 : WROWS;
+    static constexpr int A_BOX = KM ? WM * SLOTS : BM;  // rows (slots) of an A box
+    static constexpr int A_TX = A_BOX * BK * 4;         // bytes one A box brings
     // A's region in a stage, rounded up to the 1024-byte swizzle atom so that
     // B (and the next stage) start on one
     static constexpr int A_BYTES = (A_TX + 1023) / 1024 * 1024;
@@ -65,21 +73,47 @@ struct Cfg {
     static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;  // stride between stages
     static constexpr int STAGE_TX = A_TX + B_BYTES;        // bytes a stage's copies bring
     static_assert(A_BYTES % 1024 == 0 && STAGE_BYTES % 1024 == 0, "1024-byte swizzle atoms");
-    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024;  // + alignment slack
+    static constexpr int RING_BYTES = STAGES * STAGE_BYTES;
+    static constexpr int SMEM_BYTES = RING_BYTES + 1024;  // + alignment slack
+
+    // The i-th row of lane row lm within a warp's tile.  KM: two runs, of 4 and
+    // TM - 4 rows, so the rows of a k come in two 128-bit loads.
+    __host__ __device__ static constexpr int row(int lm, int i) {
+        if (!KM) return lm + 4 * i;
+        return i < 4 ? 4 * lm + i : 16 + (TM - 4) * lm + i - 4;
+    }
+    // Lane -> (lm, ln) on the 4 (m) x 8 (n) lane grid; it only decides which
+    // thread owns which outputs.  A 128-bit shared load costs 2 wavefronts
+    // instead of 4 when neighbouring lanes of a quarter-warp share an address
+    // (measured on a B200), so lane bits 1 and 4 pick the row group and bits
+    // 0, 2 and 3 the column group: both operands' loads cost 2.
+    __device__ static void lane_coords(int lane, int& lm, int& ln) {
+        lm = ((lane >> 1) & 1) | ((lane >> 3) & 2);
+        ln = (lane & 1) | ((lane >> 1) & 6);
+    }
 };
 
-
-// Lane -> (lm, ln) on the 4 (m) x 8 (n) lane grid: lm = lane % 4,
-// ln = lane / 4, so a quarter-warp owns 4 rows x 2 column groups.  The map
-// only decides which thread owns which outputs (every output keeps its own
-// k-ordered FMA chain).  Measured on a B200 at 4096..16384 against
-// lm = lane / 8 (a quarter-warp on one row) and a 2 x 4 quarter-warp block:
-// this one is 0.5-2.6% faster although the 2 x 4 block needs fewer shared
-// wavefronts (2 instead of 3 per 128-bit load) -- shared bandwidth is not
-// what limits this kernel.
-__device__ __forceinline__ void lane_coords(int lane, int& lm, int& ln) {
-    lm = lane & 3;
-    ln = lane >> 2;
+// V consecutive floats to and from memory as one access.
+template <int V>
+__device__ __forceinline__ void load_vec(const void* p, float* v) {
+    if constexpr (V == 4) {
+        const float4 x = *reinterpret_cast<const float4*>(p);
+        v[0] = x.x;
+        v[1] = x.y;
+        v[2] = x.z;
+        v[3] = x.w;
+    } else {
+        const float2 x = *reinterpret_cast<const float2*>(p);
+        v[0] = x.x;
+        v[1] = x.y;
+    }
+}
+template <int V>
+__device__ __forceinline__ void store_vec(void* p, const float* v) {
+    if constexpr (V == 4)
+        *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+    else
+        *reinterpret_cast<float2*>(p) = make_float2(v[0], v[1]);
 }
 
 // Grouped rasterisation: 8 tile-rows share a band so concurrently resident
@@ -108,28 +142,6 @@ __device__ __forceinline__ void a_coords(int wm, int lm, uint32_t& a_base, uint3
     xa1 = static_cast<uint32_t>((r0 + 4) & 7) << 4;
 }
 
-// Fragment loads of one k block: A rows for the 4-deep step k4 (4 k-values of
-// each of the thread's 8 rows) and B columns for one k.
-template <class C>
-__device__ __forceinline__ void load_a_frag(const uint8_t* __restrict__ As, uint32_t a_base,
-                                            uint32_t xa0, uint32_t xa1, int k4,
-                                            float4 (&a)[C::TM]) {
-#pragma unroll
-    for (int i = 0; i < C::TM; ++i) {
-        const uint32_t x = (i & 1) ? xa1 : xa0;
-        const uint32_t off = a_base + i * 4 * 128 + ((static_cast<uint32_t>(k4) << 4) ^ x);
-        a[i] = *reinterpret_cast<const float4*>(As + off);
-    }
-}
-
-template <class C>
-__device__ __forceinline__ void load_b_frag(const uint8_t* __restrict__ Bs, uint32_t b_base, int k,
-                                            float4 (&b)[C::TN / 4]) {
-#pragma unroll
-    for (int g = 0; g < C::TN / 4; ++g)
-        b[g] = *reinterpret_cast<const float4*>(Bs + k * C::BN * 4 + b_base + g * 128);
-}
-
 // Accumulate one 32-deep k block held in shared memory: A fragments for a
 // 4-deep step at its start, B per k (the compiler schedules the loads).  Each
 // element accumulates over k in increasing order with one FMA per term.
@@ -138,7 +150,7 @@ __device__ __forceinline__ void compute_stage(const uint8_t* __restrict__ As,
                                                      const uint8_t* __restrict__ Bs,
                                                      uint32_t a_base, uint32_t xa0, uint32_t xa1,
                                                      uint32_t b_base, float (&acc)[C::TM][C::TN]) {
-#pragma unroll C::K4U
+#pragma unroll
     for (int k4 = 0; k4 < C::BK / 4; ++k4) {
         float4 a[C::TM];
 #pragma unroll
@@ -149,11 +161,11 @@ __device__ __forceinline__ void compute_stage(const uint8_t* __restrict__ As,
         }
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk) {
-            float4 b[C::TN / 4];
+            float bv[C::TN];
 #pragma unroll
-            for (int g = 0; g < C::TN / 4; ++g)
-                b[g] = *reinterpret_cast<const float4*>(Bs + (k4 * 4 + kk) * C::BN * 4 + b_base +
-                                                        g * 128);
+            for (int g = 0; g < C::TN / C::V; ++g)
+                load_vec<C::V>(Bs + (k4 * 4 + kk) * C::BN * 4 + b_base + g * 32 * C::V,
+                               &bv[C::V * g]);
             // Outer product with packed FP32 FMAs (fma.rn.f32x2): each
             // instruction updates two neighbouring columns of one row,
             // {c[i][j], c[i][j+1]} += {a_i, a_i} * {b_j, b_j+1}, with one
@@ -163,17 +175,10 @@ __device__ __forceinline__ void compute_stage(const uint8_t* __restrict__ As,
             // consecutive instructions share an operand at every turn.
             // Measured on a B200: +7.5% at 8192^3 over one fmaf per element
             // (which was issue-bound); serpentine order +0.7% over row-major.
-            float av[C::TM], bv[C::TN];
+            float av[C::TM];
 #pragma unroll
             for (int i = 0; i < C::TM; ++i)
                 av[i] = kk == 0 ? a[i].x : kk == 1 ? a[i].y : kk == 2 ? a[i].z : a[i].w;
-#pragma unroll
-            for (int g = 0; g < C::TN / 4; ++g) {
-                bv[4 * g + 0] = b[g].x;
-                bv[4 * g + 1] = b[g].y;
-                bv[4 * g + 2] = b[g].z;
-                bv[4 * g + 3] = b[g].w;
-            }
 #pragma unroll
             for (int i = 0; i < C::TM; ++i) {
                 const float2 a2 = make_float2(av[i], av[i]);
@@ -187,6 +192,55 @@ __device__ __forceinline__ void compute_stage(const uint8_t* __restrict__ As,
                 }
             }
         }
+    }
+}
+
+// Accumulate one k block with A kept [k][slot]: per k the thread's rows come
+// in two 128-bit loads and its columns in TN / 4, and one packed FMA (fma.rn.f32x2) updates two neighbouring columns
+// of a row with one rounding per element.
+//
+// Why this layout: with A [row][k], a thread's 128-bit load holds 4 k of one
+// row, so the TM values a k step multiplies sit in registers whose numbers
+// agree modulo 4, and the packed FMAs wait for register reads: the same loop
+// on resident tiles (no loads from memory, no barriers) reaches 73% of the
+// FP32 peak that way, 89-92% with the k step's rows in consecutive registers,
+// and 93.6% with the FMAs in this order -- pairs of column pairs, zigzag, so
+// neighbouring instructions share A's or B's operand.  (B200, 8 x 8 per
+// thread; registers only, no shared loads: 97%.)
+template <class C>
+__device__ __forceinline__ void compute_stage_kmajor(const uint8_t* __restrict__ At,
+                                                     const uint8_t* __restrict__ Bs, int wm,
+                                                     int lm, uint32_t b_base,
+                                                     float (&acc)[C::TM][C::TN]) {
+    const uint8_t* ap = At + (C::SLOTS * wm + 4 * lm) * 4;
+    const uint8_t* bp = Bs + b_base;
+#pragma unroll
+    for (int k = 0; k < C::BK; ++k) {
+        constexpr int TM = C::TM;
+        float a[8], b[C::TN];
+        load_vec<4>(ap + k * C::A_BOX * 4, a);
+        if constexpr (TM > 4) load_vec<4>(ap + k * C::A_BOX * 4 + 64, a + 4);
+#pragma unroll
+        for (int g = 0; g < C::TN / C::V; ++g)
+            load_vec<C::V>(bp + k * C::BN * 4 + g * 32 * C::V, &b[C::V * g]);
+        auto fma2 = [&](int i, int q) {
+            float2 c = make_float2(acc[i][2 * q], acc[i][2 * q + 1]);
+            c = __ffma2_rn(make_float2(a[i], a[i]), make_float2(b[2 * q], b[2 * q + 1]), c);
+            acc[i][2 * q] = c.x;
+            acc[i][2 * q + 1] = c.y;
+        };
+#pragma unroll
+        for (int q = 0; q < C::TN / 2; q += 2)
+#pragma unroll
+            for (int ii = 0; ii < TM; ++ii) {
+                const int i = (q & 2) ? TM - 1 - ii : ii;
+                if constexpr (C::TN == 2) {
+                    fma2(i, 0);
+                } else {
+                    fma2(i, q + (ii & 1));
+                    fma2(i, q + 1 - (ii & 1));
+                }
+            }
     }
 }
 
@@ -232,31 +286,29 @@ __device__ __forceinline__ void load_stage_async4(const Operands& p, uint8_t* As
 template <class C>
 __device__ __forceinline__ void epilogue_rows(const Operands& p, int m0, int n0, int wm, int wn,
                                               int lm, int ln, const float (&acc)[C::TM][C::TN]) {
-    const int col0 = n0 + wn * 8 * C::TN + ln * 4;
+    const int col0 = n0 + wn * 8 * C::TN + ln * C::V;
 #pragma unroll
     for (int i = 0; i < C::TM; ++i) {
-        const int row = m0 + wm * C::WROWS + lm + 4 * i;
+        const int row = m0 + wm * C::WROWS + C::row(lm, i);
         if (row >= p.m) continue;
         float* crow = p.C + (int64_t)row * p.ldc;
 #pragma unroll
-        for (int g = 0; g < C::TN / 4; ++g) {
-            const int col = col0 + 32 * g;
-            float v[4];
+        for (int g = 0; g < C::TN / C::V; ++g) {
+            const int col = col0 + 8 * C::V * g;
+            float v[C::V];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) v[e] = __fmul_rn(acc[i][4 * g + e], p.alpha);
-            if (p.vec_c && col + 3 < p.n) {
-                float4* dst = reinterpret_cast<float4*>(crow + col);
+            for (int e = 0; e < C::V; ++e) v[e] = __fmul_rn(acc[i][C::V * g + e], p.alpha);
+            if (p.vec_c && col + C::V - 1 < p.n) {
                 if (p.beta != 0.0f) {
-                    const float4 o = *dst;
-                    v[0] = fmaf(o.x, p.beta, v[0]);
-                    v[1] = fmaf(o.y, p.beta, v[1]);
-                    v[2] = fmaf(o.z, p.beta, v[2]);
-                    v[3] = fmaf(o.w, p.beta, v[3]);
+                    float o[C::V];
+                    load_vec<C::V>(crow + col, o);
+#pragma unroll
+                    for (int e = 0; e < C::V; ++e) v[e] = fmaf(o[e], p.beta, v[e]);
                 }
-                *dst = make_float4(v[0], v[1], v[2], v[3]);
+                store_vec<C::V>(crow + col, v);
             } else {
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
+                for (int e = 0; e < C::V; ++e) {
                     if (col + e < p.n) {
                         float out = v[e];
                         if (p.beta != 0.0f) out = fmaf(crow[col + e], p.beta, out);
@@ -287,25 +339,23 @@ __device__ __forceinline__ void epilogue_batched(const Operands& op, int m0, int
     // a private copy: the problem description may sit in global memory, where
     // each store to C would otherwise force it to be read again
     const Operands p = op;
-    const int col0 = n0 + wn * 8 * C::TN + ln * 4;
+    const int col0 = n0 + wn * 8 * C::TN + ln * C::V;
     // rows per chunk: the chunk's BATCH old C values live in registers
     constexpr int RC = BATCH / C::TN > 0 ? BATCH / C::TN : 1;
 #pragma unroll
     for (int i0 = 0; i0 < C::TM; i0 += RC) {
-        float4 old[RC][C::TN / 4];
+        float old[RC][C::TN];
         if (p.beta != 0.0f) {
 #pragma unroll
             for (int ii = 0; ii < RC; ++ii) {
                 const int i = i0 + ii;
                 if (i >= C::TM) break;
-                const int row = m0 + wm * C::WROWS + lm + 4 * i;
+                const int row = m0 + wm * C::WROWS + C::row(lm, i);
 #pragma unroll
-                for (int g = 0; g < C::TN / 4; ++g) {
-                    const int col = col0 + 32 * g;
-                    old[ii][g] = make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (row < p.m && p.vec_c && col + 3 < p.n)
-                        old[ii][g] = *reinterpret_cast<const float4*>(p.C + (int64_t)row * p.ldc +
-                                                                      col);
+                for (int g = 0; g < C::TN / C::V; ++g) {
+                    const int col = col0 + 8 * C::V * g;
+                    if (row < p.m && p.vec_c && col + C::V - 1 < p.n)
+                        load_vec<C::V>(p.C + (int64_t)row * p.ldc + col, &old[ii][C::V * g]);
                 }
             }
         }
@@ -313,27 +363,25 @@ __device__ __forceinline__ void epilogue_batched(const Operands& op, int m0, int
         for (int ii = 0; ii < RC; ++ii) {
             const int i = i0 + ii;
             if (i >= C::TM) break;
-            const int row = m0 + wm * C::WROWS + lm + 4 * i;
+            const int row = m0 + wm * C::WROWS + C::row(lm, i);
             if (row >= p.m) continue;
             float* crow = p.C + (int64_t)row * p.ldc;
 #pragma unroll
-            for (int g = 0; g < C::TN / 4; ++g) {
-                const int col = col0 + 32 * g;
-                float v[4];
+            for (int g = 0; g < C::TN / C::V; ++g) {
+                const int col = col0 + 8 * C::V * g;
+                float v[C::V];
 #pragma unroll
-                for (int e = 0; e < 4; ++e) v[e] = __fmul_rn(acc[i][4 * g + e], p.alpha);
-                if (p.vec_c && col + 3 < p.n) {
+                for (int e = 0; e < C::V; ++e) v[e] = __fmul_rn(acc[i][C::V * g + e], p.alpha);
+                if (p.vec_c && col + C::V - 1 < p.n) {
                     if (p.beta != 0.0f) {
-                        const float4 o = old[ii][g];
-                        v[0] = fmaf(o.x, p.beta, v[0]);
-                        v[1] = fmaf(o.y, p.beta, v[1]);
-                        v[2] = fmaf(o.z, p.beta, v[2]);
-                        v[3] = fmaf(o.w, p.beta, v[3]);
+#pragma unroll
+                        for (int e = 0; e < C::V; ++e)
+                            v[e] = fmaf(old[ii][C::V * g + e], p.beta, v[e]);
                     }
-                    *reinterpret_cast<float4*>(crow + col) = make_float4(v[0], v[1], v[2], v[3]);
+                    store_vec<C::V>(crow + col, v);
                 } else {
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) {
+                    for (int e = 0; e < C::V; ++e) {
                         if (col + e < p.n) {
                             float out = v[e];
                             if (p.beta != 0.0f) out = fmaf(crow[col + e], p.beta, out);
@@ -370,47 +418,32 @@ __device__ __forceinline__ void epilogue_staged(const Operands& p, int m0, int n
                                                 const float (&acc)[C::TM][C::TN], uint8_t* smem) {
     constexpr int W = 8 * C::TN;  // columns of a warp's tile
     constexpr int LD = W + 8;     // row pitch: 8 banks between rows, conflict-free float4 stores
-    static_assert((C::COMPUTE_THREADS / 32) * C::WROWS * LD * 4 <= C::STAGES * C::STAGE_BYTES,
+    static_assert((C::COMPUTE_THREADS / 32) * C::WROWS * LD * 4 <= C::RING_BYTES,
                   "the staged tile fits in the stage ring");
     float* buf = reinterpret_cast<float*>(smem) + warp * C::WROWS * LD;
 #pragma unroll
     for (int i = 0; i < C::TM; ++i)
 #pragma unroll
-        for (int g = 0; g < C::TN / 4; ++g)
-            *reinterpret_cast<float4*>(buf + (lm + 4 * i) * LD + 4 * ln + 32 * g) =
-                make_float4(acc[i][4 * g], acc[i][4 * g + 1], acc[i][4 * g + 2], acc[i][4 * g + 3]);
+        for (int g = 0; g < C::TN / C::V; ++g)
+            store_vec<C::V>(buf + C::row(lm, i) * LD + C::V * (ln + 8 * g), &acc[i][C::V * g]);
     __syncwarp();
     const int col0 = n0 + wn * W;
-    if constexpr (BATCH == 0) {  // one row at a time
-        for (int r = 0; r < C::WROWS; ++r) {
-            const int row = m0 + wm * C::WROWS + r;
-            if (row >= p.m) break;
-            float* crow = p.C + (int64_t)row * p.ldc;
-#pragma unroll
-            for (int t = 0; t < W / 32; ++t) {
-                const int col = col0 + lane + 32 * t;
-                if (col < p.n) {
-                    float v = __fmul_rn(buf[r * LD + lane + 32 * t], p.alpha);
-                    if (p.beta != 0.0f) v = fmaf(crow[col], p.beta, v);
-                    crow[col] = v;
-                }
-            }
-        }
-        return;
-    }
-    // rows in chunks of 8 whose C values are all loaded before the chunk's
-    // first store (see epilogue: one DRAM round trip per chunk, not per row)
-    constexpr int RC = 8;
-    for (int r0 = 0; r0 < C::WROWS; r0 += RC) {
-        float old[RC][W / 32];
+    // consecutive lanes on consecutive columns: a row per step, or two 16-column rows
+    constexpr int LPR = W < 32 ? W : 32, RPS = 32 / LPR, T = W / LPR;
+    const int lr = lane / LPR, lc = lane % LPR;
+    // steps in chunks whose C values are all loaded before the chunk's first
+    // store (see epilogue: one DRAM round trip per chunk, not per row)
+    constexpr int RC = BATCH == 0 ? 1 : 8;
+    for (int r0 = 0; r0 < C::WROWS; r0 += RC * RPS) {
+        float old[RC][T];
         if (p.beta != 0.0f) {
 #pragma unroll
             for (int rr = 0; rr < RC; ++rr) {
-                const int row = m0 + wm * C::WROWS + r0 + rr;
+                const int r = r0 + rr * RPS + lr, row = m0 + wm * C::WROWS + r;
 #pragma unroll
-                for (int t = 0; t < W / 32; ++t) {
-                    const int col = col0 + lane + 32 * t;
-                    old[rr][t] = (r0 + rr < C::WROWS && row < p.m && col < p.n)
+                for (int t = 0; t < T; ++t) {
+                    const int col = col0 + lc + LPR * t;
+                    old[rr][t] = (r < C::WROWS && row < p.m && col < p.n)
                                      ? p.C[(int64_t)row * p.ldc + col]
                                      : 0.0f;
                 }
@@ -418,15 +451,14 @@ __device__ __forceinline__ void epilogue_staged(const Operands& p, int m0, int n
         }
 #pragma unroll
         for (int rr = 0; rr < RC; ++rr) {
-            const int r = r0 + rr;
-            const int row = m0 + wm * C::WROWS + r;
+            const int r = r0 + rr * RPS + lr, row = m0 + wm * C::WROWS + r;
             if (r >= C::WROWS || row >= p.m) break;
             float* crow = p.C + (int64_t)row * p.ldc;
 #pragma unroll
-            for (int t = 0; t < W / 32; ++t) {
-                const int col = col0 + lane + 32 * t;
+            for (int t = 0; t < T; ++t) {
+                const int col = col0 + lc + LPR * t;
                 if (col < p.n) {
-                    float v = __fmul_rn(buf[r * LD + lane + 32 * t], p.alpha);
+                    float v = __fmul_rn(buf[r * LD + lc + LPR * t], p.alpha);
                     if (p.beta != 0.0f) v = fmaf(old[rr][t], p.beta, v);
                     crow[col] = v;
                 }
@@ -438,7 +470,7 @@ __device__ __forceinline__ void epilogue_staged(const Operands& p, int m0, int n
 // Barrier over the compute warps only (the producer warp, if any, has left).
 template <class C>
 __device__ __forceinline__ void compute_barrier() {
-    if constexpr (C::PRODUCER)
+    if constexpr (C::TMA)
         asm volatile("bar.sync 1, %0;" ::"n"(C::COMPUTE_THREADS) : "memory");
     else
         __syncthreads();
@@ -484,35 +516,28 @@ template <class C, bool STORE>
 __device__ __forceinline__ void acc_move(const Operands& p, const float* in, float* out, int ld,
                                          int m0, int n0, int wm, int wn, int lm, int ln,
                                          float (&acc)[C::TM][C::TN]) {
-    const int col0 = n0 + wn * 8 * C::TN + ln * 4;
+    const int col0 = n0 + wn * 8 * C::TN + ln * C::V;
 #pragma unroll
     for (int i = 0; i < C::TM; ++i) {
-        const int row = m0 + wm * C::WROWS + lm + 4 * i;
+        const int row = m0 + wm * C::WROWS + C::row(lm, i);
         if (row >= p.m) continue;
 #pragma unroll
-        for (int g = 0; g < C::TN / 4; ++g) {
-            const int col = col0 + 32 * g;
+        for (int g = 0; g < C::TN / C::V; ++g) {
+            const int col = col0 + 8 * C::V * g;
             const int64_t off = (int64_t)row * ld + col;
-            if (col + 3 < p.n) {
-                if constexpr (STORE) {
-                    *reinterpret_cast<float4*>(out + off) =
-                        make_float4(acc[i][4 * g], acc[i][4 * g + 1], acc[i][4 * g + 2],
-                                    acc[i][4 * g + 3]);
-                } else {
-                    const float4 v = *reinterpret_cast<const float4*>(in + off);
-                    acc[i][4 * g] = v.x;
-                    acc[i][4 * g + 1] = v.y;
-                    acc[i][4 * g + 2] = v.z;
-                    acc[i][4 * g + 3] = v.w;
-                }
+            if (col + C::V - 1 < p.n) {
+                if constexpr (STORE)
+                    store_vec<C::V>(out + off, &acc[i][C::V * g]);
+                else
+                    load_vec<C::V>(in + off, &acc[i][C::V * g]);
             } else {
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
+                for (int e = 0; e < C::V; ++e) {
                     if (col + e < p.n) {
                         if constexpr (STORE)
-                            out[off + e] = acc[i][4 * g + e];
+                            out[off + e] = acc[i][C::V * g + e];
                         else
-                            acc[i][4 * g + e] = in[off + e];
+                            acc[i][C::V * g + e] = in[off + e];
                     }
                 }
             }
@@ -536,27 +561,29 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
     ffma_gemm_kernel(const __grid_constant__ CUtensorMap tmA,
                      const __grid_constant__ CUtensorMap tmB, const Params p) {
     extern __shared__ uint8_t smem_raw[];
-    __shared__ __align__(8) uint64_t full_bar[C::STAGES];
-    __shared__ __align__(8) uint64_t empty_bar[C::PRODUCER ? C::STAGES : 1];
     uint8_t* smem = align_smem_1024(smem_raw);
 
     const int tid = threadIdx.x;
     const int warp = tid >> 5, lane = tid & 31;
+    int tm, tn;
+    tile_coords(blockIdx.x, p.tiles_m, p.tiles_n, tm, tn);
+    const int m0 = tm * C::BM, n0 = tn * C::BN;
+    const int nk = (p.op.k + C::BK - 1) / C::BK;
 
-    if constexpr (C::PRODUCER) {
-        int tm, tn;
-        tile_coords(blockIdx.x, p.tiles_m, p.tiles_n, tm, tn);
-        const int nk = (p.op.k + C::BK - 1) / C::BK;
+    if constexpr (C::TMA) {
+        constexpr int NW = C::WM * C::WN;
+        __shared__ __align__(8) uint64_t full_bar[C::STAGES];
+        __shared__ __align__(8) uint64_t empty_bar[C::STAGES];
         if (tid == 0) {
             for (int s = 0; s < C::STAGES; ++s) {
                 mbar_init(&full_bar[s], 1);
-                mbar_init(&empty_bar[s], C::WM * C::WN);  // one arrival per compute warp
+                mbar_init(&empty_bar[s], NW);  // one arrival per compute warp
             }
             fence_barrier_init();
         }
         __syncthreads();  // the only CTA-wide barrier: barriers initialised
         grid_wait();
-        if (warp == C::WM * C::WN) {
+        if (warp == NW) {
             // ------------------------------------------------ TMA producer --
             if (lane == 0 && nk > 0) {
                 tma_prefetch_desc(&tmA);
@@ -564,37 +591,36 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
                 int kb = 0;
                 for (; kb < nk; ++kb) {
                     const int s = kb % C::STAGES;
-                    if (kb >= C::STAGES &&
-                        !mbar_wait(&empty_bar[s], ((kb / C::STAGES) - 1) & 1)) {
-                        atomicExch(p.status, SGEMM_B200_ERR_TIMEOUT);
-                        break;
+                    if (kb >= C::STAGES) {
+                        if (!mbar_wait(&empty_bar[s], ((kb / C::STAGES) - 1) & 1)) break;
+                        // The compute warps' generic-proxy reads of the stage,
+                        // acquired through the empty barrier, before the
+                        // async-proxy (TMA) writes that refill it.  Without this
+                        // fence a warp of the 28 x 256 tile occasionally took one
+                        // k block's products from the refill (one warp's 28 x 32
+                        // patch of C wrong, under concurrent launches on a B200).
+                        fence_proxy_async_shared();
                     }
-                    // The compute warps' generic-proxy reads of the stage,
-                    // acquired through the empty barrier, before the
-                    // async-proxy (TMA) writes that refill it.  Without this
-                    // fence a warp of the 28 x 256 tile occasionally took one
-                    // k block's products from the refill (one warp's 28 x 32
-                    // patch of C wrong, under concurrent launches on a B200).
-                    if (kb >= C::STAGES) fence_proxy_async_shared();
                     uint8_t* st = smem + s * C::STAGE_BYTES;
                     mbar_arrive_expect_tx(&full_bar[s], C::STAGE_TX);
-                    tma_load_2d(st, &tmA, &full_bar[s], kb * C::BK, tm * C::BM);
-                    tma_load_2d(st + C::A_BYTES, &tmB, &full_bar[s], tn * C::BN, kb * C::BK);
+                    if constexpr (C::KM)
+                        tma_load_2d(st, &tmA, &full_bar[s], tm * C::A_BOX, kb * C::BK);
+                    else
+                        tma_load_2d(st, &tmA, &full_bar[s], kb * C::BK, m0);
+                    tma_load_2d(st + C::A_BYTES, &tmB, &full_bar[s], n0, kb * C::BK);
                 }
+                if (kb < nk) atomicExch(p.status, SGEMM_B200_ERR_TIMEOUT);
                 // Copies still in flight land before the CTA's smem is released
                 // (the compute warps may have given up on a stage).
-                for (int j = (kb > C::STAGES ? kb - C::STAGES : 0); j < kb; ++j)
+                for (int j = max(0, kb - C::STAGES); j < kb; ++j)
                     if (!mbar_wait(&full_bar[j % C::STAGES], (j / C::STAGES) & 1)) break;
             }
             return;
         }
         const int wm = warp / C::WN, wn = warp % C::WN;
         int lm, ln;
-        lane_coords(lane, lm, ln);
-        const int m0 = tm * C::BM, n0 = tn * C::BN;
-        uint32_t a_base, xa0, xa1;
-        a_coords<C>(wm, lm, a_base, xa0, xa1);
-        const uint32_t b_base = static_cast<uint32_t>((wn * 8 * C::TN + ln * 4) * 4);
+        C::lane_coords(lane, lm, ln);
+        const uint32_t b_base = static_cast<uint32_t>((wn * 8 * C::TN + ln * C::V) * 4);
         float acc[C::TM][C::TN];
 #pragma unroll
         for (int i = 0; i < C::TM; ++i)
@@ -602,6 +628,8 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
             for (int j = 0; j < C::TN; ++j) acc[i][j] = 0.0f;
         if (p.acc_in)
             acc_move<C, false>(p.op, p.acc_in, nullptr, p.ld_acc, m0, n0, wm, wn, lm, ln, acc);
+        uint32_t a_base = 0, xa0 = 0, xa1 = 0;  // A's offsets when it stays [row][k]
+        if constexpr (!C::KM) a_coords<C>(wm, lm, a_base, xa0, xa1);
         for (int kb = 0; kb < nk; ++kb) {
             const int s = kb % C::STAGES;
             if (!mbar_wait(&full_bar[s], (kb / C::STAGES) & 1)) {
@@ -609,88 +637,30 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
                 return;
             }
             const uint8_t* st = smem + s * C::STAGE_BYTES;
-            compute_stage<C>(st, st + C::A_BYTES, a_base, xa0, xa1, b_base, acc);
+            if constexpr (C::KM)
+                compute_stage_kmajor<C>(st, st + C::A_BYTES, wm, lm, b_base, acc);
+            else
+                compute_stage<C>(st, st + C::A_BYTES, a_base, xa0, xa1, b_base, acc);
             __syncwarp();
             if (lane == 0) mbar_arrive(&empty_bar[s]);  // this warp is done with the stage
         }
         finish_tile<C>(p, m0, n0, wm, wn, lm, ln, acc, smem);
-        return;
-    }
-
-    grid_wait();
-    const int wm = warp / C::WN, wn = warp % C::WN;
-    int lm, ln;
-    lane_coords(lane, lm, ln);
-
-    int tm, tn;
-    tile_coords(blockIdx.x, p.tiles_m, p.tiles_n, tm, tn);
-    const int m0 = tm * C::BM, n0 = tn * C::BN;
-    const int nk = (p.op.k + C::BK - 1) / C::BK;
-
-    // Per-thread shared-memory offsets (bytes within a stage).
-    uint32_t a_base, xa0, xa1;
-    a_coords<C>(wm, lm, a_base, xa0, xa1);
-    const uint32_t b_base = static_cast<uint32_t>((wn * 8 * C::TN + ln * 4) * 4);
-
-    float acc[C::TM][C::TN];
-#pragma unroll
-    for (int i = 0; i < C::TM; ++i)
-#pragma unroll
-        for (int j = 0; j < C::TN; ++j) acc[i][j] = 0.0f;
-    if (p.acc_in)
-        acc_move<C, false>(p.op, p.acc_in, nullptr, p.ld_acc, m0, n0, wm, wn, lm, ln, acc);
-
-    if constexpr (C::LOADER == kLoaderTma) {
-        int issued = 0;
-        auto issue = [&](int kb) {
-            const int s = kb % C::STAGES;
-            uint8_t* st = smem + s * C::STAGE_BYTES;
-            mbar_arrive_expect_tx(&full_bar[s], C::STAGE_TX);
-            tma_load_2d(st, &tmA, &full_bar[s], kb * C::BK, m0);
-            tma_load_2d(st + C::A_BYTES, &tmB, &full_bar[s], n0, kb * C::BK);
-        };
-        if (tid == 0) {
-            for (int s = 0; s < C::STAGES; ++s) mbar_init(&full_bar[s], 1);
-            fence_barrier_init();
-            if (nk > 0) {
-                tma_prefetch_desc(&tmA);
-                tma_prefetch_desc(&tmB);
-            }
-        }
-        __syncthreads();
-        if (tid == 0) {
-            for (; issued < C::STAGES && issued < nk; ++issued) issue(issued);
-        }
-        int kb = 0;
-        bool failed = false;
-        for (; kb < nk; ++kb) {
-            const int s = kb % C::STAGES;
-            const bool ok = mbar_wait(&full_bar[s], (kb / C::STAGES) & 1);
-            if (__syncthreads_or(!ok)) {
-                failed = true;
-                break;
-            }
-            // Every thread finished block kb-1, so its stage ((kb-1) % STAGES,
-            // which is where block kb-1+STAGES == issued lands) may be refilled.
-            if (tid == 0 && kb > 0 && issued < nk) {
-                // every thread's generic-proxy reads of the stage (ordered by the
-                // barrier) before the async-proxy (TMA) writes that refill it
-                fence_proxy_async_shared();
-                issue(issued++);
-            }
-            const uint8_t* st = smem + s * C::STAGE_BYTES;
-            compute_stage<C>(st, st + C::A_BYTES, a_base, xa0, xa1, b_base, acc);
-        }
-        if (failed) {
-            if (tid == 0) {
-                atomicExch(p.status, SGEMM_B200_ERR_TIMEOUT);
-                // Let copies still in flight land before the CTA's smem is released.
-                for (int j = kb; j < issued; ++j)
-                    if (!mbar_wait(&full_bar[j % C::STAGES], (j / C::STAGES) & 1)) break;
-            }
-            return;
-        }
     } else {
+        grid_wait();
+        const int wm = warp / C::WN, wn = warp % C::WN;
+        int lm, ln;
+        C::lane_coords(lane, lm, ln);
+        // Per-thread shared-memory offsets (bytes within a stage).
+        uint32_t a_base, xa0, xa1;
+        a_coords<C>(wm, lm, a_base, xa0, xa1);
+        const uint32_t b_base = static_cast<uint32_t>((wn * 8 * C::TN + ln * C::V) * 4);
+        float acc[C::TM][C::TN];
+#pragma unroll
+        for (int i = 0; i < C::TM; ++i)
+#pragma unroll
+            for (int j = 0; j < C::TN; ++j) acc[i][j] = 0.0f;
+        if (p.acc_in)
+            acc_move<C, false>(p.op, p.acc_in, nullptr, p.ld_acc, m0, n0, wm, wn, lm, ln, acc);
 #pragma unroll
         for (int s = 0; s < C::STAGES - 1; ++s) {
             if (s < nk) {
@@ -712,9 +682,8 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
             compute_stage<C>(st, st + C::A_BYTES, a_base, xa0, xa1, b_base, acc);
         }
         cp_async_wait<0>();
+        finish_tile<C>(p, m0, n0, wm, wn, lm, ln, acc, smem);
     }
-
-    finish_tile<C>(p, m0, n0, wm, wn, lm, ln, acc, smem);
 }
 
 }  // namespace ffma

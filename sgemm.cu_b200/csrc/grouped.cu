@@ -50,11 +50,11 @@ using ffma::Operands;
 // only a few rows tall, whose rows a 64- or 128-row tile would mostly pad
 // with zeros.  3 stages fit 3 CTAs per SM, 4 stages fit 2.
 template <int S>
-using CfgT = ffma::Cfg<128, 64, 4, 1, 8, S, ffma::kLoaderTma, (S == 3 ? 3 : 2)>;  // 128 x 64
+using CfgT = ffma::Cfg<128, 64, 4, 1, 8, S, ffma::kLoaderAsync4, (S == 3 ? 3 : 2)>;  // 128 x 64
 template <int S>
-using CfgW = ffma::Cfg<64, 128, 2, 2, 8, S, ffma::kLoaderTma, (S == 3 ? 3 : 2)>;  // 64 x 128
+using CfgW = ffma::Cfg<64, 128, 2, 2, 8, S, ffma::kLoaderAsync4, (S == 3 ? 3 : 2)>;  // 64 x 128
 template <int S>
-using CfgS = ffma::Cfg<32, 128, 1, 4, 4, S, ffma::kLoaderTma, (S == 3 ? 3 : 2)>;  // 32 x 128
+using CfgS = ffma::Cfg<32, 128, 1, 4, 4, S, ffma::kLoaderAsync4, (S == 3 ? 3 : 2)>;  // 32 x 128
 
 constexpr int THREADS = 128;
 constexpr int SLOT_BYTES = 24 * 1024;  // 16 KB + 8 KB per 32-deep k block (4 + 16 KB skinny)
@@ -123,7 +123,7 @@ __device__ __forceinline__ bool run_item(const GParams& gp, const GProblem& pr, 
     const int warp = tid >> 5, lane = tid & 31;
     const int wm = warp / C::WN, wn = warp % C::WN;
     int lm, ln;
-    ffma::lane_coords(lane, lm, ln);
+    C::lane_coords(lane, lm, ln);
     const int m0 = it.m0, n0 = it.n0;
     const int nk = (pr.op.k + C::BK - 1) / C::BK;
     const int kb0 = it.ks * pr.kbps;
@@ -148,7 +148,7 @@ __device__ __forceinline__ bool run_item(const GParams& gp, const GProblem& pr, 
             const uint32_t gs = g + j;
             const int s = gs % S;
             uint8_t* st = smem + s * SLOT_BYTES;
-            mbar_arrive_expect_tx(&full_bar[s], C::STAGE_TX);
+            mbar_arrive_expect_tx(&full_bar[s], C::A_TX + C::B_BYTES);
             tma_load_2d(st, tmA, &full_bar[s], (kb0 + j) * C::BK, m0);
             tma_load_2d(st + C::A_BYTES, tmB, &full_bar[s], n0, (kb0 + j) * C::BK);
         };

@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB) texld_gemm_kernel(const P
     const int warp = tid >> 5, lane = tid & 31;
     const int wm = warp / C::WN, wn = warp % C::WN;
     int lm, ln;
-    ffma::lane_coords(lane, lm, ln);
+    C::lane_coords(lane, lm, ln);
     int tm, tn;
     ffma::tile_coords(blockIdx.x, p.tiles_m, p.tiles_n, tm, tn);
     const int m0 = tm * C::BM, n0 = tn * C::BN;

@@ -117,6 +117,31 @@ def test_seven_row_thread_tile_bit_exact(name, m, n, k, ldc, ab):
     _assert_equal(got, oracle.sgemm_basic(A, B, C, *ab, basic=False))
 
 
+@pytest.mark.parametrize("name", ["tma_128x64_w4_t8x8_s3", "tma_28x256_w4p_t7x8_s3",
+                                  "tma_64x64_w4_t8x4_at", "tma_32x64_w4_t4x4_at"])
+@pytest.mark.parametrize("m,n,k", [(1, 4, 4), (27, 260, 68), (29, 132, 64), (65, 68, 132),
+                                   (130, 516, 252)])
+def test_transposed_a_bit_exact(name, m, n, k):
+    # configurations that read A transposed, at the edges of the transpose's
+    # 64 x 64 tiles, of the 28-row slot groups and of the 32-deep k blocks
+    A, B, _ = _inputs(m, n, k, 11, 0)
+    C = np.full((m, n), np.nan, dtype=np.float32)  # beta == 0: C is never read
+    got = _run_ours(A, B, C, 1.5, 0.0, config=sg.config_names().index(name))
+    _assert_equal(got, oracle.sgemm_basic(A, B, np.zeros_like(C), 1.5, 0.0, basic=False))
+
+
+@pytest.mark.parametrize("m,n,k,pads", [(100, 2000, 777, (0, 0, 0)), (24, 1503, 1000, (0, 0, 1)),
+                                        (401, 399, 403, (0, 0, 0)), (700, 701, 703, (2, 3, 0)),
+                                        (300, 301, 299, (0, 0, 0))],
+                         ids=["a_only", "b_only", "both_small", "both_large", "in_place"])
+def test_unaligned_rows_below_the_large_tiles(m, n, k, pads):
+    # unaligned strides on the small-thread tiles: copied rows (A, B or both) from
+    # 317^3 of work, the 4-byte loader below
+    A, B, C = _inputs(m, n, k, 12, 0)
+    got = _run_ours(A, B, C, 1.5, 0.5, lds=(k + pads[0], n + pads[1], n + pads[2]))
+    _assert_equal(got, oracle.sgemm_basic(A, B, C, 1.5, 0.5, basic=False))
+
+
 @pytest.mark.parametrize("size,beta,want", [
     (1024, 0.0, "tma_28x256_w4p_t7x8_s4"),
     (1024, 0.5, "tma_28x256_w4p_t7x8_s4"),
