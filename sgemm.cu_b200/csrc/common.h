@@ -85,20 +85,30 @@ inline int div_up(int a, int b) { return (a + b - 1) / b; }
 // 64 x 64 tiles: 35 us per GEMM instead of 24.7 with the release at the
 // epilogue, 24 x 4096 x 4096 on 32 x 32 tiles 62 instead of 42 with it at the
 // start).
+// `cluster`: CTAs per thread-block cluster.
 template <class... P, class... A>
-inline cudaError_t launch_chained(void (*kernel)(P...), int grid, int threads, size_t smem,
-                                  cudaStream_t stream, A... args) {
+inline cudaError_t launch_chained_cluster(int cluster, void (*kernel)(P...), int grid, int threads,
+                                          size_t smem, cudaStream_t stream, A... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = cluster;
+    at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
+template <class... P, class... A>
+inline cudaError_t launch_chained(void (*kernel)(P...), int grid, int threads, size_t smem,
+                                  cudaStream_t stream, A... args) {
+    return launch_chained_cluster(1, kernel, grid, threads, smem, stream, args...);
 }
 
 }  // namespace sgb

@@ -406,6 +406,14 @@ static int launch_config(int cfg, int m, int n, int k, float alpha, const float*
 }
 
 
+int plain_pack_rows(int a_rows, int a_cols, const float* A, int lda, float* A2, int lda2,
+                    int b_rows, int b_cols, const float* B, int ldb, float* B2, int ldb2,
+                    cudaStream_t stream) {
+    return cuda_status(ffma::prepare(ffma::TransposeJob{},
+                                     ffma::PackJob{A, A2, a_rows, a_cols, lda, lda2},
+                                     ffma::PackJob{B, B2, b_rows, b_cols, ldb, ldb2}, stream));
+}
+
 int plain_launch(int cfg, int m, int n, int k, float alpha, const float* A, int lda,
                  const float* B, int ldb, float beta, float* C, int ldc, cudaStream_t stream) {
     return plain_launch_acc(cfg, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, nullptr, nullptr,

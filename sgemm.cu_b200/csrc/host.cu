@@ -19,7 +19,7 @@
 // of it; the chunk widths come from a small timing model of this pipeline
 // (PCIe bandwidth and per-path GEMM rate measured on a B200), evaluated for
 // even and uneven splits per call.  Every block is the same GEMM on a sub-matrix, issued
-// through sgemm_b200_gemm(); each C element keeps its k-ordered accumulation,
+// as sgemm_b200_gemm() would; each C element keeps its k-ordered accumulation,
 // so the result is bit-identical to copying the whole matrices and calling the
 // device entry point once.
 //
@@ -33,6 +33,7 @@
 
 #include "common.h"
 #include "plain.h"
+#include "split.h"
 
 namespace sgb {
 namespace host {
@@ -451,9 +452,14 @@ static int run(int path, int m, int n, int k, const float* alpha, const float* A
             // Compute.
             if (k > 0 && !ok(cudaStreamWaitEvent(cs, eng->b_in[j], 0))) break;
             if (!ok(cudaStreamWaitEvent(cs, eng->in[blk], 0))) break;
-            const int g = sgemm_b200_gemm(path, nr, nc, k, alpha, dA + (size_t)r0 * lda_d, lda_d,
-                                          dB + c0, ldb_d, beta, dC + (size_t)r0 * ldc_d + c0,
-                                          ldc_d, reinterpret_cast<sgemm_b200_stream_t>(cs));
+            const float *bA = dA + (size_t)r0 * lda_d, *bB = dB + c0;
+            float* bC = dC + (size_t)r0 * ldc_d + c0;
+            const int g =
+                path == SGEMM_B200_PATH_PLAIN || k == 0
+                    ? sgemm_b200(nr, nc, k, alpha, bA, lda_d, bB, ldb_d, beta, bC, ldc_d,
+                                 reinterpret_cast<sgemm_b200_stream_t>(cs))
+                    : split::block_launch(path, m, n, nr, nc, k, *alpha, bA, lda_d, bB, ldb_d,
+                                          *beta, bC, ldc_d, cs);
             if (g != SGEMM_B200_OK) {
                 status = g;
                 break;

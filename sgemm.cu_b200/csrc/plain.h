@@ -22,4 +22,10 @@ int plain_launch_acc(int cfg, int m, int n, int k, float alpha, const float* A, 
                      const float* B, int ldb, float beta, float* C, int ldc, const float* acc_in,
                      float* acc_out, int ld_acc, cudaStream_t stream);
 
+// Copy rows of up to two matrices to other pitches in one launch (a_rows or b_rows
+// may be 0).
+int plain_pack_rows(int a_rows, int a_cols, const float* A, int lda, float* A2, int lda2,
+                    int b_rows, int b_cols, const float* B, int ldb, float* B2, int ldb2,
+                    cudaStream_t stream);
+
 }  // namespace sgb

@@ -58,6 +58,7 @@ constexpr int BM = 128, BN = 256;
 constexpr int DRAIN_WARPS = 8, PRODUCER_WARP = 8, MMA_WARP = 9;
 constexpr int THREADS = 32 * (DRAIN_WARPS + 2);
 constexpr int TMEM_COLS = 512;
+constexpr int PART_LD = BN + 1;  // row pitch of a slab's sums in shared memory
 constexpr int KCHUNK = 256;  // K depth D1 accumulates in the tensor core before a drain
 
 template <int PATH>
@@ -101,6 +102,7 @@ struct Layout {
     static constexpr int CHUNK_STEPS = KCHUNK / T::KMMA;    // k steps per D1 chunk
     static_assert(KCHUNK % T::BK == 0, "whole stages per chunk");
     static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
+    static_assert(BM * PART_LD * 4 <= T::STAGES * STAGE_BYTES, "a slab's sums fit the ring");
 };
 
 struct Params {
@@ -111,6 +113,7 @@ struct Params {
     int* status;
     int tiles_m, tiles_n;
     int vec_c;
+    int splits, blocks;  // k slabs (= cluster size), k blocks per slab
 };
 
 __device__ __forceinline__ void tile_coords(int bid, int tiles_m, int tiles_n, int& tm, int& tn) {
@@ -142,9 +145,11 @@ __global__ void __launch_bounds__(THREADS, 1)
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     int tm, tn;
-    tile_coords(blockIdx.x, p.tiles_m, p.tiles_n, tm, tn);
+    const int slab = blockIdx.x % p.splits;
+    tile_coords(blockIdx.x / p.splits, p.tiles_m, p.tiles_n, tm, tn);
     const int m0 = tm * BM, n0 = tn * BN;
-    const int nk = (p.k + T::BK - 1) / T::BK;
+    const int kb0 = slab * p.blocks;
+    const int nk = min(p.blocks, (p.k + T::BK - 1) / T::BK - kb0);  // k blocks of this slab
     const int nsteps = nk * L::STEPS;
     const int nchunks = (nsteps + L::CHUNK_STEPS - 1) / L::CHUNK_STEPS;
 
@@ -168,6 +173,8 @@ __global__ void __launch_bounds__(THREADS, 1)
     tc_fence_after();
     const uint32_t tmem = tmem_base_s;
 
+    grid_wait();
+
     int issued = 0;
     if (warp == PRODUCER_WARP) {
         if (lane == 0) {
@@ -185,8 +192,8 @@ __global__ void __launch_bounds__(THREADS, 1)
                 }
                 uint8_t* st = smem + s * L::STAGE_BYTES;
                 mbar_arrive_expect_tx(&full_bar[s], L::STAGE_BYTES);
-                tma_load_3d(st, &tmA, &full_bar[s], kb * T::BK, m0, 0);
-                tma_load_3d(st + L::A_BYTES, &tmB, &full_bar[s], kb * T::BK, n0, 0);
+                tma_load_3d(st, &tmA, &full_bar[s], (kb0 + kb) * T::BK, m0, 0);
+                tma_load_3d(st + L::A_BYTES, &tmB, &full_bar[s], (kb0 + kb) * T::BK, n0, 0);
                 ++issued;
             }
         }
@@ -282,6 +289,19 @@ __global__ void __launch_bounds__(THREADS, 1)
         if (!ok) {
             abort_s = 1;
             atomicExch(p.status, SGEMM_B200_ERR_TIMEOUT);
+        } else if (!abort_s && p.splits > 1) {
+            // The slab's sums, to meet the other slabs' in shared memory (the stage
+            // ring, every MMA being done): [row][PART_LD].
+            float* part = reinterpret_cast<float*>(smem) + (q * 32 + lane) * PART_LD + h * 128;
+#pragma unroll
+            for (int g = 0; g < 4; ++g) {
+                uint32_t r[32];
+                tmem_ld_32x32b_x32(trow + BN + g * 32, r);
+                tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < 32; ++j)
+                    part[g * 32 + j] = __fadd_rn(acc[g * 32 + j], __uint_as_float(r[j]));
+            }
         } else if (!abort_s) {
             // D2 is complete: the last D1 commit came after every MMA.
             const int row = m0 + q * 32 + lane;
@@ -328,6 +348,28 @@ __global__ void __launch_bounds__(THREADS, 1)
         }
     }
 
+    if (p.splits > 1) {
+        // Every CTA of the cluster adds its share of the rows over the slabs, in
+        // slab order, as split_fused_kernel does.
+        cluster_sync_all();
+        if (!abort_s && warp < DRAIN_WARPS) {
+            const int share = (BM + p.splits - 1) / p.splits;
+            const int rend = min(min(BM, p.m - m0), (slab + 1) * share);
+            for (int r = slab * share + warp; r < rend; r += DRAIN_WARPS) {
+                float* crow = p.C + (int64_t)(m0 + r) * p.ldc + n0;
+                for (int c = lane; c < BN && n0 + c < p.n; c += 32) {
+                    const uint32_t at =
+                        smem_u32(smem) + static_cast<uint32_t>(r * PART_LD + c) * 4;
+                    float v = ld_cluster_f1(at, 0);
+                    for (int s = 1; s < p.splits; ++s) v = __fadd_rn(v, ld_cluster_f1(at, s));
+                    v = __fmul_rn(v, p.alpha);
+                    crow[c] = p.beta != 0.0f ? fmaf(crow[c], p.beta, v) : v;
+                }
+            }
+        }
+        cluster_sync_all();  // peers have read this CTA's sums
+    }
+
     // ------------------------------------------------------------ teardown --
     tc_fence_before();
     __syncthreads();  // every TMEM load and MMA is done; consumed_s is visible
@@ -368,6 +410,8 @@ __device__ __forceinline__ void split_value(float x, float (&out)[3]) {
         out[2] = 0.0f;
     }
 }
+
+#include "split_fused.cuh"
 
 // Store 8 consecutive split values (one per plane) as 16-byte vectors.
 template <int PATH>
@@ -414,6 +458,7 @@ __device__ __forceinline__ void split_a_chunk(const float* __restrict__ A, int m
 template <int PATH>
 __global__ void split_a_kernel(const float* __restrict__ A, int m, int k, int lda, int kp,
                                uint8_t* __restrict__ out) {
+    grid_wait();
     const int64_t total = (int64_t)m * (kp / 8);
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total;
          i += (int64_t)gridDim.x * blockDim.x)
@@ -455,6 +500,7 @@ template <int PATH>
 __global__ void split_bt_kernel(const float* __restrict__ B, int k, int n, int ldb, int kp,
                                 uint8_t* __restrict__ out, int tiles_n, int tiles) {
     __shared__ float tile[64][65];
+    grid_wait();
     for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
         split_bt_tile<PATH>(B, k, n, ldb, kp, out, t % tiles_n, t / tiles_n, tile);
         __syncthreads();  // the next tile's loads overwrite `tile`
@@ -469,12 +515,16 @@ static size_t workspace_bytes(int m, int n, int k, size_t* a_bytes_out = nullptr
     const size_t b = (size_t)T::NSPLIT * n * kp * T::ESZ;
     const size_t a_al = (a + 1023) / 1024 * 1024;
     if (a_bytes_out) *a_bytes_out = a_al;
-    return a_al + b + 1024;  // + alignment slack for the base
+    // planes, or copies of the operands at 16-byte-aligned rows (the larger only for
+    // a few columns); + alignment slack for the base
+    const size_t rows = sizeof(float) * ((size_t)m * ((k + 3) / 4 * 4) +
+                                         (size_t)k * ((n + 3) / 4 * 4));
+    return std::max(a_al + b, rows) + 1024;
 }
 
 template <int PATH>
 static int launch(int m, int n, int k, float alpha, const float* A, int lda, const float* B,
-                  int ldb, float beta, float* C, int ldc, void* ws, size_t ws_bytes,
+                  int ldb, float beta, float* C, int ldc, int splits, void* ws, size_t ws_bytes,
                   cudaStream_t stream) {
     using T = Traits<PATH>;
     using L = Layout<PATH>;
@@ -489,13 +539,15 @@ static int launch(int m, int n, int k, float alpha, const float* A, int lda, con
 
     {
         const int64_t total = (int64_t)m * (kp / 8);
-        int64_t blocks = (total + 255) / 256;
-        if (blocks > 148 * 32) blocks = 148 * 32;
-        split_a_kernel<PATH><<<(int)blocks, 256, 0, stream>>>(A, m, k, lda, kp, wa);
+        const int blocks = (int)std::min<int64_t>((total + 255) / 256, 148 * 32);
         const int tiles_n = div_up(n, 64), tiles = tiles_n * div_up(kp, 64);
         const int sms = device_info().sm_count > 0 ? device_info().sm_count : 148;
-        split_bt_kernel<PATH><<<std::min(tiles, sms * 8), 256, 0, stream>>>(B, k, n, ldb, kp, wb,
-                                                                             tiles_n, tiles);
+        cudaError_t e =
+            launch_chained(split_a_kernel<PATH>, blocks, 256, 0, stream, A, m, k, lda, kp, wa);
+        if (e == cudaSuccess)
+            e = launch_chained(split_bt_kernel<PATH>, std::min(tiles, sms * 8), 256, 0, stream, B, k,
+                               n, ldb, kp, wb, tiles_n, tiles);
+        if (e != cudaSuccess) return cuda_status(e);
     }
 
     const CUtensorMapDataType dt =
@@ -542,9 +594,134 @@ static int launch(int m, int n, int k, float alpha, const float* A, int lda, con
             attr_set[dev].store(true, std::memory_order_release);
         }
     }
-    split_gemm_kernel<PATH><<<p.tiles_m * p.tiles_n, THREADS, L::SMEM_BYTES, stream>>>(tmA, tmB,
-                                                                                      p);
-    return cuda_status(cudaGetLastError());
+    p.splits = splits;
+    p.blocks = div_up(div_up(k, KCHUNK), splits) * (KCHUNK / T::BK);
+    return cuda_status(launch_chained_cluster(splits, split_gemm_kernel<PATH>,
+                                              p.tiles_m * p.tiles_n * splits, THREADS,
+                                              L::SMEM_BYTES, stream, tmA, tmB, p));
+}
+
+// How a problem is computed: `splits` k slabs whose sums are added in slab order,
+// and whether the fused kernel is the faster one for it.  A function of the path
+// and the sizes alone: every entry point, grouped launch and block of the host
+// pipeline gives a problem the same slabs, and so the same bits, whichever kernel
+// its strides and workspace allow.
+struct Route {
+    bool fused;
+    int splits;
+};
+
+// Modelled times in microseconds, from B200 timings.  Fused kernel: a block of 32
+// k takes a + b NT per CTA (NT rows of the tile), SMs take whole rounds of CTAs.
+// Pre-pass and 128 x 256 tiles: the planes' bytes, and 0.93 us (BF16X6) or 1.0 us
+// (TF32X3) per block of 32 k and round.
+static Route route(int path, int m, int n, int k) {
+    const bool bf = path == SGEMM_B200_PATH_BF16X6;
+    const double sms = 148;
+    const int tiles_m = div_up(m, fused::NT_MAX), nt = div_up(div_up(m, tiles_m), 16) * 16;
+    const int tiles = tiles_m * div_up(n, fused::TN), chunks = div_up(k, KCHUNK);
+    const double block = bf ? 0.43 + 0.0023 * nt : 0.58 + 0.0027 * nt;
+    Route best{true, 1};
+    double best_t = 1e300;
+    for (int s = 1; s <= 8; s *= 2) {
+        if (s > 1 && (div_up(chunks, s) * (s - 1) >= chunks || tiles * s > 148)) break;
+        const double t = 4.0 + (s > 1 ? 2.5 : 0.0) +
+                         std::ceil(tiles * s / sms) * div_up(chunks, s) * (KCHUNK / 32) * block;
+        if (t < best_t * 0.95) {
+            best_t = t;
+            best.splits = s;
+        }
+    }
+    const double planes = (double(m) + n) * k * (bf ? 10.0 : 12.0) / 4.5e6;
+    const double tiles256 = std::ceil(double(div_up(m, BM)) * div_up(n, BN) / sms);
+    const double t_planes = 10.0 + planes + tiles256 * div_up(k, 32) * (bf ? 0.93 : 1.0);
+    if (t_planes < best_t) best = Route{false, 1};
+    return best;
+}
+
+// Whether split_fused_kernel's TMA boxes can describe the operands.
+static bool fused_ok(const float* A, int lda, const float* B, int ldb) {
+    return lda % 4 == 0 && ldb % 4 == 0 && reinterpret_cast<uintptr_t>(A) % 16 == 0 &&
+           reinterpret_cast<uintptr_t>(B) % 16 == 0;
+}
+
+// The operands as the fused kernel reads them: in place, or copied to 16-byte
+// aligned rows in `ws` (the copy itself is the caller's) when their strides are
+// not ones TMA can describe.  bytes: of ws that the copies take, 0 in place.
+struct Packed {
+    const float *A, *B;
+    int lda, ldb;
+    bool pa, pb;
+    size_t bytes;
+};
+static Packed packed(int m, int n, int k, const float* A, int lda, const float* B, int ldb,
+                     void* ws) {
+    Packed p{A, B, lda, ldb, false, false, 0};
+    p.pa = lda % 4 != 0 || reinterpret_cast<uintptr_t>(A) % 16 != 0;
+    p.pb = ldb % 4 != 0 || reinterpret_cast<uintptr_t>(B) % 16 != 0;
+    float* base = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(ws) + 1023) &
+                                           ~static_cast<uintptr_t>(1023));
+    size_t floats = 0;
+    if (p.pa) {
+        p.lda = (k + 3) / 4 * 4;
+        p.A = base;
+        floats += (size_t)m * p.lda;
+    }
+    if (p.pb) {
+        p.ldb = (n + 3) / 4 * 4;
+        p.B = base + floats;
+        floats += (size_t)k * p.ldb;
+    }
+    if (floats) p.bytes = floats * sizeof(float) + 1024;
+    return p;
+}
+
+static bool fused_maps(int m, int n, int k, const float* A, int lda, const float* B, int ldb,
+                       int nt, CUtensorMap* ma, CUtensorMap* mb) {
+    return encode_tensor_map_2d(ma, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, A, (uint64_t)k, (uint64_t)m,
+                                (uint64_t)lda * 4, fused::BK, nt, CU_TENSOR_MAP_SWIZZLE_128B) &&
+           encode_tensor_map_2d(mb, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, B, (uint64_t)n, (uint64_t)k,
+                                (uint64_t)ldb * 4, fused::TN, fused::BK,
+                                CU_TENSOR_MAP_SWIZZLE_NONE);
+}
+
+template <int PATH>
+static int launch_fused(int m, int n, int k, float alpha, const float* A, int lda, const float* B,
+                        int ldb, float beta, float* C, int ldc, int splits, cudaStream_t stream) {
+    using L = fused::Lay<PATH>;
+    fused::Params p;
+    p.m = m;
+    p.n = n;
+    p.k = k;
+    p.ldc = ldc;
+    p.alpha = alpha;
+    p.beta = beta;
+    p.C = C;
+    p.status = device_status_ptr();
+    if (!p.status) return SGEMM_B200_ERR_CUDA;
+    p.tiles_m = div_up(m, fused::NT_MAX);
+    p.nt = div_up(div_up(m, p.tiles_m), 16) * 16;
+    p.splits = splits;
+    p.blocks = div_up(div_up(k, KCHUNK), splits) * fused::CHUNK_BLOCKS;
+    CUtensorMap tmA, tmB;
+    std::memset(&tmA, 0, sizeof(tmA));
+    std::memset(&tmB, 0, sizeof(tmB));
+    if (!fused_maps(m, n, k, A, lda, B, ldb, p.nt, &tmA, &tmB)) return SGEMM_B200_ERR_CUDA;
+    static std::atomic<bool> attr_set[64];
+    static std::mutex attr_mu;
+    const int dev = device_info().device;
+    if (dev < 0 || dev >= 64) return SGEMM_B200_ERR_CUDA;
+    if (!attr_set[dev].load(std::memory_order_acquire)) {
+        std::lock_guard<std::mutex> lock(attr_mu);
+        const cudaError_t e =
+            cudaFuncSetAttribute(fused::split_fused_kernel<PATH>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, L::SMEM);
+        if (e != cudaSuccess) return cuda_status(e);
+        attr_set[dev].store(true, std::memory_order_release);
+    }
+    const int grid = p.tiles_m * div_up(n, fused::TN) * splits;
+    return cuda_status(launch_chained_cluster(splits, fused::split_fused_kernel<PATH>, grid,
+                                              fused::THREADS, L::SMEM, stream, tmA, tmB, p));
 }
 
 // ------------------------------------------------------- grouped split GEMM --
@@ -626,6 +803,8 @@ __global__ void __launch_bounds__(THREADS, 1) split_grouped_kernel(const GSParam
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_base_s;
+
+    grid_wait();
 
     uint32_t issued = 0;
     if (warp == PRODUCER_WARP) {
@@ -849,10 +1028,13 @@ __global__ void __launch_bounds__(THREADS, 1) split_grouped_kernel(const GSParam
     }
 }
 
-// Grouped pre-pass: the A and B planes of many problems in one launch.
-// Blocks [0, a_blocks) split A chunks (256 chunks of 8 k-values per block),
-// blocks [a_blocks, a_blocks + b_blocks) transpose-and-split 64 x 64 tiles of
-// B; a block finds its problem by binary search over the prefix sums.
+// Grouped pre-pass: the A and B planes of many problems in one launch, and the
+// row copies of those whose strides the fused kernel's TMA cannot describe.
+// Blocks [0, a_blocks) split A chunks (256 chunks of 8 k-values per block), the
+// next b_blocks transpose-and-split 64 x 64 tiles of B, the rest copy rows of A
+// and B to 16-byte-aligned rows (PACK_ROWS each); a block finds its problem by
+// binary search over the prefix sums.
+constexpr int PACK_ROWS = 8;
 struct PrepJob {
     const float* A;
     const float* B;
@@ -863,28 +1045,55 @@ struct PrepJob {
     int pad;
 };
 
+struct PackJob {
+    const float* A;
+    const float* B;
+    float* a2;
+    float* b2;
+    int m, n, k, lda, ldb, lda2, ldb2;
+    int a_rows;  // m, or 0 when A is read in place; likewise b_rows
+    int b_rows;
+    int pad;
+};
+
 struct PrepParams {
     const PrepJob* jobs;
+    const PackJob* packs;
     const int* a_prefix;  // n_jobs + 1 entries
     const int* b_prefix;
-    int n_jobs;
-    int a_blocks;
+    const int* p_prefix;  // n_packs + 1 entries
+    int n_jobs, n_packs;
+    int a_blocks, b_blocks;
 };
 
 template <int PATH>
 __global__ void __launch_bounds__(256) split_prepass_grouped_kernel(const PrepParams pp) {
     __shared__ float tile[64][65];
+    grid_wait();
     int b = blockIdx.x;
-    const bool is_a = b < pp.a_blocks;
-    const int* pref = is_a ? pp.a_prefix : pp.b_prefix;
-    if (!is_a) b -= pp.a_blocks;
-    int lo = 0, hi = pp.n_jobs - 1;  // the last job whose first block is <= b
+    const bool is_a = b < pp.a_blocks, is_p = b >= pp.a_blocks + pp.b_blocks;
+    const int* pref = is_a ? pp.a_prefix : is_p ? pp.p_prefix : pp.b_prefix;
+    b -= is_a ? 0 : is_p ? pp.a_blocks + pp.b_blocks : pp.a_blocks;
+    int lo = 0, hi = (is_p ? pp.n_packs : pp.n_jobs) - 1;  // the last job whose first block is <= b
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
         if (pref[mid] <= b)
             lo = mid;
         else
             hi = mid - 1;
+    }
+    if (is_p) {
+        const PackJob& j = pp.packs[lo];
+        const int r0 = (b - pref[lo]) * PACK_ROWS;
+        for (int r = r0; r < min(r0 + PACK_ROWS, j.a_rows + j.b_rows); ++r) {
+            const bool in_a = r < j.a_rows;
+            const float* src = in_a ? j.A + (int64_t)r * j.lda
+                                    : j.B + (int64_t)(r - j.a_rows) * j.ldb;
+            float* dst = in_a ? j.a2 + (int64_t)r * j.lda2
+                              : j.b2 + (int64_t)(r - j.a_rows) * j.ldb2;
+            for (int c = threadIdx.x; c < (in_a ? j.k : j.n); c += 256) dst[c] = src[c];
+        }
+        return;
     }
     const PrepJob& j = pp.jobs[lo];
     const int local = b - pref[lo];
@@ -902,8 +1111,16 @@ __global__ void __launch_bounds__(256) split_prepass_grouped_kernel(const PrepPa
 
 // Host copy of a grouped launch's tables, laid out as one blob so one copy
 // moves it to the device: problems | tiles | tensor maps (64-byte aligned) |
-// pre-pass jobs | A prefix sums | B prefix sums.
+// pre-pass jobs | A prefix sums | B prefix sums, then the fused kernel's
+// problems | tiles | tensor maps.
 struct GroupedTables {
+    std::vector<fused::GProblem> fprobs;
+    std::vector<fused::GTile> ftiles;
+    std::vector<CUtensorMap> fmaps;
+    std::vector<PackJob> packs;
+    std::vector<int> p_prefix;
+    bool fsums = false;  // some fused problem has several slabs
+    size_t off_fprobs = 0, off_ftiles = 0, off_fmaps = 0, off_packs = 0, off_ppref = 0;
     std::vector<GSProblem> probs;
     std::vector<GSTile> tiles;
     std::vector<CUtensorMap> maps;
@@ -915,18 +1132,114 @@ struct GroupedTables {
 
 static size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
+// Which problems of a grouped launch the fused kernel computes (the others come
+// from planes; a problem of several slabs is always fused).  Modelled in
+// microseconds from B200 timings: a fused 128 x NT tile takes 0.43 + 0.0023 NT per
+// block of 32 k, a 128 x 256 one 0.93, a slab about 2 more, and the planes' bytes
+// occupy every SM.  The two kernels run one after the other, each as long as its
+// dearest tile or its share of the SMs, so it is either everything fused or every
+// problem on the kernel that takes it fewer SM-microseconds.
+static std::vector<char> grouped_classes(int path, const sgemm_b200_problem* pr, int count) {
+    const bool bf = path == SGEMM_B200_PATH_BF16X6;
+    struct Phase {
+        double work = 0, longest = 0;
+        void add(double tiles, double tile) {
+            work += tiles * tile;
+            longest = std::max(longest, tile);
+        }
+        double us() const { return std::max(work / 148.0, longest); }
+    };
+    std::vector<char> mixed(count, 0), all(count, 0);
+    Phase all_fused, some_fused, rest;
+    double planes = 0;
+    for (int i = 0; i < count; ++i) {
+        const sgemm_b200_problem& q = pr[i];
+        if (q.m <= 0 || q.n <= 0 || q.k <= 0) continue;
+        const int splits = route(path, q.m, q.n, q.k).splits;
+        const int tiles_m = div_up(q.m, fused::NT_MAX), nt = div_up(div_up(q.m, tiles_m), 16) * 16;
+        const double blocks = div_up(q.k, 32);
+        const double ft = blocks * (bf ? 0.43 + 0.0023 * nt : 0.5 + 0.0024 * nt) + 2.0 * splits;
+        const double f = double(tiles_m) * div_up(q.n, fused::TN);
+        const double pt = blocks * (bf ? 0.93 : 1.0) + 3.0;
+        const double p = double(div_up(q.m, BM)) * div_up(q.n, BN);
+        const double bytes = (double(q.m) + q.n) * q.k * (bf ? 10.0 : 12.0) / 4.5e6;
+        all[i] = 1;
+        all_fused.add(f, ft);
+        mixed[i] = splits > 1 || f * ft < p * pt + 148.0 * bytes;
+        if (mixed[i]) {
+            some_fused.add(f, ft);
+        } else {
+            rest.add(p, pt);
+            planes += bytes;
+        }
+    }
+    if (rest.work == 0) return all;
+    return all_fused.us() < some_fused.us() + rest.us() + planes + 10.0 ? all : mixed;
+}
+
+// One problem's entries for the fused grouped kernel.
 template <int PATH>
-static int grouped_tables(const sgemm_b200_problem* pr, void* const* ws, int count,
-                          GroupedTables* out) {
+static int add_fused(const sgemm_b200_problem& q, void* ws, int splits, GroupedTables* gt,
+                     std::vector<double>* cost) {
+    const Packed pk = packed(q.m, q.n, q.k, q.A, q.lda, q.B, q.ldb, ws);
+    if (pk.bytes) {
+        const int rows = (pk.pa ? q.m : 0) + (pk.pb ? q.k : 0);
+        gt->packs.push_back(PackJob{q.A, q.B, const_cast<float*>(pk.A), const_cast<float*>(pk.B),
+                                    q.m, q.n, q.k, q.lda, q.ldb, pk.lda, pk.ldb, pk.pa ? q.m : 0,
+                                    pk.pb ? q.k : 0, 0});
+        gt->p_prefix.push_back(gt->p_prefix.back() + div_up(rows, PACK_ROWS));
+    }
+    fused::GProblem g;
+    g.m = q.m;
+    g.n = q.n;
+    g.k = q.k;
+    g.ldc = q.ldc;
+    g.alpha = q.alpha;
+    g.beta = q.beta;
+    g.C = q.C;
+    g.pad = 0;
+    const int tiles_m = div_up(q.m, fused::NT_MAX);
+    g.nt = div_up(div_up(q.m, tiles_m), 16) * 16;
+    g.splits = splits;
+    g.blocks = div_up(div_up(q.k, KCHUNK), splits) * fused::CHUNK_BLOCKS;
+    CUtensorMap maps[2];
+    std::memset(maps, 0, sizeof(maps));
+    if (!fused_maps(q.m, q.n, q.k, pk.A, pk.lda, pk.B, pk.ldb, g.nt, &maps[0], &maps[1]))
+        return SGEMM_B200_ERR_CUDA;
+    const int idx = (int)gt->fprobs.size();
+    gt->fprobs.push_back(g);
+    gt->fmaps.push_back(maps[0]);
+    gt->fmaps.push_back(maps[1]);
+    gt->fsums = gt->fsums || splits > 1;
+    const double c = div_up(q.k, fused::BK) * (0.43 + 0.0023 * g.nt) + 2.0 * splits;
+    for (int b = 0; b < div_up(q.n, fused::TN); ++b)
+        for (int a = 0; a < tiles_m; ++a) {
+            gt->ftiles.push_back(fused::GTile{idx, a * g.nt, b * fused::TN, 0});
+            cost->push_back(c);
+        }
+    return SGEMM_B200_OK;
+}
+
+template <int PATH>
+static int grouped_tables(const sgemm_b200_problem* pr, void* const* ws,
+                          const std::vector<char>& fused, int count, GroupedTables* out) {
     using T = Traits<PATH>;
     GroupedTables gt;
+    std::vector<double> fcost;  // of each fused tile
     gt.a_prefix.push_back(0);
     gt.b_prefix.push_back(0);
+    gt.p_prefix.push_back(0);
     for (int i = 0; i < count; ++i) {
         const sgemm_b200_problem& q = pr[i];
         if (q.m == 0 || q.n == 0) continue;
         if (q.k == 0) {
             gt.k_zero.push_back(i);
+            continue;
+        }
+        if (fused[i]) {
+            const int splits = route(PATH, q.m, q.n, q.k).splits;
+            const int st = add_fused<PATH>(q, ws[i], splits, &gt, &fcost);
+            if (st != SGEMM_B200_OK) return st;
             continue;
         }
         size_t a_bytes = 0;
@@ -991,7 +1304,20 @@ static int grouped_tables(const sgemm_b200_problem* pr, void* const* ws, int cou
     gt.off_jobs = align_up(gt.off_maps + sizeof(CUtensorMap) * gt.maps.size(), 64);
     gt.off_apref = align_up(gt.off_jobs + sizeof(PrepJob) * gt.jobs.size(), 64);
     gt.off_bpref = align_up(gt.off_apref + sizeof(int) * gt.a_prefix.size(), 64);
-    gt.bytes = align_up(gt.off_bpref + sizeof(int) * gt.b_prefix.size(), 64);
+    // the fused tiles, dearest first
+    std::vector<int> order(gt.ftiles.size());
+    for (size_t i = 0; i < order.size(); ++i) order[i] = (int)i;
+    std::stable_sort(order.begin(), order.end(),
+                     [&](int x, int y) { return fcost[x] > fcost[y]; });
+    std::vector<fused::GTile> sorted(order.size());
+    for (size_t i = 0; i < order.size(); ++i) sorted[i] = gt.ftiles[order[i]];
+    gt.ftiles.swap(sorted);
+    gt.off_fprobs = align_up(gt.off_bpref + sizeof(int) * gt.b_prefix.size(), 64);
+    gt.off_ftiles = align_up(gt.off_fprobs + sizeof(fused::GProblem) * gt.fprobs.size(), 64);
+    gt.off_fmaps = align_up(gt.off_ftiles + sizeof(fused::GTile) * gt.ftiles.size(), 64);
+    gt.off_packs = align_up(gt.off_fmaps + sizeof(CUtensorMap) * gt.fmaps.size(), 64);
+    gt.off_ppref = align_up(gt.off_packs + sizeof(PackJob) * gt.packs.size(), 64);
+    gt.bytes = align_up(gt.off_ppref + sizeof(int) * gt.p_prefix.size(), 64);
     *out = std::move(gt);
     return SGEMM_B200_OK;
 }
@@ -1003,6 +1329,11 @@ static void pack_tables(const GroupedTables& gt, uint8_t* h) {
     std::memcpy(h + gt.off_jobs, gt.jobs.data(), sizeof(PrepJob) * gt.jobs.size());
     std::memcpy(h + gt.off_apref, gt.a_prefix.data(), sizeof(int) * gt.a_prefix.size());
     std::memcpy(h + gt.off_bpref, gt.b_prefix.data(), sizeof(int) * gt.b_prefix.size());
+    std::memcpy(h + gt.off_fprobs, gt.fprobs.data(), sizeof(fused::GProblem) * gt.fprobs.size());
+    std::memcpy(h + gt.off_ftiles, gt.ftiles.data(), sizeof(fused::GTile) * gt.ftiles.size());
+    std::memcpy(h + gt.off_fmaps, gt.fmaps.data(), sizeof(CUtensorMap) * gt.fmaps.size());
+    std::memcpy(h + gt.off_packs, gt.packs.data(), sizeof(PackJob) * gt.packs.size());
+    std::memcpy(h + gt.off_ppref, gt.p_prefix.data(), sizeof(int) * gt.p_prefix.size());
 }
 
 // The grouped kernel's shared-memory attribute, once per device.
@@ -1015,36 +1346,74 @@ static int set_grouped_attribute() {
     if (done[dev].load(std::memory_order_acquire)) return SGEMM_B200_OK;
     std::lock_guard<std::mutex> lock(mu);
     if (!done[dev].load(std::memory_order_relaxed)) {
-        const cudaError_t e =
+        cudaError_t e =
             cudaFuncSetAttribute(split_grouped_kernel<PATH>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  Layout<PATH>::SMEM_BYTES);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(fused::split_fused_grouped_kernel<PATH>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     fused::Lay<PATH>::SMEM);
         if (e != cudaSuccess) return cuda_status(e);
         done[dev].store(true, std::memory_order_release);
     }
     return SGEMM_B200_OK;
 }
 
-// Pre-pass and persistent kernel over the tables at device address d.
+// CTAs of the fused grouped kernel, and the bytes of slab sums a launch needs.
+static int fused_grid(const GroupedTables& gt) {
+    const int sms = device_info().sm_count > 0 ? device_info().sm_count : 148;
+    return std::min((int)gt.ftiles.size(), sms);
+}
+static size_t sums_bytes(const GroupedTables& gt) {
+    return gt.fsums ? sizeof(float) * fused::TN * fused::NT_MAX * fused_grid(gt) : 0;
+}
+
+// The persistent kernels (and the pre-pass) over the tables at device address d;
+// `sums`: sums_bytes of scratch.
 template <int PATH>
-static int grouped_enqueue(const GroupedTables& gt, const uint8_t* d, cudaStream_t stream) {
-    if (gt.tiles.empty()) return SGEMM_B200_OK;
+static int grouped_enqueue(const GroupedTables& gt, const uint8_t* d, float* sums,
+                           cudaStream_t stream) {
+    if (gt.tiles.empty() && gt.ftiles.empty()) return SGEMM_B200_OK;
     int st = set_grouped_attribute<PATH>();
     if (st != SGEMM_B200_OK) return st;
     PrepParams pp;
     pp.jobs = reinterpret_cast<const PrepJob*>(d + gt.off_jobs);
     pp.a_prefix = reinterpret_cast<const int*>(d + gt.off_apref);
     pp.b_prefix = reinterpret_cast<const int*>(d + gt.off_bpref);
+    pp.packs = reinterpret_cast<const PackJob*>(d + gt.off_packs);
+    pp.p_prefix = reinterpret_cast<const int*>(d + gt.off_ppref);
     pp.n_jobs = (int)gt.jobs.size();
+    pp.n_packs = (int)gt.packs.size();
     pp.a_blocks = gt.a_prefix.back();
-    const int blocks = gt.a_prefix.back() + gt.b_prefix.back();
-    split_prepass_grouped_kernel<PATH><<<blocks, 256, 0, stream>>>(pp);
-    cudaError_t e = cudaGetLastError();
+    pp.b_blocks = gt.b_prefix.back();
+    const int blocks = pp.a_blocks + pp.b_blocks + gt.p_prefix.back();
+    cudaError_t e = cudaSuccess;
+    if (blocks)
+        e = launch_chained(split_prepass_grouped_kernel<PATH>, blocks, 256, 0, stream, pp);
     if (e != cudaSuccess) {
         note_error("grouped split pre-pass launch (%d blocks): %s", blocks, cudaGetErrorString(e));
         return cuda_status(e) == SGEMM_B200_ERR_NO_MEMORY ? SGEMM_B200_ERR_NO_MEMORY
                                                            : SGEMM_B200_ERR_CUDA;
     }
+    if (!gt.ftiles.empty()) {
+        fused::GParams fp;
+        fp.probs = reinterpret_cast<const fused::GProblem*>(d + gt.off_fprobs);
+        fp.tiles = reinterpret_cast<const fused::GTile*>(d + gt.off_ftiles);
+        fp.maps = reinterpret_cast<const CUtensorMap*>(d + gt.off_fmaps);
+        fp.sums = sums;
+        fp.status = device_status_ptr();
+        fp.n_tiles = (int)gt.ftiles.size();
+        if (!fp.status) return SGEMM_B200_ERR_CUDA;
+        e = launch_chained(fused::split_fused_grouped_kernel<PATH>, fused_grid(gt), fused::THREADS,
+                           fused::Lay<PATH>::SMEM, stream, fp);
+        if (e != cudaSuccess) {
+            note_error("grouped fused split launch (%d CTAs): %s", fused_grid(gt),
+                       cudaGetErrorString(e));
+            return SGEMM_B200_ERR_CUDA;
+        }
+    }
+    if (gt.tiles.empty()) return SGEMM_B200_OK;
     GSParams gp;
     gp.probs = reinterpret_cast<const GSProblem*>(d);
     gp.tiles = reinterpret_cast<const GSTile*>(d + gt.off_tiles);
@@ -1054,8 +1423,8 @@ static int grouped_enqueue(const GroupedTables& gt, const uint8_t* d, cudaStream
     if (!gp.status) return SGEMM_B200_ERR_CUDA;
     const int sms = device_info().sm_count > 0 ? device_info().sm_count : 148;
     const int grid = std::min(gp.n_tiles, sms);
-    split_grouped_kernel<PATH><<<grid, THREADS, Layout<PATH>::SMEM_BYTES, stream>>>(gp);
-    e = cudaGetLastError();
+    e = launch_chained(split_grouped_kernel<PATH>, grid, THREADS, Layout<PATH>::SMEM_BYTES, stream,
+                       gp);
     if (e != cudaSuccess) {
         note_error("grouped split kernel launch (%d CTAs x %d threads, %d B shared): %s", grid,
                    THREADS, Layout<PATH>::SMEM_BYTES, cudaGetErrorString(e));
@@ -1068,9 +1437,9 @@ template <int PATH>
 static int grouped_arena_launch(Arena* a, const sgemm_b200_problem* probs, void* const* ws,
                                 int count, cudaStream_t stream) {
     GroupedTables gt;
-    int st = grouped_tables<PATH>(probs, ws, count, &gt);
+    int st = grouped_tables<PATH>(probs, ws, grouped_classes(PATH, probs, count), count, &gt);
     if (st != SGEMM_B200_OK) return st;
-    if (!gt.tiles.empty()) {
+    if (!gt.tiles.empty() || !gt.ftiles.empty()) {
         if (gt.bytes > a->cap) {
             // grow: generous first size (64 KiB covers ~100 problems), doubling
             const size_t n = std::max({gt.bytes, a->cap * 2, (size_t)65536});
@@ -1087,9 +1456,20 @@ static int grouped_arena_launch(Arena* a, const sgemm_b200_problem* probs, void*
             if (e != cudaSuccess) return cuda_status(e);
             a->cap = n;
         }
+        if (const size_t n = sums_bytes(gt); n > a->sums_cap) {
+            if (a->sums) cudaFreeAsync(a->sums, stream);
+            a->sums = nullptr;
+            a->sums_cap = 0;
+            cudaMemPool_t pool = library_pool();
+            if (!pool) return SGEMM_B200_ERR_CUDA;
+            const cudaError_t e =
+                cudaMallocFromPoolAsync(reinterpret_cast<void**>(&a->sums), n, pool, stream);
+            if (e != cudaSuccess) return cuda_status(e);
+            a->sums_cap = n;
+        }
         pack_tables(gt, a->h);
         st = cuda_status(cudaMemcpyAsync(a->d, a->h, gt.bytes, cudaMemcpyHostToDevice, stream));
-        if (st == SGEMM_B200_OK) st = grouped_enqueue<PATH>(gt, a->d, stream);
+        if (st == SGEMM_B200_OK) st = grouped_enqueue<PATH>(gt, a->d, a->sums, stream);
         if (st != SGEMM_B200_OK) return st;
     }
     for (int i : gt.k_zero) {  // C := beta * C
@@ -1119,19 +1499,57 @@ int grouped_launch(Arena* a, int path, const sgemm_b200_problem* probs, void* co
 
 void arena_release(Arena* a) {
     cudaFree(a->d);
+    cudaFree(a->sums);
     cudaFreeHost(a->h);
     *a = Arena();
 }
 
 }  // namespace split
 
-int split_launch(int path, int m, int n, int k, float alpha, const float* A, int lda,
-                 const float* B, int ldb, float beta, float* C, int ldc, void* ws,
-                 size_t ws_bytes, cudaStream_t stream) {
+// `whole`: the slabs come from this problem's route, of which m x n is a block.
+struct Whole {
+    int m, n;
+};
+static int split_launch(int path, int m, int n, int k, float alpha, const float* A, int lda,
+                        const float* B, int ldb, float beta, float* C, int ldc, void* ws,
+                        size_t ws_bytes, cudaStream_t stream, bool ws_optional = false,
+                        Whole whole = {0, 0}) {
     if (m == 0 || n == 0) return SGEMM_B200_OK;
     if (!device_is_sm100()) return SGEMM_B200_ERR_UNSUPPORTED;
     if (k == 0)  // C = beta*C: no products to split
         return plain_launch(-1, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, stream);
+    split::Route r = split::route(path, m, n, k);
+    if (whole.m) r.splits = split::route(path, whole.m, whole.n, k).splits;
+    // (a workspace the caller passes receives the operand planes)
+    if ((!ws || ws_optional) && r.fused) {
+        split::Packed pk = split::packed(m, n, k, A, lda, B, ldb, nullptr);
+        if (pk.bytes <= (ws_optional ? ws_bytes : SIZE_MAX)) {
+            void* rows = ws;
+            if (pk.bytes && !ws) {
+                cudaMemPool_t pool = library_pool();
+                if (!pool) return SGEMM_B200_ERR_CUDA;
+                const cudaError_t e = cudaMallocFromPoolAsync(&rows, pk.bytes, pool, stream);
+                if (e != cudaSuccess) return cuda_status(e);
+            }
+            int s = SGEMM_B200_OK;
+            if (pk.bytes) {
+                pk = split::packed(m, n, k, A, lda, B, ldb, rows);
+                s = plain_pack_rows(pk.pa ? m : 0, k, A, lda, const_cast<float*>(pk.A), pk.lda,
+                                    pk.pb ? k : 0, n, B, ldb, const_cast<float*>(pk.B), pk.ldb,
+                                    stream);
+            }
+            if (s == SGEMM_B200_OK)
+                s = path == SGEMM_B200_PATH_BF16X6
+                        ? split::launch_fused<SGEMM_B200_PATH_BF16X6>(m, n, k, alpha, pk.A, pk.lda,
+                                                                      pk.B, pk.ldb, beta, C, ldc,
+                                                                      r.splits, stream)
+                        : split::launch_fused<SGEMM_B200_PATH_TF32X3>(m, n, k, alpha, pk.A, pk.lda,
+                                                                      pk.B, pk.ldb, beta, C, ldc,
+                                                                      r.splits, stream);
+            if (rows != ws) cudaFreeAsync(rows, stream);
+            return s;
+        }
+    }
     const size_t need = path == SGEMM_B200_PATH_BF16X6
                             ? split::workspace_bytes<SGEMM_B200_PATH_BF16X6>(m, n, k)
                             : split::workspace_bytes<SGEMM_B200_PATH_TF32X3>(m, n, k);
@@ -1146,14 +1564,23 @@ int split_launch(int path, int m, int n, int k, float alpha, const float* A, int
     }
     int s;
     if (path == SGEMM_B200_PATH_BF16X6)
-        s = split::launch<SGEMM_B200_PATH_BF16X6>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, ws,
-                                                  ws_bytes, stream);
+        s = split::launch<SGEMM_B200_PATH_BF16X6>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc,
+                                                  r.splits, ws, ws_bytes, stream);
     else
-        s = split::launch<SGEMM_B200_PATH_TF32X3>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, ws,
-                                                  ws_bytes, stream);
+        s = split::launch<SGEMM_B200_PATH_TF32X3>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc,
+                                                  r.splits, ws, ws_bytes, stream);
     if (owned) cudaFreeAsync(ws, stream);
     return s;
 }
+
+namespace split {
+int block_launch(int path, int whole_m, int whole_n, int m, int n, int k, float alpha,
+                 const float* A, int lda, const float* B, int ldb, float beta, float* C, int ldc,
+                 cudaStream_t stream) {
+    return split_launch(path, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, nullptr, 0, stream,
+                        false, Whole{whole_m, whole_n});
+}
+}  // namespace split
 
 }  // namespace sgb
 
@@ -1190,11 +1617,16 @@ template <int PATH>
 static int grouped_oneshot(const sgemm_b200_problem* probs, int count, cudaStream_t stream) {
     cudaMemPool_t pool = library_pool();
     if (!pool) return SGEMM_B200_ERR_CUDA;
+    // workspace only for the problems that use it (planes, or copied rows)
+    const std::vector<char> fused = grouped_classes(PATH, probs, count);
     std::vector<size_t> off(count, 0);
     size_t total = 0;
     for (int i = 0; i < count; ++i) {
+        const sgemm_b200_problem& q = probs[i];
         off[i] = total;
-        total += align_up(problem_workspace_bytes(PATH, probs[i].m, probs[i].n, probs[i].k), 1024);
+        if (q.m > 0 && q.n > 0 && q.k > 0 &&
+            !(fused[i] && fused_ok(q.A, q.lda, q.B, q.ldb)))
+            total += align_up(problem_workspace_bytes(PATH, q.m, q.n, q.k), 1024);
     }
     uint8_t* ws = nullptr;
     if (total) {
@@ -1205,17 +1637,19 @@ static int grouped_oneshot(const sgemm_b200_problem* probs, int count, cudaStrea
     std::vector<void*> wsp(count);
     for (int i = 0; i < count; ++i) wsp[i] = ws + off[i];
     GroupedTables gt;
-    int st = grouped_tables<PATH>(probs, wsp.data(), count, &gt);
+    int st = grouped_tables<PATH>(probs, wsp.data(), fused, count, &gt);
     uint8_t* d = nullptr;
-    if (st == SGEMM_B200_OK && !gt.tiles.empty()) {
+    if (st == SGEMM_B200_OK && (!gt.tiles.empty() || !gt.ftiles.empty())) {
         std::vector<uint8_t> h(gt.bytes);
         pack_tables(gt, h.data());
-        st = cuda_status(cudaMallocFromPoolAsync(reinterpret_cast<void**>(&d), gt.bytes, pool,
-                                                 stream));
+        const size_t sums = align_up(gt.bytes, 256);  // after the tables
+        st = cuda_status(cudaMallocFromPoolAsync(reinterpret_cast<void**>(&d),
+                                                 sums + sums_bytes(gt), pool, stream));
         if (st == SGEMM_B200_OK)
             st = cuda_status(cudaMemcpyAsync(d, h.data(), gt.bytes, cudaMemcpyHostToDevice,
                                              stream));
-        if (st == SGEMM_B200_OK) st = grouped_enqueue<PATH>(gt, d, stream);
+        if (st == SGEMM_B200_OK)
+            st = grouped_enqueue<PATH>(gt, d, reinterpret_cast<float*>(d + sums), stream);
     }
     for (size_t z = 0; st == SGEMM_B200_OK && z < gt.k_zero.size(); ++z) {
         const sgemm_b200_problem& q = probs[gt.k_zero[z]];
@@ -1334,7 +1768,7 @@ extern "C" int sgemm_b200_split_noalloc(int path, int m, int n, int k, const flo
     if (s == SGEMM_B200_OK) scratch = sgb::noalloc::scratch_address(&s);
     if (s == SGEMM_B200_OK)
         s = sgb::split_launch(path, m, n, k, *alpha, A, lda, B, ldb, *beta, C, ldc, scratch,
-                              sgb::noalloc::kNoAllocScratchBytes, sgb::as_stream(stream));
+                              sgb::noalloc::kNoAllocScratchBytes, sgb::as_stream(stream), true);
     sgb::set_last_status(s);
     return s;
 }

@@ -102,3 +102,23 @@ def test_grouped_split_many_uneven_problems(path):
     assert sg.device_status() == sg.OK
     for (A, B, C, alpha, beta), (_, _, Cs, _, _) in zip(specs, seq):
         assert torch.equal(C, Cs), (A.shape, B.shape)
+
+
+@pytest.mark.parametrize("path", PATHS)
+@pytest.mark.parametrize("pad", [0, 3])
+def test_grouped_split_kernel_mix(path, pad):
+    """A launch that computes some problems from planes (large squares), some with
+    the operands split inside the GEMM, in one k slab or several, and with rows
+    copied first where strides ask for it: each problem's own bits."""
+    torch = _torch()
+    shapes = [(2048, 2048, 1024), (64, 64, 4096), (24, 4096, 4096), (130, 1, 700),
+              (2304, 2048, 512), (200, 700, 1284), (16, 128, 256), (300, 130, 2100)]
+    specs, c0 = _make(shapes, 1300, pad=pad)
+    sg.grouped_split(path, sg.make_problems(specs))
+    torch.cuda.synchronize()
+    assert sg.device_status() == sg.OK
+    for (A, B, C, alpha, beta), C0 in zip(specs, c0):
+        want = C0.clone()
+        sg.gemm(path, A, B, want, alpha, beta)
+        torch.cuda.synchronize()
+        assert torch.equal(C, want), (A.shape, B.shape)

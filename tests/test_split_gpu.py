@@ -238,3 +238,53 @@ def test_prepass_planes_bit_exact(path, m, n, k):
     for s, (pa, pb) in enumerate(zip(_planes(path, Ap), _planes(path, Bt))):
         assert np.array_equal(got_a[s].view(np.uint32), pa.view(np.uint32)), f"A plane {s}"
         assert np.array_equal(got_b[s].view(np.uint32), pb.view(np.uint32)), f"B plane {s}"
+
+
+# Shapes whose call without a workspace splits the operands inside the GEMM, at
+# the edges of its 128-column and 16-row tiles, its 32-deep blocks, its 256-deep
+# chunks and the 1 to 8 k slabs a cluster adds; strides that need copied rows.
+FUSED = [(1, 4, 4), (16, 128, 256), (17, 129, 260), (24, 132, 2052), (64, 64, 4096),
+         (129, 260, 1028), (200, 700, 1284), (77, 93, 1301), (130, 1, 700)]
+
+
+@pytest.mark.parametrize("path", PATHS)
+@pytest.mark.parametrize("shape", FUSED, ids=lambda s: "x".join(map(str, s)))
+def test_split_inside_equals_planes(path, shape):
+    """With a workspace the operands are split by a pre-pass, without one inside
+    the GEMM: the same bits, for one k slab and for several, and an error within
+    the path's bound."""
+    m, n, k = shape
+    A = oracle.fill(m, k, 15, 1, 0)
+    B = oracle.fill(k, n, 15, 2, 0)
+    C = oracle.fill(m, n, 15, 3, 0)
+    planes = _run(path, A, B, C, 1.5, 0.5, ws=True)
+    inside = _run(path, A, B, C, 1.5, 0.5, ws=False)
+    assert np.array_equal(planes.view(np.uint32), inside.view(np.uint32))
+    e = _errors(inside, A, B, C, 1.5, 0.5)
+    ep = _errors(oracle.sgemm_basic(A, B, C, 1.5, 0.5, basic=False), A, B, C, 1.5, 0.5)
+    assert e["max_componentwise"] <= _bound(ep["max_componentwise"])
+
+
+@pytest.mark.parametrize("path", PATHS)
+def test_split_beta_zero_ignores_c_in_slabs(path):
+    m, n, k = 33, 140, 4096
+    A, B = oracle.fill(m, k, 16, 1, 0), oracle.fill(k, n, 16, 2, 0)
+    nan = np.full((m, n), np.nan, dtype=np.float32)
+    got = _run(path, A, B, nan, 1.0, 0.0, ws=False, lds=(None, None, n + 3))
+    want = _run(path, A, B, np.zeros_like(nan), 1.0, 0.0, ws=False)
+    assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("path", PATHS)
+def test_split_host_blocks_keep_the_whole_problems_slabs(path):
+    """Blocks of a caller's plan have the k slabs of the whole problem, not their
+    own: the device entry point's bits."""
+    torch = _torch()
+    m, n, k = 384, 512, 4096
+    A, B, C = (oracle.fill(r, c, 17, t, 0) for r, c, t in ((m, k, 1), (k, n, 2), (m, n, 3)))
+    want = _run(path, A, B, C, 1.5, 0.5, ws=False)
+    hC = torch.from_numpy(C.copy()).pin_memory()
+    sg.sgemm_host(torch.from_numpy(A).pin_memory(), torch.from_numpy(B).pin_memory(), hC, 1.5,
+                  0.5, path=path, plan=(128, [128, 384]))
+    torch.cuda.synchronize()
+    assert np.array_equal(hC.numpy(), want)
