@@ -8,17 +8,22 @@
 //  - The plan flattens every problem into work items (tile_m, tile_n, k
 //    split), sorted longest-first so the tail of the launch is short items.
 //  - Persistent 4-warp CTAs (2 or 3 per SM) claim items with an atomic
-//    counter and run the same FFMA core as the plain path on each: one of two
-//    tile shapes (128x64 or 64x128, 8 x 8 thread tiles) and one of two
-//    loaders (TMA with per-problem tensor maps kept in global memory, or
-//    4-byte cp.async for strides TMA cannot describe), chosen per problem at
-//    plan time.
+//    counter and run the same FFMA core as the plain path on each: one of three
+//    tile shapes and one of three ways to read the operands (load_of), chosen
+//    per problem at plan time; the tensor maps are kept in global memory.
+//  - A launch is two kernels, chained: one transposes A (and copies rows TMA
+//    cannot describe) for the problems that read prepared operands and resets
+//    the tickets, the other runs the items.  What bounds the items is the FMA
+//    pipe, and with A [row][k] its register reads: a server's 32 requests took
+//    9435 us that way (57.9 TFLOP/s), 8486 with A transposed (64.3, the pass
+//    included; 86% of the FP32 peak); 24 odd problems of 300..3000 2245 -> 995.
+//  - Without memory for the prepared operands every problem is read in place.
 //  - Items with split == 1 run the plain path's exact arithmetic, so their
 //    results equal sgemm_b200's bit for bit.  Split-K items write partial sums
 //    to a workspace; the last split of a tile to finish (atomic ticket) adds
 //    the partials in split order 0, 1, 2, ... and applies alpha/beta, so the
 //    result is deterministic and independent of scheduling.
-//  - The launch (counter reset + kernel) is captured once into a CUDA graph
+//  - The launch is captured once into a CUDA graph
 //    and replayed.
 //  - Tile shape, split-K and stage count per size bucket come from the
 //    autotuner (sgemm_b200_autotune_grouped), persisted as JSON keyed by the
@@ -32,12 +37,14 @@
 #include <numeric>
 #include <sstream>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "common.h"
 #include "ffma_kernel.cuh"
 #include "grouped.h"
 #include "plain.h"
+#include "transpose.cuh"
 
 namespace sgb {
 namespace grouped {
@@ -56,10 +63,20 @@ using CfgW = ffma::Cfg<64, 128, 2, 2, 8, S, ffma::kLoaderAsync4, (S == 3 ? 3 : 2
 template <int S>
 using CfgS = ffma::Cfg<32, 128, 1, 4, 4, S, ffma::kLoaderAsync4, (S == 3 ? 3 : 2)>;  // 32 x 128
 
+// The same tiles on A transposed (compute_stage_kmajor).
+template <int S>
+using KmT = ffma::Cfg<128, 64, 4, 1, 8, S, ffma::kLoaderTma, (S == 3 ? 3 : 2), 8, true>;
+template <int S>
+using KmW = ffma::Cfg<64, 128, 2, 2, 8, S, ffma::kLoaderTma, (S == 3 ? 3 : 2), 8, true>;
+template <int S>
+using KmS = ffma::Cfg<32, 128, 1, 4, 4, S, ffma::kLoaderTma, (S == 3 ? 3 : 2), 8, true>;
+
 constexpr int THREADS = 128;
 constexpr int SLOT_BYTES = 24 * 1024;  // 16 KB + 8 KB per 32-deep k block (4 + 16 KB skinny)
 static_assert(CfgT<3>::STAGE_BYTES == SLOT_BYTES && CfgW<3>::STAGE_BYTES == SLOT_BYTES &&
-                  CfgS<3>::STAGE_BYTES <= SLOT_BYTES && CfgS<3>::THREADS == THREADS,
+                  CfgS<3>::STAGE_BYTES <= SLOT_BYTES && CfgS<3>::THREADS == THREADS &&
+                  KmT<3>::STAGE_BYTES == SLOT_BYTES && KmW<3>::STAGE_BYTES == SLOT_BYTES &&
+                  KmS<3>::STAGE_BYTES <= SLOT_BYTES && KmS<3>::COMPUTE_THREADS == THREADS,
               "");
 enum TileShape { kTileTall = 0, kTileWide = 1, kTileSkinny = 2 };  // 128x64, 64x128, 32x128
 
@@ -67,12 +84,17 @@ inline int tile_bm(int t) { return t == kTileTall ? 128 : t == kTileWide ? 64 : 
 inline int tile_bn(int t) { return t == kTileTall ? 64 : 128; }
 
 // Throughput of each tile relative to 128 x 64 on work that fills them
-// (measured on a B200 with the single-GEMM kernels of the same shapes).  A
+// (measured on a B200 with single-GEMM kernels of the same shapes).  A
 // problem leaves its bucket's tile for another when that tile's zero-padded
 // area divided by its efficiency is at least 2% smaller.
 inline double tile_efficiency(int t) {
     return t == kTileTall ? 1.0 : t == kTileWide ? 0.994 : 0.75;
 }
+
+// How a problem's tiles are read: in place by 4-byte cp.async (strides or bases
+// TMA cannot describe), in place by TMA, or by TMA from a transposed copy of A
+// (and, where needed, a copy of B in aligned rows) that the launch makes first.
+enum Load { kLoadAsync4 = 0, kLoadRows = 1, kLoadTransposed = 2 };
 
 struct GProblem {
     Operands op;
@@ -81,7 +103,8 @@ struct GProblem {
     int rem_tile;  // tile of the last rows when they are a strip of their own, else -1
     int rem_m0;    // first row of that strip
     int shapes;    // bit t: the problem has tiles of shape t (a map pair per shape)
-    int tma;       // tensor maps valid
+    int load;      // a Load: how the problem's tiles reach shared memory
+    int pack_b;    // B is copied to aligned rows first (kLoadTransposed only)
     int split;     // k splits
     int kbps;      // k blocks per split
     int depth;     // k blocks kept in flight through the stage ring (2..S)
@@ -96,6 +119,14 @@ struct GProblem {
 struct GItem {
     int prob, m0, n0, ks;
     int tile, tl;
+};
+
+// One matrix that the launch prepares: A transposed, or B copied to aligned
+// rows, by 64 x 64 tiles; its tiles are blocks first, first + 1, ...
+struct GPrep {
+    ffma::TransposeJob job;
+    int copy;
+    int first;
 };
 
 struct GParams {
@@ -115,7 +146,7 @@ constexpr int smem_bytes() {
 
 // One work item on the FFMA core.  Returns false (uniformly across the CTA)
 // if a bounded wait expired.
-template <class C, bool TMA, int S>
+template <class C, int LOAD, int S>
 __device__ __forceinline__ bool run_item(const GParams& gp, const GProblem& pr, const GItem& it,
                                          int item_prob, uint8_t* smem, uint64_t* full_bar,
                                          uint32_t& g, int* last_s) {
@@ -130,8 +161,8 @@ __device__ __forceinline__ bool run_item(const GParams& gp, const GProblem& pr, 
     const int kb1 = min(nk, kb0 + pr.kbps);
     const int nkb = max(0, kb1 - kb0);
 
-    uint32_t a_base, xa0, xa1;
-    ffma::a_coords<C>(wm, lm, a_base, xa0, xa1);
+    uint32_t a_base = 0, xa0 = 0, xa1 = 0;  // A's offsets when it stays [row][k]
+    if constexpr (!C::KM) ffma::a_coords<C>(wm, lm, a_base, xa0, xa1);
     const uint32_t b_base = static_cast<uint32_t>((wn * 8 * C::TN + ln * 4) * 4);
 
     float acc[C::TM][C::TN];
@@ -140,7 +171,7 @@ __device__ __forceinline__ bool run_item(const GParams& gp, const GProblem& pr, 
 #pragma unroll
         for (int j = 0; j < C::TN; ++j) acc[i][j] = 0.0f;
 
-    if constexpr (TMA) {
+    if constexpr (LOAD != kLoadAsync4) {
         const CUtensorMap* tmA = gp.maps + 6 * item_prob + 2 * it.tile;
         const CUtensorMap* tmB = tmA + 1;
         int issued = 0;
@@ -149,7 +180,10 @@ __device__ __forceinline__ bool run_item(const GParams& gp, const GProblem& pr, 
             const int s = gs % S;
             uint8_t* st = smem + s * SLOT_BYTES;
             mbar_arrive_expect_tx(&full_bar[s], C::A_TX + C::B_BYTES);
-            tma_load_2d(st, tmA, &full_bar[s], (kb0 + j) * C::BK, m0);
+            if constexpr (C::KM)
+                tma_load_2d(st, tmA, &full_bar[s], m0, (kb0 + j) * C::BK);
+            else
+                tma_load_2d(st, tmA, &full_bar[s], (kb0 + j) * C::BK, m0);
             tma_load_2d(st + C::A_BYTES, tmB, &full_bar[s], n0, (kb0 + j) * C::BK);
         };
         if (tid == 0) {
@@ -176,7 +210,10 @@ __device__ __forceinline__ bool run_item(const GParams& gp, const GProblem& pr, 
                 issue(issued++);
             }
             const uint8_t* st = smem + s * SLOT_BYTES;
-            ffma::compute_stage<C>(st, st + C::A_BYTES, a_base, xa0, xa1, b_base, acc);
+            if constexpr (C::KM)
+                ffma::compute_stage_kmajor<C>(st, st + C::A_BYTES, wm, lm, b_base, acc);
+            else
+                ffma::compute_stage<C>(st, st + C::A_BYTES, a_base, xa0, xa1, b_base, acc);
         }
         g += nkb;
     } else {
@@ -274,31 +311,81 @@ __global__ void __launch_bounds__(THREADS, (S == 3 ? 3 : 2)) grouped_kernel(cons
         fence_barrier_init();
     }
     __syncthreads();
+    grid_wait();
     uint32_t g = 0;  // k blocks consumed through the TMA ring (phase tracking)
-    while (true) {
-        if (tid == 0) item_s = atomicAdd(&gp.counters[0], 1);
+    // The first item by block index: blocks are spread over the SMs in order, so
+    // the longest items do not share one, as they may when the resident CTAs of a
+    // chained launch all claim at once (12 uneven problems 349 us, 211 so).
+    for (bool first = true;; first = false) {
+        if (tid == 0)
+            item_s = first ? (int)blockIdx.x : (int)gridDim.x + atomicAdd(&gp.counters[0], 1);
         __syncthreads();
         const int idx = item_s;
         if (idx >= gp.n_items) break;
+
         const GItem it = gp.items[idx];
         const GProblem& pr = gp.probs[it.prob];
         bool ok;
-        if (it.tile == kTileTall) {
-            ok = pr.tma ? run_item<CfgT<S>, true, S>(gp, pr, it, it.prob, smem, full_bar, g, &last_s)
-                        : run_item<CfgT<S>, false, S>(gp, pr, it, it.prob, smem, full_bar, g,
-                                                      &last_s);
-        } else if (it.tile == kTileSkinny) {
-            ok = pr.tma ? run_item<CfgS<S>, true, S>(gp, pr, it, it.prob, smem, full_bar, g, &last_s)
-                        : run_item<CfgS<S>, false, S>(gp, pr, it, it.prob, smem, full_bar, g,
-                                                      &last_s);
-        } else {
-            ok = pr.tma ? run_item<CfgW<S>, true, S>(gp, pr, it, it.prob, smem, full_bar, g, &last_s)
-                        : run_item<CfgW<S>, false, S>(gp, pr, it, it.prob, smem, full_bar, g,
-                                                      &last_s);
-        }
+        auto run = [&](auto* km, auto* rows) {
+            using K = std::remove_pointer_t<decltype(km)>;
+            using R = std::remove_pointer_t<decltype(rows)>;
+            ok = pr.load == kLoadTransposed
+                     ? run_item<K, kLoadTransposed, S>(gp, pr, it, it.prob, smem, full_bar, g,
+                                                       &last_s)
+                 : pr.load == kLoadRows
+                     ? run_item<R, kLoadRows, S>(gp, pr, it, it.prob, smem, full_bar, g, &last_s)
+                     : run_item<R, kLoadAsync4, S>(gp, pr, it, it.prob, smem, full_bar, g,
+                                                   &last_s);
+        };
+        if (it.tile == kTileTall)
+            run((KmT<S>*)nullptr, (CfgT<S>*)nullptr);
+        else if (it.tile == kTileSkinny)
+            run((KmS<S>*)nullptr, (CfgS<S>*)nullptr);
+        else
+            run((KmW<S>*)nullptr, (CfgW<S>*)nullptr);
         if (!ok) break;
         __syncthreads();  // stages and item_s are free for the next item
     }
+}
+
+// Before the grouped kernel: block 0 resets its tickets, the others prepare a
+// 64 x 64 tile each.  HBM-bound.
+constexpr int kPrepThreads = 256;
+__global__ void __launch_bounds__(kPrepThreads)
+    grouped_prepare_kernel(const GPrep* preps, int count, int* counters, int n_counters) {
+    __shared__ float tile[ffma::kTrTile][ffma::kTrTile + 1];
+    grid_wait();
+    if (blockIdx.x == 0) {
+        for (int i = threadIdx.x; i < n_counters; i += kPrepThreads) counters[i] = 0;
+        return;
+    }
+    const int b = blockIdx.x - 1;
+    int lo = 0, hi = count - 1;  // the last matrix whose first block is <= b
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) / 2;
+        if (preps[mid].first <= b)
+            lo = mid;
+        else
+            hi = mid - 1;
+    }
+    const GPrep p = preps[lo];
+    if (!p.copy) {
+        ffma::transpose_tile(p.job, b - p.first, tile);
+        return;
+    }
+    const int tk = (p.job.k + ffma::kTrTile - 1) / ffma::kTrTile;
+    const int c = (b - p.first) % tk * ffma::kTrTile + threadIdx.x % 64;
+    const int r0 = (b - p.first) / tk * ffma::kTrTile + threadIdx.x / 64;
+    float v[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+        v[i] = c < p.job.k && r0 + 4 * i < p.job.m
+                   ? p.job.src[(int64_t)(r0 + 4 * i) * p.job.ld_src + c]
+                   : 0.0f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+        if (c < p.job.k && r0 + 4 * i < p.job.m)
+            p.job.dst[(int64_t)(r0 + 4 * i) * p.job.ld_dst + c] = v[i];
 }
 
 // ------------------------------------------------------------------ host --
@@ -389,10 +476,9 @@ static bool save_table(const char* path, const Table& t) {
     return bool(f);
 }
 
-static bool tma_ok(const sgemm_b200_problem& p) {
-    return p.k > 0 && (p.lda % 4 == 0) && (p.ldb % 4 == 0) &&
-           (reinterpret_cast<uintptr_t>(p.A) % 16 == 0) &&
-           (reinterpret_cast<uintptr_t>(p.B) % 16 == 0);
+static bool tma_ok(int k, const float* A, int lda, const float* B, int ldb) {
+    return k > 0 && lda % 4 == 0 && ldb % 4 == 0 && reinterpret_cast<uintptr_t>(A) % 16 == 0 &&
+           reinterpret_cast<uintptr_t>(B) % 16 == 0;
 }
 
 }  // namespace grouped
@@ -406,10 +492,14 @@ struct sgemm_b200_grouped_plan {
     int grid = 0;
     size_t ws_floats = 0;
     int n_counters = 0;
+    uint8_t* d_block = nullptr;  // what follows it, one allocation
     sgb::grouped::GProblem* d_probs = nullptr;
     sgb::grouped::GItem* d_items = nullptr;
     CUtensorMap* d_maps = nullptr;
     float* d_ws = nullptr;
+    float* d_scratch = nullptr;  // transposed A (and copied B) of the problems that use them
+    sgb::grouped::GPrep* d_preps = nullptr;
+    int n_preps = 0, prep_tiles = 0;
     int* d_counters = nullptr;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -424,11 +514,9 @@ static void free_plan(sgemm_b200_grouped_plan* p) {
     if (p->exec) cudaGraphExecDestroy(p->exec);
     if (p->graph) cudaGraphDestroy(p->graph);
     if (p->cap_stream) cudaStreamDestroy(p->cap_stream);
-    cudaFree(p->d_probs);
-    cudaFree(p->d_items);
-    cudaFree(p->d_maps);
+    cudaFree(p->d_block);
     cudaFree(p->d_ws);
-    cudaFree(p->d_counters);
+    cudaFree(p->d_scratch);  // back to the library pool, after the frees that wait for the device
     delete p;
 }
 
@@ -439,7 +527,33 @@ struct Schedule {
     long long ws_floats = 0;
     int tickets = 0;
     int tiles = 0;
+    size_t scratch_floats = 0;  // prepared operands (kLoadTransposed)
 };
+
+// Which problems read prepared operands (the launch has a pass before its items
+// anyway, which resets the tickets).
+//  - Aligned operands: A transposed pays from 512 columns on, where the faster
+//    FMA loop (64 TFLOP/s from 58) outweighs moving 8 m k bytes.  48 problems of
+//    512 x n x 1024, transposed against in place: n = 512 466 us against 489,
+//    n = 1024 845 against 907.
+//  - Operands TMA cannot describe: the copies beat the 4-byte loader, whose k
+//    block costs about 4 us of latency, wherever there is more than one block.
+constexpr int kTransposeMinN = 512;
+constexpr double kTransposeMinWork = 32.0e6;  // m n k
+
+static int load_of(const sgemm_b200_problem& p) {
+    const bool in_place = tma_ok(p.k, p.A, p.lda, p.B, p.ldb);
+    const double work = double(p.m) * p.n * p.k;
+    if (in_place)
+        return p.n >= kTransposeMinN && work >= kTransposeMinWork ? kLoadTransposed : kLoadRows;
+    return p.k > 32 ? kLoadTransposed : kLoadAsync4;
+}
+
+// Floats of a prepared matrix of `rows` rows of `cols` (32-byte rows, 256-byte start).
+inline int prep_pitch(int cols) { return div_up(cols, 8) * 8; }
+inline size_t prep_floats(int rows, int cols) {
+    return ((size_t)rows * prep_pitch(cols) + 63) / 64 * 64;
+}
 
 static int make_schedule(const sgemm_b200_problem* probs, int count, const Table& table,
                          Schedule* out) {
@@ -514,7 +628,12 @@ static int make_schedule(const sgemm_b200_problem* probs, int count, const Table
                     }
                 }
         }
-        g.tma = tma_ok(q) ? 1 : 0;
+        g.load = load_of(q);
+        g.pack_b = g.load == kLoadTransposed &&
+                   (q.ldb % 4 != 0 || reinterpret_cast<uintptr_t>(q.B) % 16 != 0);
+        if (g.load == kLoadTransposed)
+            sc.scratch_floats +=
+                prep_floats(q.k, q.m) + (g.pack_b ? prep_floats(q.k, q.n) : 0);
         g.shapes = (1 << g.tile) | (g.rem_tile >= 0 ? 1 << g.rem_tile : 0);
         const int bm = tile_bm(g.tile), bn = tile_bn(g.tile);
         const int tm = q.m > 0 ? div_up(g.rem_m0, bm) : 0;
@@ -552,18 +671,80 @@ static int make_schedule(const sgemm_b200_problem* probs, int count, const Table
     return SGEMM_B200_OK;
 }
 
+// The matrices a launch prepares, laid out in `scratch` in problem order; returns
+// their 64 x 64 tiles.
+static int make_preps(const Schedule& sc, float* scratch, std::vector<GPrep>* out) {
+    int tiles = 0;
+    size_t used = 0;
+    auto add = [&](const float* src, int rows, int cols, int ld, bool copy) {
+        GPrep p;
+        p.job.src = src;
+        p.job.dst = scratch + used;
+        p.job.m = rows;
+        p.job.k = cols;
+        p.job.ld_src = ld;
+        p.job.ld_dst = prep_pitch(copy ? cols : rows);
+        p.job.sevens = 0;
+        p.job.vec = ld % 4 == 0 && reinterpret_cast<uintptr_t>(src) % 16 == 0;
+        p.job.blocks = 0;
+        p.copy = copy;
+        p.first = tiles;
+        used += copy ? prep_floats(rows, cols) : prep_floats(cols, rows);
+        tiles += div_up(rows, ffma::kTrTile) * div_up(cols, ffma::kTrTile);
+        out->push_back(p);
+    };
+    for (const GProblem& g : sc.probs) {
+        if (g.load != kLoadTransposed) continue;
+        add(g.op.A, g.op.m, g.op.k, g.op.lda, false);
+        if (g.pack_b) add(g.op.B, g.op.k, g.op.n, g.op.ldb, true);
+    }
+    return tiles;
+}
+
+// No scratch to be had: every problem is read in place.
+static void read_in_place(Schedule* sc) {
+    for (GProblem& g : sc->probs) {
+        if (g.load != kLoadTransposed) continue;
+        const bool ok = tma_ok(g.op.k, g.op.A, g.op.lda, g.op.B, g.op.ldb);
+        g.load = ok ? kLoadRows : kLoadAsync4;
+        g.pack_b = 0;
+    }
+    sc->scratch_floats = 0;
+}
+
 // The tensor maps of one problem: an (A, B) pair for each tile shape it uses,
-// at maps[2 * shape] and maps[2 * shape + 1] (six slots per problem).
-static bool encode_problem_maps(const GProblem& g, CUtensorMap* maps) {
+// at maps[2 * shape] and maps[2 * shape + 1] (six slots per problem).  `prep`:
+// the problem's prepared matrices (A, then B if it is copied), or null.
+static bool encode_problem_maps(const GProblem& g, const GPrep* prep, CUtensorMap* maps) {
     for (int t = 0; t < 3; ++t) {
         if (!(g.shapes & (1 << t))) continue;
-        if (!encode_tensor_map_2d(&maps[2 * t], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, g.op.A,
-                                  (uint64_t)g.op.k, (uint64_t)g.op.m, (uint64_t)g.op.lda * 4, 32,
-                                  tile_bm(t), CU_TENSOR_MAP_SWIZZLE_128B) ||
-            !encode_tensor_map_2d(&maps[2 * t + 1], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, g.op.B,
-                                  (uint64_t)g.op.n, (uint64_t)g.op.k, (uint64_t)g.op.ldb * 4,
-                                  tile_bn(t), 32, CU_TENSOR_MAP_SWIZZLE_NONE))
+        const bool okA =
+            prep ? encode_tensor_map_2d(&maps[2 * t], CU_TENSOR_MAP_DATA_TYPE_FLOAT32,
+                                        prep[0].job.dst, (uint64_t)g.op.m, (uint64_t)g.op.k,
+                                        (uint64_t)prep[0].job.ld_dst * 4, tile_bm(t), 32,
+                                        CU_TENSOR_MAP_SWIZZLE_NONE)
+                 : encode_tensor_map_2d(&maps[2 * t], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, g.op.A,
+                                        (uint64_t)g.op.k, (uint64_t)g.op.m,
+                                        (uint64_t)g.op.lda * 4, 32, tile_bm(t),
+                                        CU_TENSOR_MAP_SWIZZLE_128B);
+        const float* B = g.pack_b ? prep[1].job.dst : g.op.B;
+        const int ldb = g.pack_b ? prep[1].job.ld_dst : g.op.ldb;
+        if (!okA || !encode_tensor_map_2d(&maps[2 * t + 1], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, B,
+                                          (uint64_t)g.op.n, (uint64_t)g.op.k, (uint64_t)ldb * 4,
+                                          tile_bn(t), 32, CU_TENSOR_MAP_SWIZZLE_NONE))
             return false;
+    }
+    return true;
+}
+
+static bool encode_maps(const Schedule& sc, const std::vector<GPrep>& preps, CUtensorMap* maps) {
+    size_t next = 0;
+    for (size_t i = 0; i < sc.probs.size(); ++i) {
+        const GProblem& g = sc.probs[i];
+        if (g.load == kLoadAsync4) continue;
+        const GPrep* prep = g.load == kLoadTransposed ? &preps[next] : nullptr;
+        if (prep) next += 1 + g.pack_b;
+        if (!encode_problem_maps(g, prep, maps + 6 * i)) return false;
     }
     return true;
 }
@@ -611,35 +792,54 @@ static int build_plan(const sgemm_b200_problem* probs, int count, const Table& t
     plan->ws_floats = (size_t)sc.ws_floats;
     plan->n_counters = 1 + sc.tickets;
 
-    std::vector<CUtensorMap> maps(6 * (size_t)std::max(count, 1));
-    std::memset(maps.data(), 0, maps.size() * sizeof(CUtensorMap));
-    for (int i = 0; i < count; ++i) {
-        const GProblem& g = sc.probs[i];
-        if (g.tma && !encode_problem_maps(g, &maps[6 * (size_t)i])) {
-            free_plan(plan);
-            return SGEMM_B200_ERR_CUDA;
+    // Scratch from the library pool: a plan made for one launch does not pay a
+    // cudaMalloc of its operands' size.  On the null stream, whose copies below
+    // end before this call does.
+    if (sc.scratch_floats) {
+        cudaMemPool_t pool = library_pool();
+        if (!pool || cudaMallocFromPoolAsync(reinterpret_cast<void**>(&plan->d_scratch),
+                                             sizeof(float) * sc.scratch_floats, pool,
+                                             (cudaStream_t)0) != cudaSuccess) {
+            cudaGetLastError();
+            plan->d_scratch = nullptr;
+            read_in_place(&sc);
         }
     }
+    std::vector<GPrep> preps;
+    plan->prep_tiles = make_preps(sc, plan->d_scratch, &preps);
+    plan->n_preps = (int)preps.size();
+    std::vector<CUtensorMap> maps(6 * (size_t)std::max(count, 1));
+    std::memset(maps.data(), 0, maps.size() * sizeof(CUtensorMap));
+    if (!encode_maps(sc, preps, maps.data())) {
+        free_plan(plan);
+        return SGEMM_B200_ERR_CUDA;
+    }
 
-    cudaError_t e = cudaSuccess;
-    auto chk = [&](cudaError_t x) {
-        if (e == cudaSuccess) e = x;
-    };
-    chk(cudaMalloc(&plan->d_probs, sizeof(GProblem) * std::max(count, 1)));
-    chk(cudaMalloc(&plan->d_items, sizeof(GItem) * std::max<size_t>(sc.items.size(), 1)));
-    chk(cudaMalloc(&plan->d_maps, sizeof(CUtensorMap) * maps.size()));
-    chk(cudaMalloc(&plan->d_counters, sizeof(int) * plan->n_counters));
-    if (plan->ws_floats) chk(cudaMalloc(&plan->d_ws, sizeof(float) * plan->ws_floats));
-    if (e == cudaSuccess && count)
-        chk(cudaMemcpy(plan->d_probs, sc.probs.data(), sizeof(GProblem) * count,
-                       cudaMemcpyHostToDevice));
-    if (e == cudaSuccess && !sc.items.empty())
-        chk(cudaMemcpy(plan->d_items, sc.items.data(), sizeof(GItem) * sc.items.size(),
-                       cudaMemcpyHostToDevice));
-    if (e == cudaSuccess)
-        chk(cudaMemcpy(plan->d_maps, maps.data(), sizeof(CUtensorMap) * maps.size(),
-                       cudaMemcpyHostToDevice));
-    if (e == cudaSuccess) chk(cudaMemset(plan->d_counters, 0, sizeof(int) * plan->n_counters));
+    // One block, one copy: maps, problems, prepared matrices, items; then the
+    // tickets, which each launch resets.
+    const size_t n_maps = sizeof(CUtensorMap) * maps.size(), n_probs = sizeof(GProblem) * count,
+                 n_prep = sizeof(GPrep) * preps.size(), n_it = sizeof(GItem) * sc.items.size();
+    static_assert(sizeof(CUtensorMap) % 8 == 0 && sizeof(GProblem) % 8 == 0 &&
+                      sizeof(GPrep) % 8 == 0 && sizeof(GItem) % 8 == 0,
+                  "every part of the block is aligned");
+    const size_t copied = n_maps + n_probs + n_prep + n_it;
+    cudaError_t e = cudaMalloc(&plan->d_block, copied + sizeof(int) * plan->n_counters);
+    if (e == cudaSuccess && plan->ws_floats)
+        e = cudaMalloc(&plan->d_ws, sizeof(float) * plan->ws_floats);
+    if (e == cudaSuccess) {
+        std::vector<uint8_t> h(copied);
+        auto put = [&](size_t at, const void* src, size_t bytes) {
+            if (bytes) std::memcpy(h.data() + at, src, bytes);
+            return plan->d_block + at;
+        };
+        plan->d_maps = reinterpret_cast<CUtensorMap*>(put(0, maps.data(), n_maps));
+        plan->d_probs = reinterpret_cast<GProblem*>(put(n_maps, sc.probs.data(), n_probs));
+        plan->d_preps = reinterpret_cast<GPrep*>(put(n_maps + n_probs, preps.data(), n_prep));
+        plan->d_items =
+            reinterpret_cast<GItem*>(put(n_maps + n_probs + n_prep, sc.items.data(), n_it));
+        plan->d_counters = reinterpret_cast<int*>(plan->d_block + copied);
+        e = cudaMemcpy(plan->d_block, h.data(), copied, cudaMemcpyHostToDevice);
+    }
     if (e != cudaSuccess) {
         free_plan(plan);
         return cuda_status(e);
@@ -649,6 +849,19 @@ static int build_plan(const sgemm_b200_problem* probs, int count, const Table& t
     plan->grid = std::max(1, std::min(sms * resident_per_sm(plan->stages), plan->n_items));
     *out = plan;
     return SGEMM_B200_OK;
+}
+
+// The launch: operands prepared and tickets reset, then the items.
+static int enqueue_kernels(const GParams& p, int stages, int grid, const GPrep* preps, int n_preps,
+                           int prep_tiles, int n_counters, cudaStream_t stream) {
+    cudaError_t e = launch_chained(grouped_prepare_kernel, 1 + prep_tiles, kPrepThreads, 0, stream,
+                                   preps, n_preps, p.counters, n_counters);
+    if (e == cudaSuccess)
+        e = stages == 3 ? launch_chained(grouped_kernel<3>, grid, THREADS, smem_bytes<3>(), stream,
+                                         p)
+                        : launch_chained(grouped_kernel<4>, grid, THREADS, smem_bytes<4>(), stream,
+                                         p);
+    return cuda_status(e);
 }
 
 static int enqueue(sgemm_b200_grouped_plan* plan, cudaStream_t stream) {
@@ -662,13 +875,8 @@ static int enqueue(sgemm_b200_grouped_plan* plan, cudaStream_t stream) {
     p.status = device_status_ptr();
     p.n_items = plan->n_items;
     if (!p.status) return SGEMM_B200_ERR_CUDA;
-    cudaError_t e = cudaMemsetAsync(plan->d_counters, 0, sizeof(int) * plan->n_counters, stream);
-    if (e != cudaSuccess) return cuda_status(e);
-    if (plan->stages == 3)
-        grouped_kernel<3><<<plan->grid, THREADS, smem_bytes<3>(), stream>>>(p);
-    else
-        grouped_kernel<4><<<plan->grid, THREADS, smem_bytes<4>(), stream>>>(p);
-    return cuda_status(cudaGetLastError());
+    return enqueue_kernels(p, plan->stages, plan->grid, plan->d_preps, plan->n_preps,
+                           plan->prep_tiles, plan->n_counters, stream);
 }
 
 static int launch(sgemm_b200_grouped_plan* plan, cudaStream_t stream, int use_graph) {
@@ -719,6 +927,7 @@ static cudaError_t grow(T** d, T** h, size_t* cap, size_t need, cudaStream_t s,
     const size_t n = std::max({need, *cap * 2, min_cap});
     if (*d) cudaFreeAsync(*d, s);
     *d = nullptr;
+    *cap = 0;
     if (h && *h) {
         cudaFreeHost(*h);
         *h = nullptr;
@@ -751,12 +960,24 @@ int arena_launch(Arena* a, const sgemm_b200_problem* probs, int count, cudaStrea
     chk(grow<float>(&a->d_ws, nullptr, &a->cap_ws, std::max<size_t>(sc.ws_floats, 1), stream,
                     1));
     if (e != cudaSuccess) return cuda_status(e);
+    if (sc.scratch_floats && grow<float>(&a->d_scratch, nullptr, &a->cap_scratch,
+                                         sc.scratch_floats, stream, 1 << 22) != cudaSuccess) {
+        cudaGetLastError();
+        read_in_place(&sc);
+    }
+    std::vector<GPrep> preps;
+    const int prep_tiles = make_preps(sc, a->d_scratch, &preps);
+    chk(grow(&a->d_preps, &a->h_preps, &a->cap_preps, std::max<size_t>(preps.size(), 1), stream,
+             512));
+    if (e != cudaSuccess) return cuda_status(e);
     std::memcpy(a->h_probs, sc.probs.data(), sizeof(GProblem) * count);
     std::memcpy(a->h_items, sc.items.data(), sizeof(GItem) * sc.items.size());
     std::memset(a->h_maps, 0, sizeof(CUtensorMap) * 6 * count);
-    for (int i = 0; i < count; ++i) {
-        const GProblem& g = sc.probs[i];
-        if (g.tma && !encode_problem_maps(g, &a->h_maps[6 * (size_t)i])) return SGEMM_B200_ERR_CUDA;
+    if (!encode_maps(sc, preps, a->h_maps)) return SGEMM_B200_ERR_CUDA;
+    if (!preps.empty()) {
+        std::memcpy(a->h_preps, preps.data(), sizeof(GPrep) * preps.size());
+        chk(cudaMemcpyAsync(a->d_preps, a->h_preps, sizeof(GPrep) * preps.size(),
+                            cudaMemcpyHostToDevice, stream));
     }
     chk(cudaMemcpyAsync(a->d_probs, a->h_probs, sizeof(GProblem) * count, cudaMemcpyHostToDevice,
                         stream));
@@ -764,7 +985,6 @@ int arena_launch(Arena* a, const sgemm_b200_problem* probs, int count, cudaStrea
                         cudaMemcpyHostToDevice, stream));
     chk(cudaMemcpyAsync(a->d_maps, a->h_maps, sizeof(CUtensorMap) * 6 * count,
                         cudaMemcpyHostToDevice, stream));
-    chk(cudaMemsetAsync(a->d_counters, 0, sizeof(int) * n_counters, stream));
     if (e != cudaSuccess) return cuda_status(e);
     set_kernel_attributes();
     GParams p;
@@ -778,8 +998,8 @@ int arena_launch(Arena* a, const sgemm_b200_problem* probs, int count, cudaStrea
     if (!p.status) return SGEMM_B200_ERR_CUDA;
     static const int per_sm = resident_per_sm(3);  // after the attributes; once, thread-safe
     const int grid = std::max(1, std::min(device_info().sm_count * per_sm, p.n_items));
-    grouped_kernel<3><<<grid, THREADS, smem_bytes<3>(), stream>>>(p);
-    return cuda_status(cudaGetLastError());
+    return enqueue_kernels(p, 3, grid, a->d_preps, (int)preps.size(), prep_tiles, (int)n_counters,
+                           stream);
 }
 
 void arena_release(Arena* a) {
@@ -788,6 +1008,9 @@ void arena_release(Arena* a) {
     cudaFree(a->d_maps);
     cudaFree(a->d_counters);
     cudaFree(a->d_ws);
+    cudaFree(a->d_scratch);
+    cudaFree(a->d_preps);
+    cudaFreeHost(a->h_preps);
     cudaFreeHost(a->h_probs);
     cudaFreeHost(a->h_items);
     cudaFreeHost(a->h_maps);

@@ -12,6 +12,7 @@ namespace grouped {
 
 struct GProblem;
 struct GItem;
+struct GPrep;
 
 // Reusable device + pinned staging buffers for back-to-back grouped launches.
 struct Arena {
@@ -20,10 +21,14 @@ struct Arena {
     CUtensorMap* d_maps = nullptr;
     int* d_counters = nullptr;
     float* d_ws = nullptr;
+    float* d_scratch = nullptr;
+    GPrep* d_preps = nullptr;
+    GPrep* h_preps = nullptr;
     GProblem* h_probs = nullptr;
     GItem* h_items = nullptr;
     CUtensorMap* h_maps = nullptr;
-    size_t cap_probs = 0, cap_items = 0, cap_maps = 0, cap_counters = 0, cap_ws = 0;
+    size_t cap_probs = 0, cap_items = 0, cap_maps = 0, cap_counters = 0, cap_ws = 0,
+           cap_scratch = 0, cap_preps = 0;
 };
 
 // Schedule `count` problems (built-in choices, no split-K) and launch one

@@ -79,6 +79,55 @@ def test_grouped_bit_exact_with_plain_path():
     plan.close()
 
 
+# Around the rule for A transposed (work from 32e6 and 512 columns, or an operand
+# TMA cannot describe and k > 32), at the edges of the 64 x 64 transpose and of each tile:
+# one row, remainder strips of 32 and 64 rows, k not a multiple of 32 or 64.
+PREPARED = [(128, 512, 512), (128, 511, 512), (122, 512, 512), (1, 8192, 4096), (33, 640, 2051),
+            (161, 516, 385), (191, 1028, 323), (320, 320, 320), (257, 643, 197), (65, 513, 1000),
+            (5, 7, 32), (5, 7, 33), (1, 1, 3000)]
+PREPARED_LDS = {7: (321, None, None), 8: (None, 645, 643), 3: (4099, 8195, None)}
+
+
+@pytest.mark.parametrize("split", [1, 3])
+@pytest.mark.parametrize("use_graph", [False, True])
+def test_grouped_transposed_a_bit_exact(tmp_path, split, use_graph):
+    """The same bits as single calls (one chain per element; three k splits:
+    as problems small enough to be read in place would give), on new contents
+    of the same buffers too."""
+    torch = _torch()
+    lds = [PREPARED_LDS.get(i, (None, None, None)) for i in range(len(PREPARED))]
+    specs, host = _make(PREPARED, 700, lds)
+    plan = sg.GroupedPlan(specs, _table(tmp_path / "t.json", split, tile=0))
+    for scale in (1.0, -2.0):  # exact scaling: the results scale with it
+        for (dA, _, dC, _, _), (A, _, C, _, _) in zip(specs, host):
+            dA.copy_(torch.from_numpy(A * np.float32(scale)))
+            dC.copy_(torch.from_numpy(C))
+        plan.launch(use_graph=use_graph)
+        torch.cuda.synchronize()
+        assert sg.device_status() == sg.OK
+        for (dA, dB, dC, a, b), (A, B, C, _, _) in zip(specs, host):
+            A = A * np.float32(scale)
+            if split == 1:
+                want = oracle.sgemm_basic(A, B, C, a, b, basic=False)
+            else:
+                # partial sums over whole 32-deep blocks, added in split order
+                nk = -(-A.shape[1] // 32)
+                step = 32 * -(-nk // min(split, nk))
+                parts = [oracle.sgemm_basic(A[:, k:k + step].copy(), B[k:k + step].copy(),
+                                            np.zeros_like(C), 1.0, 0.0, basic=False)
+                         for k in range(0, A.shape[1], step)]
+                acc = parts[0]
+                for x in parts[1:]:
+                    acc = acc + x
+                # beta 0.5: C * beta is exact, so one rounding from 64 bits is the FMA's
+                t = torch.from_numpy(acc * np.float32(a)).double()
+                if b != 0:
+                    t = t + torch.from_numpy(C).double() * b
+                want = t.float().numpy()
+            assert np.array_equal(dC.cpu().numpy(), want), f"{A.shape}x{B.shape}"
+    plan.close()
+
+
 def test_grouped_graph_replay_equals_direct():
     torch = _torch()
     specs, host = _make(SHAPES, 200, _lds())
