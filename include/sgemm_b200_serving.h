@@ -48,7 +48,8 @@ extern "C" {
 typedef struct sgemm_b200_server sgemm_b200_server;
 
 typedef struct {
-    size_t hbm_budget_bytes;  /* device pool size */
+    size_t hbm_budget_bytes;  /* device pool size (launches may hold up to an eighth of it more,
+                                 for operands they prepare) */
     int slots;                /* batches that may be in flight at once (streams) */
     int max_batch;            /* most requests in one batch */
     int path;                 /* sgemm_b200_path */

@@ -701,15 +701,23 @@ static int make_preps(const Schedule& sc, float* scratch, std::vector<GPrep>* ou
     return tiles;
 }
 
-// No scratch to be had: every problem is read in place.
-static void read_in_place(Schedule* sc) {
+// At most `floats` of scratch: problems whose prepared matrices do not fit beside
+// those before them are read in place.
+static void limit_scratch(Schedule* sc, size_t floats) {
+    size_t used = 0;
     for (GProblem& g : sc->probs) {
         if (g.load != kLoadTransposed) continue;
+        const size_t need =
+            prep_floats(g.op.k, g.op.m) + (g.pack_b ? prep_floats(g.op.k, g.op.n) : 0);
+        if (need <= floats - used) {
+            used += need;
+            continue;
+        }
         const bool ok = tma_ok(g.op.k, g.op.A, g.op.lda, g.op.B, g.op.ldb);
         g.load = ok ? kLoadRows : kLoadAsync4;
         g.pack_b = 0;
     }
-    sc->scratch_floats = 0;
+    sc->scratch_floats = used;
 }
 
 // The tensor maps of one problem: an (A, B) pair for each tile shape it uses,
@@ -802,7 +810,7 @@ static int build_plan(const sgemm_b200_problem* probs, int count, const Table& t
                                              (cudaStream_t)0) != cudaSuccess) {
             cudaGetLastError();
             plan->d_scratch = nullptr;
-            read_in_place(&sc);
+            limit_scratch(&sc, 0);
         }
     }
     std::vector<GPrep> preps;
@@ -922,9 +930,9 @@ static int launch(sgemm_b200_grouped_plan* plan, cudaStream_t stream, int use_gr
 
 template <class T>
 static cudaError_t grow(T** d, T** h, size_t* cap, size_t need, cudaStream_t s,
-                        size_t min_cap) {
+                        size_t min_cap, size_t max_cap = SIZE_MAX) {
     if (need <= *cap) return cudaSuccess;
-    const size_t n = std::max({need, *cap * 2, min_cap});
+    const size_t n = std::min(std::max({need, *cap * 2, min_cap}), max_cap);
     if (*d) cudaFreeAsync(*d, s);
     *d = nullptr;
     *cap = 0;
@@ -960,10 +968,13 @@ int arena_launch(Arena* a, const sgemm_b200_problem* probs, int count, cudaStrea
     chk(grow<float>(&a->d_ws, nullptr, &a->cap_ws, std::max<size_t>(sc.ws_floats, 1), stream,
                     1));
     if (e != cudaSuccess) return cuda_status(e);
-    if (sc.scratch_floats && grow<float>(&a->d_scratch, nullptr, &a->cap_scratch,
-                                         sc.scratch_floats, stream, 1 << 22) != cudaSuccess) {
+    const size_t limit = a->scratch_limit / sizeof(float);
+    limit_scratch(&sc, limit);
+    if (sc.scratch_floats &&
+        grow<float>(&a->d_scratch, nullptr, &a->cap_scratch, sc.scratch_floats, stream,
+                    (size_t)1 << 22, limit) != cudaSuccess) {
         cudaGetLastError();
-        read_in_place(&sc);
+        limit_scratch(&sc, 0);
     }
     std::vector<GPrep> preps;
     const int prep_tiles = make_preps(sc, a->d_scratch, &preps);

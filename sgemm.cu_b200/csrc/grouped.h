@@ -5,6 +5,9 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <cstddef>
+#include <cstdint>
+
 #include "../../include/sgemm_b200.h"
 
 namespace sgb {
@@ -29,6 +32,9 @@ struct Arena {
     CUtensorMap* h_maps = nullptr;
     size_t cap_probs = 0, cap_items = 0, cap_maps = 0, cap_counters = 0, cap_ws = 0,
            cap_scratch = 0, cap_preps = 0;
+    // Bytes of prepared operands a launch may hold (problems beyond them are read
+    // in place).
+    size_t scratch_limit = SIZE_MAX;
 };
 
 // Schedule `count` problems (built-in choices, no split-K) and launch one

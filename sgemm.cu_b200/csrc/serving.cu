@@ -8,8 +8,8 @@
 //  - one worker thread admits requests in arrival order while their operands
 //    fit in the pool (generating them on an ingest stream), forms a batch
 //    whenever one of `slots` streams is free, and launches it: one persistent
-//    grouped FFMA kernel (plain path) or one grouped split pre-pass and one
-//    persistent grouped tcgen05 kernel (split paths), followed by an event on
+//    grouped FFMA kernel (plain path) or persistent grouped tcgen05 kernels (split
+//    paths), each after a pass that prepares operands, followed by an event on
 //    the slot's stream;
 //  - one completion thread polls the events of the batches in flight
 //    (cudaEventQuery, about every 20 us, asleep while nothing is in flight),
@@ -407,7 +407,7 @@ static int launch_batch(Server* s, int si) {
         }
         st = grouped::arena_launch(&sl.arena, probs.data(), (int)probs.size(), sl.stream);
     } else if (st == SGEMM_B200_OK) {
-        // one grouped pre-pass and one persistent tcgen05 launch for the batch
+        // one grouped split launch for the batch
         std::vector<sgemm_b200_problem> probs(sl.batch.size());
         std::vector<void*> ws(sl.batch.size());
         for (size_t i = 0; i < sl.batch.size(); ++i) {
@@ -577,6 +577,8 @@ extern "C" int sgemm_b200_server_create(sgemm_b200_server** out,
     if (e == cudaSuccess) e = cudaEventCreate(&s->epoch);
     s->slots.resize(cfg->slots);
     for (int i = 0; i < cfg->slots && e == cudaSuccess; ++i) {
+        // prepared operands live beside the budget: an eighth of it for all slots
+        s->slots[i].arena.scratch_limit = cfg->hbm_budget_bytes / 8 / cfg->slots;
         e = cudaStreamCreateWithFlags(&s->slots[i].stream, cudaStreamNonBlocking);
         if (e == cudaSuccess) e = cudaEventCreate(&s->slots[i].ev_start);
         if (e == cudaSuccess) e = cudaEventCreate(&s->slots[i].ev_end);

@@ -112,3 +112,25 @@ def test_isolated_time_and_wait():
     rid = srv.submit(256, 256, 256, seed=1)
     assert srv.wait(rid) > 0
     srv.close()
+
+
+# An eighth of the budget, over the slots, holds operands that a batch prepares: for
+# 300 x 520 x 1001 about 1.2 MB of A and 2.1 MB of B (its strides are odd).
+@pytest.mark.parametrize("budget", [1 << 16, 3 << 20, 24 << 20, 1 << 28])
+def test_prepared_operands_stay_within_their_share_of_the_budget(budget):
+    """The same bits whether none, some or all of a batch's operands are prepared."""
+    torch = _torch()
+    srv = sg.Server(budget, slots=1, max_batch=16, path="plain")
+    cases = []
+    for i, (m, n, k) in enumerate([(300, 520, 1001), (257, 640, 512), (300, 520, 1001)]):
+        A, B, C = (oracle.fill(*s, 900 + i, t, 0) for t, s in ((1, (m, k)), (2, (k, n)), (3, (m, n))))
+        pad = 0 if i == 1 else 2
+        cases.append((A, B, C, _padded(A, pad), _padded(B, pad), _padded(C, 0)))
+    torch.cuda.synchronize()
+    for _, _, _, dA, dB, dC in cases:
+        srv.submit_device(dA, dB, dC, 1.5, 0.5)
+    srv.drain()
+    srv.close()
+    assert sg.device_status() == sg.OK
+    for A, B, C, _, _, dC in cases:
+        assert np.array_equal(dC.cpu().numpy(), _want("plain", A, B, C, 1.5, 0.5))
