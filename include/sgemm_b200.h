@@ -68,8 +68,11 @@ typedef enum {
  * C = fmaf(C_old, beta, acc), so results equal the reference kernels' bit for
  * bit on the same inputs.  After one call on the device outside stream
  * capture (which caches the device's properties and the library pool), calls
- * can be captured into a CUDA graph, including ones whose unaligned strides
- * take the pack-to-aligned-rows path (its scratch is stream-ordered). */
+ * can be captured into a CUDA graph, including ones that prepare operands
+ * first: large problems read a transposed copy of A, and unaligned strides are
+ * copied to aligned rows (the scratch, 4 m k bytes and the copies', is
+ * stream-ordered from the library's pool; without it a call reads its operands
+ * in place, with the same result). */
 int sgemm_b200(int m, int n, int k,
                const float* alpha,
                const float* A, int lda,
@@ -97,9 +100,9 @@ const char* sgemm_b200_config_name(int cfg);
  * pointers when C is read (beta != 0); host-only.  C and ldc are not used
  * (kept for callers of the first form of this query).  Strides that TMA
  * cannot describe (not a multiple of 4 floats, or a base not 16-byte aligned)
- * on problems of at least 512^3 are first copied to aligned rows (see
- * sgemm_b200_packs), so the answer is then a TMA configuration; smaller such
- * problems use a cp.async configuration. */
+ * on problems of at least 32e6 multiply-adds (317^3) are first copied to
+ * aligned rows (see sgemm_b200_packs), so the answer is then a TMA
+ * configuration; smaller such problems use a cp.async configuration. */
 int sgemm_b200_select_config(int m, int n, int k,
                              const float* A, int lda,
                              const float* B, int ldb,
@@ -158,9 +161,14 @@ size_t sgemm_b200_split_workspace_size(int path, int m, int n, int k);
 /* C := alpha*A*B + beta*C with A and B split into BF16 (path BF16X6) or TF32
  * (path TF32X3) terms whose cross products run on tcgen05 with FP32
  * accumulation in tensor memory.  Same argument meaning as sgemm_b200.
- * workspace may be NULL, in which case the call allocates it stream-ordered
- * on `stream` from a memory pool the library keeps per device (freed blocks
- * are reused by later calls). */
+ * A workspace receives the operands' split planes.  It may be NULL, in which
+ * case the call takes what it needs stream-ordered on `stream` from a memory pool
+ * the library keeps per device (freed blocks are reused by later calls): nothing
+ * for outputs of up to about 2000 x 2000 with aligned strides, whose kernel splits
+ * the operands itself, else the planes or aligned copies.  Small outputs are also
+ * computed in several slabs of k whose sums are added in order; how many depends
+ * on path, m, n and k alone, so a problem's result does not depend on the
+ * workspace, the strides or the entry point. */
 int sgemm_b200_split(int path, int m, int n, int k,
                      const float* alpha,
                      const float* A, int lda,
@@ -180,6 +188,7 @@ int sgemm_b200_split(int path, int m, int n, int k,
  * deployments that must not fail for lack of memory at run time.
  *
  * Same arguments and result as sgemm_b200_split, but the split operand planes
+ * (or aligned copies, where the kernel splits the operands itself)
  * go to one static device array inside this library instead of a workspace:
  * the call makes no cudaMalloc, cudaFree or other allocation.  The array
  * (64 MiB of planes plus 1 KiB of base alignment) exists on every GPU that
@@ -300,7 +309,9 @@ typedef struct sgemm_b200_grouped_plan sgemm_b200_grouped_plan;
 int sgemm_b200_grouped_plan_create(sgemm_b200_grouped_plan** plan,
                                    const sgemm_b200_problem* problems, int count,
                                    const char* tuning_json);
-/* One persistent launch over every problem of the plan on `stream`.
+/* One persistent launch over every problem of the plan on `stream` (after a pass
+ * that prepares operands in scratch the plan holds: a transposed copy of A where
+ * that pays, aligned copies where strides need them).
  * use_graph != 0 replays a CUDA graph captured on the first call.  A plan
  * holds its own work-ticket counters, so launches of one plan must not
  * overlap on the GPU: order them on one stream (distinct plans may run
@@ -330,10 +341,10 @@ int sgemm_b200_grouped_schedule(const sgemm_b200_problem* problems, int count,
 
 /* Grouped split-precision GEMM (no reference counterpart): every problem of
  * the table -- C := alpha*A*B + beta*C, each with sgemm_b200's argument
- * meaning -- through one grouped pre-pass launch that writes all problems'
- * BF16 (path BF16X6) or TF32 (path TF32X3) planes, and one launch of a
- * persistent tcgen05 kernel over the 128 x 256 tiles of all problems
- * (per-problem tensor maps, longest tiles first).  Each problem's result
+ * meaning -- through at most one grouped pre-pass and two persistent tcgen05
+ * kernels (per-problem tensor maps, longest tiles first): one that splits the
+ * operands itself, and one over 128 x 256 tiles from the BF16 (path BF16X6) or
+ * TF32 (path TF32X3) planes the pre-pass wrote.  Each problem's result
  * equals sgemm_b200_split's on its own, bit for bit.  Workspace for the
  * planes and the launch tables come stream-ordered from the library's pool
  * and are released after the kernels.  Problems with k == 0 run on the plain

@@ -38,6 +38,10 @@
 //
 // A split pre-pass writes the operand planes (A as [split][M][Kp], B
 // transposed to [split][N][Kp], both K-major) into a workspace.
+//
+// Outputs of fewer tiles than about 2000 x 2000 are faster on split_fused.cuh's
+// kernel, which reads FP32 and splits in the SM; route() chooses, and cuts k into
+// slabs where tiles alone would leave SMs idle.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -726,9 +730,10 @@ static int launch_fused(int m, int n, int k, float alpha, const float* A, int ld
 
 // ------------------------------------------------------- grouped split GEMM --
 //
-// Many split-precision problems in two launches: one pre-pass that writes
-// every problem's planes, and one persistent tcgen05 kernel over the tiles of
-// all problems.  Per problem: two tensor maps (A planes, B planes) in global
+// Many split-precision problems: the fused kernel's persistent form for those
+// grouped_classes() gives it, and for the others, here, two launches: one pre-pass
+// that writes their planes, and one persistent tcgen05 kernel over all their
+// tiles.  Per problem: two tensor maps (A planes, B planes) in global
 // memory, and its own epilogue scalars.  Each tile is computed exactly as
 // split_gemm_kernel computes it (same planes, same MMA order, same K chunks of
 // D1, same epilogue), so every problem's result equals sgemm_b200_split's bit

@@ -437,8 +437,8 @@ def grouped_sequential(problems, stream=None) -> None:
 
 
 def grouped_split(path, problems, stream=None) -> None:
-    """All problems through one grouped split pre-pass and one persistent
-    tcgen05 launch (path 'bf16x6' or 'tf32x3')."""
+    """All problems through one grouped split launch: a pre-pass where needed and
+    persistent tcgen05 kernels (path 'bf16x6' or 'tf32x3')."""
     p = PATHS[path] if isinstance(path, str) else int(path)
     _check(lib().sgemm_b200_grouped_split(p, problems, len(problems), _stream_ptr(stream)),
            "grouped_split")
