@@ -387,8 +387,9 @@ int sgemm_b200_fill_random(float* X, int rows, int cols, int ld,
 /* Bytes the library's own stream-ordered memory pool on the current device
  * holds for live allocations (*used_bytes) and keeps reserved from the driver
  * (*reserved_bytes).  The pool backs the scratch the library allocates itself:
- * split workspaces when the caller passes none, packed copies of unaligned
- * operands, and the host-operand path's staging.  Both are 0 before any call
+ * split workspaces when the caller passes none, operands prepared for a kernel
+ * (transposed copies of A, aligned copies; a grouped plan holds its own until it is
+ * destroyed), and the host-operand path's staging.  Both are 0 before any call
  * on the device has created the pool; the query never creates it. */
 int sgemm_b200_pool_usage(size_t* used_bytes, size_t* reserved_bytes);
 

@@ -637,14 +637,26 @@ __global__ void __launch_bounds__(THREADS, 1) split_fused_grouped_kernel(const G
                 quarter(nt, warp, r0, count);
                 float* sum = gp.sums + (int64_t)cta * TN * NT_MAX + r0 * TN + 32 * (warp & 3) +
                              lane;
+                // eight loads in flight, and no store between them: a load, an add and
+                // a store per row cost a trip to L2 each
+                if (s > 0) {
 #pragma unroll
-                for (int j = 0; j < CQ; ++j) {
-                    if (j < count) {
-                        if (s > 0) acc[j] = __fadd_rn(sum[j * TN], acc[j]);
-                        if (s + 1 < splits) sum[j * TN] = acc[j];
+                    for (int j0 = 0; j0 < CQ; j0 += 8) {
+                        float before[8];
+#pragma unroll
+                        for (int e = 0; e < 8; ++e)
+                            before[e] = j0 < count ? __ldcg(sum + (j0 + e) * TN) : 0.0f;
+#pragma unroll
+                        for (int e = 0; e < 8; ++e)
+                            acc[j0 + e] = __fadd_rn(before[e], acc[j0 + e]);
                     }
                 }
-                if (s + 1 < splits) return true;
+                if (s + 1 < splits) {
+#pragma unroll
+                    for (int j = 0; j < CQ; ++j)
+                        if (j < count) __stcg(sum + j * TN, acc[j]);
+                    return true;
+                }
             }
             store_column(p, nt, tl.m0, tl.n0, warp, lane, acc);
             return true;
