@@ -616,21 +616,26 @@ struct Route {
 };
 
 // Modelled times in microseconds, from B200 timings.  Fused kernel: a block of 32
-// k takes a + b NT per CTA (NT rows of the tile), SMs take whole rounds of CTAs.
-// Pre-pass and 128 x 256 tiles: the planes' bytes, and 0.93 us (BF16X6) or 1.0 us
-// (TF32X3) per block of 32 k and round.
+// k takes a + b NT per CTA (NT rows of the tile), SMs take whole rounds of CTAs (1%
+// more per round: the power cap).  Pre-pass and 128 x 256 tiles: the planes' bytes,
+// and 0.93 us (BF16X6; 1.16 where the planes' rows do not start on 128 bytes) or 1.0
+// us (TF32X3) per block of 32 k and round.  Both sides measured (fused, planes):
+// BF16X6 1536^3 36, 66; 1800^3 80, 103; 2048^3 99, 95; 2500^3 198, 282; 3000^3 281,
+// 367; 3500^3 534, 464; 4096^3 795, 767.  TF32X3 1536^3 39, 77; 2048^3 99, 107 to
+// 104; 2300^3 166, 202; 3000^3 352, 311.
 static Route route(int path, int m, int n, int k) {
     const bool bf = path == SGEMM_B200_PATH_BF16X6;
     const double sms = 148;
     const int tiles_m = div_up(m, fused::NT_MAX), nt = div_up(div_up(m, tiles_m), 16) * 16;
     const int tiles = tiles_m * div_up(n, fused::TN), chunks = div_up(k, KCHUNK);
-    const double block = bf ? 0.43 + 0.0023 * nt : 0.58 + 0.0027 * nt;
+    const double block = bf ? 0.235 + 0.0033 * nt : 0.33 + 0.0034 * nt;
     Route best{true, 1};
     double best_t = 1e300;
     for (int s = 1; s <= 8; s *= 2) {
         if (s > 1 && (div_up(chunks, s) * (s - 1) >= chunks || tiles * s > 148)) break;
-        const double t = 4.0 + (s > 1 ? 2.5 : 0.0) +
-                         std::ceil(tiles * s / sms) * div_up(chunks, s) * (KCHUNK / 32) * block;
+        const double rounds = std::ceil(tiles * s / sms);
+        const double t = 4.0 + (s > 1 ? 2.5 : 0.0) + rounds * (0.99 + 0.01 * rounds) *
+                                                         div_up(chunks, s) * (KCHUNK / 32) * block;
         if (t < best_t * 0.95) {
             best_t = t;
             best.splits = s;
@@ -638,7 +643,8 @@ static Route route(int path, int m, int n, int k) {
     }
     const double planes = (double(m) + n) * k * (bf ? 10.0 : 12.0) / 4.5e6;
     const double tiles256 = std::ceil(double(div_up(m, BM)) * div_up(n, BN) / sms);
-    const double t_planes = 10.0 + planes + tiles256 * div_up(k, 32) * (bf ? 0.93 : 1.0);
+    const double t_planes = 10.0 + planes +
+                            tiles256 * div_up(k, 32) * (!bf ? 1.0 : k % 64 == 0 ? 0.93 : 1.16);
     if (t_planes < best_t) best = Route{false, 1};
     return best;
 }
@@ -1137,13 +1143,24 @@ struct GroupedTables {
 
 static size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
+// What tiles of a grouped launch cost, in microseconds of an SM (B200 timings): a
+// fused tile of nt rows over `blocks` blocks of 32 k in `splits` slabs, a 128 x 256
+// tile from planes, and per element of A and B the planes' traffic (time of every
+// SM).
+static double fused_tile_us(bool bf, int nt, double blocks, int splits) {
+    return bf ? (0.235 + 0.0033 * nt) * blocks + 8.0 + 4.0 * (splits - 1)
+              : (0.5 + 0.0024 * nt) * blocks + 2.0 * splits;
+}
+static double planes_tile_us(bool bf, double blocks, bool beta) {
+    return bf ? 0.93 * blocks + 8.0 + (beta ? 8.0 : 0.0) : blocks + 3.0;
+}
+static double planes_us(bool bf, double elements) { return elements * (bf ? 4.0e-6 : 2.7e-6); }
+
 // Which problems of a grouped launch the fused kernel computes (the others come
-// from planes; a problem of several slabs is always fused).  Modelled in
-// microseconds from B200 timings: a fused 128 x NT tile takes 0.43 + 0.0023 NT per
-// block of 32 k, a 128 x 256 one 0.93, a slab about 2 more, and the planes' bytes
-// occupy every SM.  The two kernels run one after the other, each as long as its
-// dearest tile or its share of the SMs, so it is either everything fused or every
-// problem on the kernel that takes it fewer SM-microseconds.
+// from planes; a problem of several slabs is always fused).  The two kernels run one
+// after the other, each as long as its dearest tile or its share of the SMs, so it
+// is either everything fused or every problem on the kernel that takes it fewer
+// SM-microseconds.
 static std::vector<char> grouped_classes(int path, const sgemm_b200_problem* pr, int count) {
     const bool bf = path == SGEMM_B200_PATH_BF16X6;
     struct Phase {
@@ -1163,11 +1180,11 @@ static std::vector<char> grouped_classes(int path, const sgemm_b200_problem* pr,
         const int splits = route(path, q.m, q.n, q.k).splits;
         const int tiles_m = div_up(q.m, fused::NT_MAX), nt = div_up(div_up(q.m, tiles_m), 16) * 16;
         const double blocks = div_up(q.k, 32);
-        const double ft = blocks * (bf ? 0.43 + 0.0023 * nt : 0.5 + 0.0024 * nt) + 2.0 * splits;
+        const double ft = fused_tile_us(bf, nt, blocks, splits);
         const double f = double(tiles_m) * div_up(q.n, fused::TN);
-        const double pt = blocks * (bf ? 0.93 : 1.0) + 3.0;
+        const double pt = planes_tile_us(bf, blocks, q.beta != 0.0f);
         const double p = double(div_up(q.m, BM)) * div_up(q.n, BN);
-        const double bytes = (double(q.m) + q.n) * q.k * (bf ? 10.0 : 12.0) / 4.5e6;
+        const double bytes = planes_us(bf, (double(q.m) + q.n) * q.k);
         all[i] = 1;
         all_fused.add(f, ft);
         mixed[i] = splits > 1 || f * ft < p * pt + 148.0 * bytes;
@@ -1216,7 +1233,8 @@ static int add_fused(const sgemm_b200_problem& q, void* ws, int splits, GroupedT
     gt->fmaps.push_back(maps[0]);
     gt->fmaps.push_back(maps[1]);
     gt->fsums = gt->fsums || splits > 1;
-    const double c = div_up(q.k, fused::BK) * (0.43 + 0.0023 * g.nt) + 2.0 * splits;
+    const double c = fused_tile_us(PATH == SGEMM_B200_PATH_BF16X6, g.nt,
+                                   div_up(q.k, fused::BK), splits);
     for (int b = 0; b < div_up(q.n, fused::TN); ++b)
         for (int a = 0; a < tiles_m; ++a) {
             gt->ftiles.push_back(fused::GTile{idx, a * g.nt, b * fused::TN, 0});
