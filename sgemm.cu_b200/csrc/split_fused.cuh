@@ -24,13 +24,13 @@
 //               per MMA, against 16-64 of work)
 // TMEM (512 columns): D1 twice and D2 (NT each), then two buffers of B's planes
 // (48 columns each, or 64 for TF32).
-// What bounds it (B200, SM cycles): a block of 32 k takes ~1000 cycles at NT = 32
-// and ~1300 at NT = 128, whose MMAs take 200-770; the rest is the split itself
+// What bounds it (B200, SM cycles): a block of 32 k takes ~660 cycles at NT = 32
+// and ~1230 at NT = 128, whose MMAs take 200-770; the rest is the split itself
 // (ALU issue and the chain load, convert, store) and, at NT = 128, shared memory
 // (each element is landed and read, A's planes written and read by every MMA).
 // Measured per call, BF16X6, against pre-pass and 128 x 256 tiles: 24 x 4096 x 4096
-// 20 us from 161, 136 x 4096 x 4096 41 from 164, 1000^3 18 from 68, 512^3 11.5 from
-// 33, 64 x 64 x 4096 13.6 from 128; at 2048^3 the two meet (92 us).
+// 18.5 us from 161, 136 x 4096 x 4096 38.6 from 164, 1000^3 17.3 from 68, 512^3 11.5
+// from 33, 64 x 64 x 4096 13.3 from 128; at 2048^3 the two meet (95 us).
 #pragma once
 
 namespace fused {
