@@ -467,7 +467,8 @@ __device__ __forceinline__ void epilogue_staged(const Operands& p, int m0, int n
     }
 }
 
-// Barrier over the compute warps only (the producer warp, if any, has left).
+// Barrier over the compute warps only (the producer warp, if any, has left).  For
+// kernels whose warps leave together when a wait expires.
 template <class C>
 __device__ __forceinline__ void compute_barrier() {
     if constexpr (C::TMA)
@@ -545,15 +546,21 @@ __device__ __forceinline__ void acc_move(const Operands& p, const float* in, flo
     }
 }
 
-// The end of a tile: the unscaled sums to acc_out, or the epilogue to C.
-template <class C>
+// The end of a tile: the unscaled sums to acc_out, or the epilogue to C.  `released`
+// waits until every compute warp is done reading the stage ring, where the staged
+// epilogue parks its tile; false (in this lane) when its bounded wait expired.
+template <class C, class Released>
 __device__ __forceinline__ void finish_tile(const Params& p, int m0, int n0, int wm, int wn,
                                             int lm, int ln, float (&acc)[C::TM][C::TN],
-                                            uint8_t* smem) {
-    if (p.acc_out)
+                                            uint8_t* smem, Released released) {
+    if (p.acc_out) {
         acc_move<C, true>(p.op, nullptr, p.acc_out, p.ld_acc, m0, n0, wm, wn, lm, ln, acc);
-    else
-        epilogue_any<C>(p.op, m0, n0, wm, wn, lm, ln, acc, smem);
+    } else if (p.op.vec_c) {
+        epilogue<C>(p.op, m0, n0, wm, wn, lm, ln, acc);
+    } else if (released()) {
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        epilogue_staged<C>(p.op, m0, n0, wm, wn, lm, ln, warp, lane, acc, smem);
+    }
 }
 
 template <class C>
@@ -644,7 +651,16 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
             __syncwarp();
             if (lane == 0) mbar_arrive(&empty_bar[s]);  // this warp is done with the stage
         }
-        finish_tile<C>(p, m0, n0, wm, wn, lm, ln, acc, smem);
+        // A warp whose wait expired has left, so the others don't meet it at a
+        // hardware barrier, which would wait for it without end: the arrivals on the
+        // last block's empty barrier say the same, and that wait is bounded.
+        finish_tile<C>(p, m0, n0, wm, wn, lm, ln, acc, smem, [&] {
+            const int last = nk - 1;
+            const bool ok =
+                nk == 0 || mbar_wait(&empty_bar[last % C::STAGES], (last / C::STAGES) & 1);
+            if (!ok) atomicExch(p.status, SGEMM_B200_ERR_TIMEOUT);
+            return ok;
+        });
     } else {
         grid_wait();
         const int wm = warp / C::WN, wn = warp % C::WN;
@@ -682,7 +698,10 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
             compute_stage<C>(st, st + C::A_BYTES, a_base, xa0, xa1, b_base, acc);
         }
         cp_async_wait<0>();
-        finish_tile<C>(p, m0, n0, wm, wn, lm, ln, acc, smem);
+        finish_tile<C>(p, m0, n0, wm, wn, lm, ln, acc, smem, [] {
+            __syncthreads();
+            return true;
+        });
     }
 }
 

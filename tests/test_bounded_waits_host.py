@@ -1,0 +1,54 @@
+"""CPU tests, by reading the kernel sources, that a bounded wait stays bounded.
+
+A wait on an mbarrier gives up after a limit (test_failure_gpu.py); what its warp
+does next must not leave other threads at a barrier that has no limit.  Such a
+hang must not be brought about on a GPU, so these tests read the code.
+"""
+import os
+import re
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "sgemm.cu_b200",
+                    "csrc")
+
+
+def _code(name):
+    """The file without comments."""
+    with open(os.path.join(CSRC, name)) as f:
+        text = re.sub(r"/\*.*?\*/", "", f.read(), flags=re.S)
+    return re.sub(r"//[^\n]*", "", text)
+
+
+def _body(code, head):
+    """The braces of the first function (or block) whose head matches."""
+    at = re.search(head, code)
+    assert at, head
+    i = code.index("{", at.end())
+    depth = 0
+    for j in range(i, len(code)):
+        depth += {"{": 1, "}": -1}.get(code[j], 0)
+        if depth == 0:
+            return code[i:j + 1]
+    raise AssertionError(head)
+
+
+def _reaches(code, body, what, seen=()):
+    """Whether `what` is in the body or in a function template it calls."""
+    if what in body:
+        return True
+    for name in set(re.findall(r"\b(\w+)<C[^;(]*>\(", body)) - set(seen):
+        head = r"void\s+" + name + r"\("
+        if re.search(head, code) and _reaches(code, _body(code, head), what, (*seen, name)):
+            return True
+    return False
+
+
+def test_plain_tile_warps_that_leave_alone_meet_no_hardware_barrier():
+    """A compute warp of a TMA tile returns by itself when its wait expires, so none
+    of the code its siblings go on to holds a bar.sync."""
+    code = _code("ffma_kernel.cuh")
+    kernel = _body(code, r"ffma_gemm_kernel\(")
+    tma = _body(kernel, r"if constexpr \(C::TMA\)")
+    after_loop = tma[tma.index("return;"):]  # the producer's end: compute warps from here
+    assert "mbar_wait" in after_loop and "finish_tile" in after_loop
+    assert not re.search(r"__syncthreads\s*\(|bar\.sync", after_loop)
+    assert not _reaches(code, after_loop, "bar.sync")

@@ -117,6 +117,17 @@ def test_seven_row_thread_tile_bit_exact(name, m, n, k, ldc, ab):
     _assert_equal(got, oracle.sgemm_basic(A, B, C, *ab, basic=False))
 
 
+@pytest.mark.parametrize("cfg", [i for i, n in enumerate(sg.config_names())
+                                 if n.startswith("tma_")])
+def test_staged_epilogue_waits_for_every_warp(cfg):
+    # C rows that are not 16-byte aligned are parked in the stage ring, which every
+    # warp must have read out: no block, one, a ring not full, full and wrapped twice
+    for k in (0, 4, 64, 400, 900):
+        A, B, C = _inputs(139, 270, k, 13, 0)
+        got = _run_ours(A, B, C, 1.5, 0.5, lds=(max(k, 4), 272, 271), config=cfg)
+        _assert_equal(got, oracle.sgemm_basic(A, B, C, 1.5, 0.5, basic=False))
+
+
 @pytest.mark.parametrize("name", ["tma_128x64_w4_t8x8_s3", "tma_28x256_w4p_t7x8_s3",
                                   "tma_64x64_w4_t8x4_at", "tma_32x64_w4_t4x4_at"])
 @pytest.mark.parametrize("m,n,k", [(1, 4, 4), (27, 260, 68), (29, 132, 64), (65, 68, 132),
