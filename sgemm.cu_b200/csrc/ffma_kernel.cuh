@@ -548,7 +548,7 @@ __device__ __forceinline__ void acc_move(const Operands& p, const float* in, flo
 
 // The end of a tile: the unscaled sums to acc_out, or the epilogue to C.  `released`
 // waits until every compute warp is done reading the stage ring, where the staged
-// epilogue parks its tile; false (in this lane) when its bounded wait expired.
+// epilogue parks its tile; false (in the whole warp) when a bounded wait expired.
 template <class C, class Released>
 __device__ __forceinline__ void finish_tile(const Params& p, int m0, int n0, int wm, int wn,
                                             int lm, int ln, float (&acc)[C::TM][C::TN],
@@ -659,7 +659,7 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
             const bool ok =
                 nk == 0 || mbar_wait(&empty_bar[last % C::STAGES], (last / C::STAGES) & 1);
             if (!ok) atomicExch(p.status, SGEMM_B200_ERR_TIMEOUT);
-            return ok;
+            return __all_sync(0xffffffffu, ok) != 0;  // the warp leaves as a whole
         });
     } else {
         grid_wait();
