@@ -129,7 +129,22 @@ struct Barriers {
     uint64_t raw_full[RAWS_MAX], raw_empty[RAWS_MAX];
     uint64_t op_full[G], op_empty[G];
     uint64_t d1_full[2], d1_empty[2], d2_empty;
+    volatile int gone;  // a wait has expired
 };
+
+// A split warp's wait.  A lane whose wait expires stays with its warp, which goes on
+// (in bounds, on what it finds) to the chunk's vote on `gone` (convert); waits that
+// come before that no longer last.  A vote per wait instead costs 1-2% of a call.
+__device__ __forceinline__ void wait_or_gone(Barriers& b, uint64_t* bar, uint32_t parity) {
+    if (mbar_try_wait(bar, parity)) return;
+    const uint64_t t0 = globaltimer_ns();
+    while (!mbar_try_wait(bar, parity)) {
+        if (b.gone || globaltimer_ns() - t0 > kWaitLimitNs) {
+            b.gone = 1;
+            return;
+        }
+    }
+}
 
 // Where a CTA keeps things: operand buffers, landing stages (A [nt][32 k], then
 // B [32 k][128 n]) and tensor-memory columns (D1 at 0 and dcols, D2 at 2 dcols,
@@ -170,11 +185,14 @@ __device__ __forceinline__ void init_barriers(Barriers& b) {
         mbar_init(&b.d1_empty[s], SPLIT_WARPS);
     }
     mbar_init(&b.d2_empty, SPLIT_WARPS);
+    b.gone = 0;
 }
 
 // The roles, each over the nb k blocks of one slab of one tile.  Counters that
 // give the barriers' phases run on from slab to slab.  They return false when a
-// bounded wait expired.
+// bounded wait expired, a whole warp's role in all its lanes, by a vote: a lane that
+// left alone would leave its warp short in the collective instructions (votes,
+// tensor-memory loads and stores) ahead.
 
 // TMA producer (one lane).
 template <int PATH>
@@ -184,7 +202,9 @@ __device__ __forceinline__ bool produce(const Place& pl, Barriers& b, const CUte
     const uint32_t bytes = Lay<PATH>::raw_bytes(nt);
     for (int i = 0; i < nb; ++i, ring.next(), ++issued) {
         if (issued >= pl.raws) {
-            if (!mbar_wait(&b.raw_empty[ring.stage], ring.phase ^ 1)) return false;
+            // A warp arrives also when its wait for the stage expired (wait_or_gone): the
+            // copy may be in flight, and raw_full must not be armed twice in a phase.
+            if (!mbar_wait(&b.raw_empty[ring.stage], ring.phase ^ 1) || b.gone) return false;
             fence_proxy_async_shared();  // the warps' reads before the TMA refill
         }
         uint8_t* st = pl.raw + ring.stage * pl.raw_stride;
@@ -214,14 +234,12 @@ __device__ __forceinline__ bool multiply(const Place& pl, Barriers& b, int nt, i
                                         : sw128_kmajor_desc(smem_u32(pl.ops));
     const uint32_t plane16 = static_cast<uint32_t>(nt * L::ROW) >> 4;
     const uint32_t d2 = pl.tmem + 2 * pl.dcols;
-    if (slab > 0) {  // D2 of the slab before has been read
-        if (!mbar_wait(&b.d2_empty, (slab - 1) & 1)) return false;
-        tc_fence_after();
-    }
+    bool ok = true;  // of this lane's waits; the warp votes before it goes on
+    if (slab > 0) ok = mbar_wait(&b.d2_empty, (slab - 1) & 1);  // D2 of the slab before is read
     for (int i = 0; i < nb; ++i, ++g) {
         const int s = g % G;
         const bool start = i % CHUNK_BLOCKS == 0;  // D1 restarts
-        bool ok = mbar_wait(&b.op_full[s], (g / G) & 1);
+        if (ok) ok = mbar_wait(&b.op_full[s], (g / G) & 1);
         if (ok && start && cg >= 2) ok = mbar_wait(&b.d1_empty[cg & 1], ((cg >> 1) - 1) & 1);
         if (!__all_sync(0xffffffffu, ok)) return false;
         tc_fence_after();
@@ -295,7 +313,8 @@ __device__ __forceinline__ bool convert(const Place& pl, Barriers& b, int nt, in
         }
     };
     auto drain_chunk = [&] {
-        if (!mbar_wait(&b.d1_full[cg & 1], (cg >> 1) & 1)) return false;
+        wait_or_gone(b, &b.d1_full[cg & 1], (cg >> 1) & 1);
+        if (!__all_sync(0xffffffffu, !b.gone)) return false;
         tc_fence_after();
         drain((cg & 1) * pl.dcols);
         tc_fence_before();
@@ -307,7 +326,7 @@ __device__ __forceinline__ bool convert(const Place& pl, Barriers& b, int nt, in
     int left = (nb + CHUNK_BLOCKS - 1) / CHUNK_BLOCKS;  // chunks to drain
     int due = CHUNK_BLOCKS + G - 1;  // the block by which the next chunk is known done
     for (int i = (group ^ g) & 1; i < nb; i += G) {
-        if (!mbar_wait(&b.raw_full[ring.stage], ring.phase)) return false;
+        wait_or_gone(b, &b.raw_full[ring.stage], ring.phase);
         const uint8_t* ra = pl.raw + ring.stage * pl.raw_stride;
         const float* rb =
             reinterpret_cast<const float*>(ra + nt * BK * 4) + 16 * h * TN + q * 32 + lane;
@@ -336,7 +355,7 @@ __device__ __forceinline__ bool convert(const Place& pl, Barriers& b, int nt, in
                 }
             }
             if (st == 0 && g + i >= G) {  // the buffer's previous block has been multiplied
-                if (!mbar_wait(&b.op_empty[group], (((g + i) / G) - 1) & 1)) return false;
+                wait_or_gone(b, &b.op_empty[group], (((g + i) / G) - 1) & 1);
                 tc_fence_after();
             }
 #pragma unroll

@@ -7,6 +7,8 @@ hang must not be brought about on a GPU, so these tests read the code.
 import os
 import re
 
+import pytest
+
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "sgemm.cu_b200",
                     "csrc")
 
@@ -52,3 +54,29 @@ def test_plain_tile_warps_that_leave_alone_meet_no_hardware_barrier():
     assert "mbar_wait" in after_loop and "finish_tile" in after_loop
     assert not re.search(r"__syncthreads\s*\(|bar\.sync", after_loop)
     assert not _reaches(code, after_loop, "bar.sync")
+
+
+@pytest.mark.parametrize("head", [r"bool multiply\(", r"bool convert\("])
+def test_fused_split_roles_leave_as_whole_warps(head):
+    """The fused split kernel's whole-warp roles go through collective instructions
+    (votes, tensor-memory loads and stores), so no lane leaves on its own wait: a
+    role returns false only where the warp has voted."""
+    body = _body(_code("split_fused.cuh"), head)
+    assert "__all_sync(" in body
+    for leave in re.finditer(r"return false|\bbreak\b", body):
+        before = body[:leave.start()].rsplit("\n", 1)[-1]
+        if before.strip() == "if (u >= nt * 4)":  # the end of a loop without collectives
+            continue
+        assert re.search(r"if \(!(__all_sync\(0xffffffffu, \S+\)|drain_chunk\(\))\) $", before)
+
+
+def test_fused_split_producer_arms_no_barrier_twice():
+    """A split warp whose wait expired goes on to its chunk's vote and arrives on the
+    way; the producer then issues no more copies, since the one that the warp gave up
+    on may still be in flight on the same barrier."""
+    code = _code("split_fused.cuh")
+    produce = _body(code, r"bool produce\(")
+    wait = produce.index("raw_empty")
+    assert re.match(r"raw_empty[^;]*\|\| b\.gone\) return false;", produce[wait:])
+    assert wait < produce.index("mbar_arrive_expect_tx")
+    assert "b.gone = 1" in _body(code, r"void wait_or_gone\(")
