@@ -542,6 +542,7 @@ constexpr int kTransposeMinN = 512;
 constexpr double kTransposeMinWork = 32.0e6;  // m n k
 
 static int load_of(const sgemm_b200_problem& p) {
+    if (p.m == 0 || p.n == 0) return kLoadAsync4;  // no items, and no map over nothing
     const bool in_place = tma_ok(p.k, p.A, p.lda, p.B, p.ldb);
     const double work = double(p.m) * p.n * p.k;
     if (in_place)

@@ -351,3 +351,27 @@ def test_autotuner_beats_default_on_k_heavy_problems(tmp_path):
         assert torch.allclose(C.double(), want, rtol=0, atol=1e-5 * want.abs().max().item())
     default.close()
     tuned.close()
+
+
+@pytest.mark.parametrize("use_graph", [True, False])
+def test_empty_problems_beside_others(use_graph):
+    """A problem without rows or columns, whatever its strides, is no work and no
+    error: the others of its table are computed."""
+    torch = _torch()
+    shapes = [(0, 64, 100), (300, 520, 1001), (64, 0, 100), (0, 640, 1000), (640, 0, 1000),
+              (0, 0, 64), (129, 512, 512), (0, 513, 1001)]
+    lds = [(104, 64, 64), None, (101, 3, 1), (1001, 641, 641), (1000, 4, 4), (64, 1, 1), None,
+           (1001, 513, 513)]
+    lds = [l or (None, None, None) for l in lds]
+    specs, host = _make(shapes, 700, lds)
+    plan = sg.GroupedPlan(specs)
+    plan.launch(use_graph=use_graph)
+    torch.cuda.synchronize()
+    assert sg.device_status() == sg.OK
+    for (dA, dB, dC, a, b), (A, B, C, _, _) in zip(specs, host):
+        if C.size:
+            assert np.array_equal(dC.cpu().numpy(), oracle.sgemm_basic(A, B, C, a, b, basic=False))
+    plan.close()
+    only = sg.GroupedPlan([specs[0], specs[4]])
+    only.launch(use_graph=use_graph)
+    only.close()
