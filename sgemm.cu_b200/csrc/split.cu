@@ -519,11 +519,7 @@ static size_t workspace_bytes(int m, int n, int k, size_t* a_bytes_out = nullptr
     const size_t b = (size_t)T::NSPLIT * n * kp * T::ESZ;
     const size_t a_al = (a + 1023) / 1024 * 1024;
     if (a_bytes_out) *a_bytes_out = a_al;
-    // planes, or copies of the operands at 16-byte-aligned rows (the larger only for
-    // a few columns); + alignment slack for the base
-    const size_t rows = sizeof(float) * ((size_t)m * ((k + 3) / 4 * 4) +
-                                         (size_t)k * ((n + 3) / 4 * 4));
-    return std::max(a_al + b, rows) + 1024;
+    return a_al + b + 1024;  // + alignment slack for the base
 }
 
 template <int PATH>
@@ -1130,6 +1126,7 @@ struct GroupedTables {
     std::vector<CUtensorMap> fmaps;
     std::vector<PackJob> packs;
     std::vector<int> p_prefix;
+    std::vector<int> alone;  // problems for a launch of their own, from planes
     bool fsums = false;  // some fused problem has several slabs
     size_t off_fprobs = 0, off_ftiles = 0, off_fmaps = 0, off_packs = 0, off_ppref = 0;
     std::vector<GSProblem> probs;
@@ -1261,6 +1258,14 @@ static int grouped_tables(const sgemm_b200_problem* pr, void* const* ws,
         }
         if (fused[i]) {
             const int splits = route(PATH, q.m, q.n, q.k).splits;
+            // Aligned copies may take more than the workspace's planes for a product
+            // of up to 6 rows and columns together; the grouped planes kernel has no
+            // slabs, split_gemm_kernel does.
+            if (packed(q.m, q.n, q.k, q.A, q.lda, q.B, q.ldb, nullptr).bytes >
+                workspace_bytes<PATH>(q.m, q.n, q.k)) {
+                gt.alone.push_back(i);
+                continue;
+            }
             const int st = add_fused<PATH>(q, ws[i], splits, &gt, &fcost);
             if (st != SGEMM_B200_OK) return st;
             continue;
@@ -1495,6 +1500,13 @@ static int grouped_arena_launch(Arena* a, const sgemm_b200_problem* probs, void*
         if (st == SGEMM_B200_OK) st = grouped_enqueue<PATH>(gt, a->d, a->sums, stream);
         if (st != SGEMM_B200_OK) return st;
     }
+    for (int i : gt.alone) {
+        const sgemm_b200_problem& q = probs[i];
+        st = launch<PATH>(q.m, q.n, q.k, q.alpha, q.A, q.lda, q.B, q.ldb, q.beta, q.C, q.ldc,
+                          route(PATH, q.m, q.n, q.k).splits, ws[i],
+                          workspace_bytes<PATH>(q.m, q.n, q.k), stream);
+        if (st != SGEMM_B200_OK) return st;
+    }
     for (int i : gt.k_zero) {  // C := beta * C
         const sgemm_b200_problem& q = probs[i];
         st = plain_launch(-1, q.m, q.n, 0, q.alpha, q.A, q.lda, q.B, q.ldb, q.beta, q.C, q.ldc,
@@ -1673,6 +1685,12 @@ static int grouped_oneshot(const sgemm_b200_problem* probs, int count, cudaStrea
                                              stream));
         if (st == SGEMM_B200_OK)
             st = grouped_enqueue<PATH>(gt, d, reinterpret_cast<float*>(d + sums), stream);
+    }
+    for (size_t z = 0; st == SGEMM_B200_OK && z < gt.alone.size(); ++z) {
+        const sgemm_b200_problem& q = probs[gt.alone[z]];
+        st = launch<PATH>(q.m, q.n, q.k, q.alpha, q.A, q.lda, q.B, q.ldb, q.beta, q.C, q.ldc,
+                          route(PATH, q.m, q.n, q.k).splits, wsp[gt.alone[z]],
+                          workspace_bytes<PATH>(q.m, q.n, q.k), stream);
     }
     for (size_t z = 0; st == SGEMM_B200_OK && z < gt.k_zero.size(); ++z) {
         const sgemm_b200_problem& q = probs[gt.k_zero[z]];

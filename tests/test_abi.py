@@ -210,3 +210,16 @@ def test_ctypes_mirrors_match_the_c_layout(mirror, c_name, header, tmp_path):
     assert got[0] == ctypes.sizeof(mirror)
     for f, off in zip(fields, got[1:]):
         assert off == getattr(mirror, f).offset, f
+
+
+@pytest.mark.parametrize("path,planes,esz", [("bf16x6", 3, 2), ("tf32x3", 2, 4)])
+def test_split_workspace_is_the_planes_size(path, planes, esz):
+    """A workspace holds the operands' planes and nothing else, also where copies of
+    thin operands at aligned rows would be larger: the no-allocation entry point
+    accepts what fits its array by this size."""
+    for m, n, k in ((1, 1, 5_500_000), (1, 1, 1), (2, 3, 1_000_001), (700, 900, 1024)):
+        kp = (k + 7) // 8 * 8
+        a = (planes * m * kp * esz + 1023) // 1024 * 1024
+        assert sg.split_workspace_size(sg.PATHS[path], m, n, k) == \
+            a + planes * n * kp * esz + 1024
+    assert sg.split_workspace_size(sg.PATHS["bf16x6"], 1, 1, 5_500_000) <= (64 << 20) + 1024

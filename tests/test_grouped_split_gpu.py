@@ -122,3 +122,20 @@ def test_grouped_split_kernel_mix(path, pad):
         sg.gemm(path, A, B, want, alpha, beta)
         torch.cuda.synchronize()
         assert torch.equal(C, want), (A.shape, B.shape)
+
+
+@pytest.mark.parametrize("path", PATHS)
+def test_grouped_split_thin_unaligned_problems(path):
+    """Products of a few rows and columns whose operands, copied to aligned rows, take
+    more than their planes, in one k slab and in several, beside an ordinary one."""
+    torch = _torch()
+    shapes = [(1, 1, 4096), (300, 200, 700), (2, 1, 5001), (1, 3, 100), (5, 1, 40000), (1, 1, 3)]
+    specs, c0 = _make(shapes, 1400)
+    sg.grouped_split(path, sg.make_problems(specs))
+    torch.cuda.synchronize()
+    assert sg.device_status() == sg.OK
+    for (A, B, C, alpha, beta), C0 in zip(specs, c0):
+        want = C0.clone()
+        sg.gemm(path, A, B, want, alpha, beta)
+        torch.cuda.synchronize()
+        assert torch.equal(C, want), (A.shape, B.shape)

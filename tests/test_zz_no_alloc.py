@@ -167,3 +167,22 @@ def test_noalloc_refuses_problems_beyond_its_scratch():
     assert _call_noalloc("bf16x6", A, A, C, 1.0, 0.0) == sg.ERR_NO_MEMORY
     torch.cuda.synchronize()
     assert bool((C == 7.0).all())  # nothing ran
+
+
+@pytest.mark.parametrize("path,m,n,k", [("bf16x6", 1, 1, 5_500_000), ("bf16x6", 2, 1, 3_500_001),
+                                        ("tf32x3", 1, 1, 4_000_000)])
+def test_noalloc_accepts_long_thin_products(path, m, n, k):
+    """Products whose planes fit the array but whose operands, copied to aligned rows,
+    would not."""
+    import torch
+
+    A, B = torch.empty((m, k), device="cuda"), torch.empty((k, n), device="cuda")
+    C = torch.empty((m, n), device="cuda")
+    for t, X in ((1, A), (2, B), (3, C)):
+        sg.fill_random(X, 47, t, sg.DIST_UNIFORM_PM1)
+    c_new, c_old = C.clone(), C.clone()
+    assert _call_noalloc(path, A, B, c_new, 1.5, 0.5) == sg.OK
+    sg.sgemm_split(path, A, B, c_old, 1.5, 0.5)
+    torch.cuda.synchronize()
+    assert sg.device_status() == sg.OK
+    assert torch.equal(c_new, c_old)
