@@ -142,9 +142,18 @@ cudaMemPool_t library_pool() {
         props.location.type = cudaMemLocationTypeDevice;
         props.location.id = dev;
         cudaMemPool_t p = nullptr;
-        if (cudaMemPoolCreate(&p, &props) != cudaSuccess) return nullptr;
-        uint64_t threshold = ~0ull;
-        cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &threshold);
+        // The first call that needs scratch may be one that a stream captures: creating
+        // a pool is no stream operation, but ends every global-mode capture unless the
+        // thread is in relaxed mode meanwhile.
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        const cudaError_t e = cudaMemPoolCreate(&p, &props);
+        if (e == cudaSuccess) {
+            uint64_t threshold = ~0ull;
+            cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &threshold);
+        }
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (e != cudaSuccess) return nullptr;
         pools[dev] = p;
     }
     return pools[dev];

@@ -1,0 +1,50 @@
+"""GPU tests of calls captured into CUDA graphs: what a capture may be the first to
+need, and what kind of graph comes of it.  The reference launches on the legacy
+stream only (src/sgemm.cuh:33-45), which cannot be captured.
+"""
+import os
+import subprocess
+import sys
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+# A process whose only call outside capture is a small one that needs no scratch,
+# then a captured one that does.
+FIRST_SCRATCH = """
+import sys
+sys.path[:0] = [{root!r} + "/sgemm.cu_b200"]
+import torch
+import sgemm_b200 as sg
+path, size, pad = {path!r}, {size}, {pad}
+small = [torch.rand(64, 64, device="cuda") for _ in range(3)]
+sg.gemm(path, *small)
+A, B, C = (torch.rand(size, size + pad, device="cuda")[:, :size] for _ in range(3))
+torch.cuda.synchronize()
+s = torch.cuda.Stream()
+g = torch.cuda.CUDAGraph()
+with torch.cuda.graph(g, stream=s):
+    sg.gemm(path, A, B, C, 1.0, 0.0, stream=s)
+C.zero_()
+g.replay()
+torch.cuda.synchronize()
+want = torch.empty_like(C)
+sg.gemm(path, A, B, want, 1.0, 0.0)
+torch.cuda.synchronize()
+assert sg.device_status() == sg.OK
+assert torch.equal(C, want)
+print("captured")
+"""
+
+
+@pytest.mark.parametrize("path,size,pad", [("plain", 2048, 0), ("plain", 2001, 0),
+                                           ("plain", 2048, 1), ("bf16x6", 4096, 0),
+                                           ("tf32x3", 1000, 1)])
+def test_first_call_with_scratch_may_be_captured(path, size, pad):
+    r = subprocess.run([sys.executable, "-c",
+                        FIRST_SCRATCH.format(root=ROOT, path=path, size=size, pad=pad)],
+                       capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "captured" in r.stdout, r.stderr[-2000:]
