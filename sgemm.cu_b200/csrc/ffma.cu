@@ -36,16 +36,21 @@ using C12 = Cfg<64, 64, 2, 1, 8, 4, kLoaderAsync4, 3>;
 using C14 = Cfg<128, 64, 4, 1, 8, 3, kLoaderAsync4, 3>;
 using W0 = Cfg<128, 64, 4, 2, 4, 3, kLoaderTma, 2, 8, true>;
 using W1 = Cfg<128, 64, 4, 2, 4, 4, kLoaderTma, 2, 8, true>;
-using P0 = Cfg<128, 64, 4, 1, 8, 3, kLoaderTma, 3, 8, true>;
-using P1 = Cfg<128, 64, 4, 1, 8, 4, kLoaderTma, 2, 8, true>;
+using P0 = Cfg<128, 64, 4, 1, 8, 3, kLoaderTma, 3>;
+using P1 = Cfg<128, 64, 4, 1, 8, 4, kLoaderTma, 2>;
 // 28 x 256 tiles, 7 x 8 outputs per thread: a 1024 x 1024 output is 37 x 4 =
 // 148 tiles, one per SM, each thread doing 56 FMAs per k step where the
 // 128 x 64 tile (128 tiles, 20 SMs idle) does 64; two CTAs fit an SM with 3
 // stages (2048^3: 592 tiles, two full waves).  The one-CTA form keeps A
 // [row][k]: at 1024^3 the transpose costs more than it gives (47.8 against
 // 41.6 us).
+// P0, P1 and T4 keep A [row][k] too, for calls without scratch for the
+// transpose, whose other tiles are small or alone on their SM: 8192^3 18.2 ms on
+// P1, 2048^3 297 us on T4 (16.3 ms and 290 us with A transposed).  T4 is also the
+// faster one for wide A: 8192 x 512 x 8192 1173 us against 1221 on T3.
 using T0 = Cfg<28, 256, 1, 4, 8, 4, kLoaderTma, 1, 7>;
 using T3 = Cfg<28, 256, 1, 4, 8, 3, kLoaderTma, 2, 7, true>;
+using T4 = Cfg<28, 256, 1, 4, 8, 3, kLoaderTma, 2, 7>;
 // Small threads (4 x 2 and 4 x 4 outputs) for outputs too few to give every
 // scheduler an 8-row one: a few rows against a wide B, and squares below
 // ~900.  A 24 x 4096 x 4096 GEMM, whose 64 tiles of 32 x 64 left 84 SMs idle at
@@ -80,17 +85,19 @@ struct ConfigDesc {
     bool km;    // reads A transposed
     int a_box;  // rows of an A box (slots when transposed)
     Cost cost;
+    bool spare;  // only for calls without scratch: its twin on transposed A is faster
     void (*kernel)(const CUtensorMap, const CUtensorMap, const Params);
 };
 
 template <class C>
-constexpr ConfigDesc describe(const char* name, float u, float v, float w) {
+constexpr ConfigDesc describe(const char* name, float u, float v, float w, bool spare = false) {
     return ConfigDesc{name, C::BM, C::BN, C::THREADS, C::SMEM_BYTES, C::LOADER, C::KM,
-                      C::A_BOX, Cost{u, v, w}, &ffma_gemm_kernel<C>};
+                      C::A_BOX, Cost{u, v, w}, spare, &ffma_gemm_kernel<C>};
 }
 
 // u, v, w fitted per configuration to B200 timings of grids of 148 c CTAs,
-// c = 1..8, at k = 1024 and 3072 (the slope gives u c + v, the rest w).
+// c = 1..8, at k = 1024 and 3072 (the slope gives u c + v, the rest w).  T4's w is
+// T0's, so that it leaves problems of one tile per SM to T0 (1024^3 1% faster).
 static const ConfigDesc kConfigs[] = {
     describe<C0>("tma_128x256_w8_t8x16_s4", 321.6f, 1.6f, 3.6f),
     describe<C1>("tma_128x128_w8_t8x8_s3", 142.2f, 1.3f, 2.9f),
@@ -108,8 +115,8 @@ static const ConfigDesc kConfigs[] = {
     describe<C14>("cpa_128x64_w4_t8x8_s3", 118.5f, 27.0f, 1.2f),
     describe<W0>("tma_128x64_w8_t8x4_s3", 75.4f, 1.5f, 0.8f),
     describe<W1>("tma_128x64_w8_t8x4_s4", 75.4f, 1.8f, 0.8f),
-    describe<P0>("tma_128x64_w4p_t8x8_s3", 69.2f, 7.4f, 0.8f),
-    describe<P1>("tma_128x64_w4p_t8x8_s4", 70.3f, 6.5f, 0.8f),
+    describe<P0>("tma_128x64_w4p_t8x8_s3", 81.2f, 10.5f, 0.8f, true),
+    describe<P1>("tma_128x64_w4p_t8x8_s4", 78.1f, 5.4f, 0.8f, true),
     describe<T0>("tma_28x256_w4p_t7x8_s4", 74.5f, 1.0f, 2.4f),
     describe<T3>("tma_28x256_w4p_t7x8_s3", 64.6f, 9.5f, 0.9f),
     describe<K1>("tma_16x32_w2_t4x2", 9.4f, 7.0f, 0.3f),
@@ -122,6 +129,7 @@ static const ConfigDesc kConfigs[] = {
     describe<Q7>("tma_64x64_w4_t8x4_at", 37.8f, 8.6f, 0.6f),
     describe<A2>("cpa_32x32_w4_t4x2_s4", 26.0f, 16.0f, 0.5f),
     describe<A3>("cpa_32x64_w4_t4x4_s4", 41.5f, 22.0f, 0.5f),
+    describe<T4>("tma_28x256_w4p_t7x8_s3_rows", 68.4f, 7.9f, 2.4f),
 };
 constexpr int kNumConfigs = sizeof(kConfigs) / sizeof(kConfigs[0]);
 
@@ -183,7 +191,7 @@ static int select_for_loader(int m, int n, int k, int loader, bool reads_c, bool
     double best_t = 1e300;
     for (int c = 0; c < kNumConfigs; ++c) {
         const ConfigDesc& cd = kConfigs[c];
-        if (cd.loader != loader || (cd.km && !scratch)) continue;
+        if (cd.loader != loader || (scratch ? cd.spare : cd.km)) continue;
         const double t = modelled_us(cd, m, n, k, sms, reads_c);
         if (best < 0 || t < best_t) {
             best_t = t;

@@ -8,6 +8,8 @@ import sys
 
 import pytest
 
+import sgemm_b200 as sg
+
 pytestmark = pytest.mark.gpu
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
@@ -48,3 +50,37 @@ def test_first_call_with_scratch_may_be_captured(path, size, pad):
                         FIRST_SCRATCH.format(root=ROOT, path=path, size=size, pad=pad)],
                        capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and "captured" in r.stdout, r.stderr[-2000:]
+
+
+def _captured(call):
+    """The graph of call(stream) captured in global mode, and its nodes' types."""
+    import torch
+    rt = pytest.importorskip("cuda.bindings.runtime")
+
+    s = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    h = rt.cudaStream_t(s.cuda_stream)
+    assert rt.cudaStreamBeginCapture(
+        h, rt.cudaStreamCaptureMode.cudaStreamCaptureModeGlobal)[0] == 0
+    try:
+        call(s)
+    finally:
+        err, graph = rt.cudaStreamEndCapture(h)
+    assert err == 0
+    err, _, count = rt.cudaGraphGetNodes(graph)
+    err, nodes, count = rt.cudaGraphGetNodes(graph, count)
+    assert err == 0
+    return graph, [rt.cudaGraphNodeGetType(n)[1].name for n in nodes]
+
+
+@pytest.mark.parametrize("name", ["tma_128x64_w4p_t8x8_s3", "tma_128x64_w4p_t8x8_s4",
+                                  "tma_28x256_w4p_t7x8_s3_rows"])
+def test_large_tiles_that_read_a_in_place(name):
+    """Large tiles for calls that have no scratch: one kernel, no transposed copy."""
+    import torch
+
+    A, B, C = (torch.rand(512, 512, device="cuda") for _ in range(3))
+    cfg = sg.config_names().index(name)
+    sg.sgemm(A, B, C, config=cfg)
+    _, kinds = _captured(lambda s: sg.sgemm(A, B, C, config=cfg, stream=s))
+    assert kinds == ["cudaGraphNodeTypeKernel"]
