@@ -216,6 +216,18 @@ int plain_select(int m, int n, int k, const float* A, int lda, const float* B, i
     return select_for_loader(m, n, k, loader, reads_c);
 }
 
+// Whether a call may take scratch.  In a stream capture scratch becomes memory nodes,
+// and a graph that has some cannot be a child graph, nor be instantiated twice: a
+// captured call reads its operands in place, with the same result.  Only unaligned
+// operands from 512^3 multiply-adds on are copied there, too, as they always were.
+static bool scratch_allowed(int mask, int m, int n, int k, cudaStream_t stream) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    const cudaError_t e = cudaStreamIsCapturing(stream, &st);
+    if (e != cudaSuccess) cudaGetLastError();
+    if (e == cudaSuccess && st == cudaStreamCaptureStatusNone) return true;
+    return mask && double(m) * n * k >= 134217728.0;
+}
+
 namespace ffma {
 
 // Operand preparation, one launch for both operands: A transposed for the
@@ -381,14 +393,17 @@ int plain_launch_acc(int cfg, int m, int n, int k, float alpha, const float* A, 
          reinterpret_cast<uintptr_t>(acc_out) % 16 != 0))
         return SGEMM_B200_ERR_INVALID_ARG;
     // carried accumulators: the caller keeps its operands TMA-aligned (no pack step)
-    const int mask = (cfg < 0 && !acc_in && !acc_out) ? pack_mask(m, n, k, A, lda, B, ldb) : 0;
-    const bool chosen = cfg < 0;
-    if (chosen)
+    int mask = (cfg < 0 && !acc_in && !acc_out) ? pack_mask(m, n, k, A, lda, B, ldb) : 0;
+    if (cfg < 0)
         cfg = mask ? select_for_loader(m, n, k, kLoaderTma, beta != 0.0f)
                    : plain_select(m, n, k, A, lda, B, ldb, beta != 0.0f);
     if (cfg >= kNumConfigs) return SGEMM_B200_ERR_INVALID_ARG;
     if (!mask && kConfigs[cfg].loader == kLoaderTma && k > 0 && !tma_ok(A, lda, B, ldb))
         return SGEMM_B200_ERR_INVALID_ARG;
+    if (((kConfigs[cfg].km && k > 0) || mask) && !scratch_allowed(mask, m, n, k, stream)) {
+        mask = 0;
+        cfg = select_in_place(m, n, k, A, lda, B, ldb, beta != 0.0f);
+    }
 
     // Scratch from the library pool, stream-ordered: A transposed for a
     // configuration that reads it so, or operands with strides TMA cannot
@@ -413,7 +428,6 @@ int plain_launch_acc(int cfg, int m, int n, int k, float alpha, const float* A, 
             if (A2) cudaFreeAsync(A2, stream);
             if (B2) cudaFreeAsync(B2, stream);
             cudaGetLastError();
-            if (!chosen) return cuda_status(e);
             return plain_launch_acc(select_in_place(m, n, k, A, lda, B, ldb, beta != 0.0f), m, n, k,
                                     alpha, A, lda, B, ldb, beta, C, ldc, acc_in, acc_out, ld_acc,
                                     stream);

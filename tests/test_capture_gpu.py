@@ -84,3 +84,46 @@ def test_large_tiles_that_read_a_in_place(name):
     sg.sgemm(A, B, C, config=cfg)
     _, kinds = _captured(lambda s: sg.sgemm(A, B, C, config=cfg, stream=s))
     assert kinds == ["cudaGraphNodeTypeKernel"]
+
+
+# The fallback for calls without scratch; odd rows from 512^3 on are copied instead.
+@pytest.mark.parametrize("m,n,k,pad,kinds", [
+    (2048, 2048, 2048, 0, ["Kernel"]), (3000, 3000, 3000, 0, ["Kernel"]),
+    (300, 520, 4096, 0, ["Kernel"]), (401, 401, 401, 0, ["Kernel"]),
+    (2048, 640, 1028, 1, ["Kernel", "Kernel", "MemAlloc", "MemAlloc", "MemAlloc", "MemFree"])])
+def test_captured_plain_calls_need_no_memory_nodes(m, n, k, pad, kinds):
+    """A captured aligned call is one kernel, so its graph can be a child graph and be
+    instantiated twice; the bits are the direct call's."""
+    import torch
+    rt = pytest.importorskip("cuda.bindings.runtime")
+
+    A, B, C = (torch.rand(r, c + pad, device="cuda")[:, :c] for r, c in ((m, k), (k, n), (m, n)))
+    want, C0 = C.clone(), C.clone()
+    sg.sgemm(A, B, want, 1.5, 0.5)
+    graph, got = _captured(lambda s: sg.sgemm(A, B, C, 1.5, 0.5, stream=s))
+    got = {x.replace("cudaGraphNodeType", "") for x in got}
+    assert got == set(kinds)
+    if kinds != ["Kernel"]:
+        return
+    err, parent = rt.cudaGraphCreate(0)
+    assert err == 0 and rt.cudaGraphAddChildGraphNode(parent, None, 0, graph)[0] == 0
+    first, second = rt.cudaGraphInstantiate(parent, 0), rt.cudaGraphInstantiate(graph, 0)
+    assert first[0] == 0 and second[0] == 0
+    for exe in (first[1], second[1]):
+        C.copy_(C0)
+        torch.cuda.synchronize()
+        assert rt.cudaGraphLaunch(exe, rt.cudaStream_t(0))[0] == 0
+        torch.cuda.synchronize()
+        assert torch.equal(C, want)
+    assert sg.device_status() == sg.OK
+
+
+def test_captured_call_of_a_named_tile_needs_no_memory_nodes():
+    """The same where the caller names a tile that reads A transposed."""
+    import torch
+
+    A, B, C = (torch.rand(512, 512, device="cuda") for _ in range(3))
+    cfg = sg.config_names().index("tma_128x64_w4_t8x8_s3")
+    sg.sgemm(A, B, C, config=cfg)
+    _, kinds = _captured(lambda s: sg.sgemm(A, B, C, config=cfg, stream=s))
+    assert kinds == ["cudaGraphNodeTypeKernel"]
