@@ -119,22 +119,16 @@ bool encode_tensor_map_3d(CUtensorMap* map, CUtensorMapDataType dtype, const voi
     return r == CUDA_SUCCESS;
 }
 
-static cudaMemPool_t g_pools[kMaxDevices] = {nullptr};
+// Per device: [0] the library pool, [1] the scratch pool.
+static cudaMemPool_t g_pools[2][kMaxDevices] = {};
 static std::mutex g_pools_mu;
 
-cudaMemPool_t library_pool_if_created() {
+static cudaMemPool_t pool(int which, bool create) {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return nullptr;
     std::lock_guard<std::mutex> lock(g_pools_mu);
-    return g_pools[dev];
-}
-
-cudaMemPool_t library_pool() {
-    cudaMemPool_t* pools = g_pools;
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return nullptr;
-    std::lock_guard<std::mutex> lock(g_pools_mu);
-    if (!pools[dev]) {
+    cudaMemPool_t& pool = g_pools[which][dev];
+    if (!pool && create) {
         cudaMemPoolProps props;
         std::memset(&props, 0, sizeof(props));
         props.allocType = cudaMemAllocationTypePinned;
@@ -149,15 +143,18 @@ cudaMemPool_t library_pool() {
         cudaThreadExchangeStreamCaptureMode(&mode);
         const cudaError_t e = cudaMemPoolCreate(&p, &props);
         if (e == cudaSuccess) {
-            uint64_t threshold = ~0ull;
+            uint64_t threshold = which == 0 ? ~0ull : kScratchKept;
             cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &threshold);
         }
         cudaThreadExchangeStreamCaptureMode(&mode);
         if (e != cudaSuccess) return nullptr;
-        pools[dev] = p;
+        pool = p;
     }
-    return pools[dev];
+    return pool;
 }
+
+cudaMemPool_t library_pool() { return pool(0, true); }
+cudaMemPool_t scratch_pool() { return pool(1, true); }
 
 int check_gemm_args(int m, int n, int k, const float* alpha, const void* A, int lda,
                     const void* B, int ldb, const float* beta, const void* C, int ldc) {
@@ -227,13 +224,16 @@ extern "C" const char* sgemm_b200_last_error_detail(void) { return sgb::g_error_
 extern "C" int sgemm_b200_pool_usage(size_t* used_bytes, size_t* reserved_bytes) {
     if (!used_bytes || !reserved_bytes) return SGEMM_B200_ERR_INVALID_ARG;
     *used_bytes = *reserved_bytes = 0;
-    cudaMemPool_t p = sgb::library_pool_if_created();  // never creates the pool
-    if (!p) return SGEMM_B200_OK;
-    uint64_t used = 0, reserved = 0;
-    cudaError_t e = cudaMemPoolGetAttribute(p, cudaMemPoolAttrUsedMemCurrent, &used);
-    if (e == cudaSuccess) e = cudaMemPoolGetAttribute(p, cudaMemPoolAttrReservedMemCurrent, &reserved);
-    if (e != cudaSuccess) return sgb::cuda_status(e);
-    *used_bytes = (size_t)used;
-    *reserved_bytes = (size_t)reserved;
+    for (int which = 0; which < 2; ++which) {
+        cudaMemPool_t p = sgb::pool(which, false);  // never creates the pool
+        if (!p) continue;
+        uint64_t used = 0, reserved = 0;
+        cudaError_t e = cudaMemPoolGetAttribute(p, cudaMemPoolAttrUsedMemCurrent, &used);
+        if (e == cudaSuccess)
+            e = cudaMemPoolGetAttribute(p, cudaMemPoolAttrReservedMemCurrent, &reserved);
+        if (e != cudaSuccess) return sgb::cuda_status(e);
+        *used_bytes += (size_t)used;
+        *reserved_bytes += (size_t)reserved;
+    }
     return SGEMM_B200_OK;
 }

@@ -56,15 +56,31 @@ bool encode_tensor_map_3d(CUtensorMap* map, CUtensorMapDataType dtype, const voi
                           uint64_t outer_stride_bytes, uint32_t box_inner, uint32_t box_mid,
                           uint32_t box_outer, CUtensorMapSwizzle swizzle);
 
-// Library-owned stream-ordered memory pool of the current device, for
-// scratch the library allocates itself (split-path workspaces when the caller
-// passes none, packed copies of unaligned operands).  Its release threshold is
-// unlimited, so freed blocks are reused by the next call instead of going back
-// to the driver; the caller's default pool is left untouched.
+// Library-owned stream-ordered memory pools of the current device; the caller's
+// default pool is left untouched.
+//  - The library pool: split-path workspaces when the caller passes none, launch
+//    tables and host staging.  Its release threshold is unlimited, so freed blocks
+//    are reused by the next call instead of going back to the driver.
+//  - The scratch pool: operands prepared for a kernel (A transposed, rows copied),
+//    which cost a call nothing but speed to do without.  It keeps kScratchKept
+//    bytes; what it holds beyond that goes back to the driver at the next
+//    synchronisation.
 cudaMemPool_t library_pool();
-// The current device's library pool if a call has created it, else null
-// (never creates it).
-cudaMemPool_t library_pool_if_created();
+cudaMemPool_t scratch_pool();
+// Give back memory of either pool that no stream uses any more.  (cudaFree does, too,
+// but the pool goes on counting the memory as used.)
+inline void pool_free(void* p) {
+    if (!p || cudaFreeAsync(p, (cudaStream_t)0) == cudaSuccess) return;
+    cudaGetLastError();
+    cudaFree(p);
+}
+
+// Most that a call takes to transpose A (16384 x 16384; larger ones are read in
+// place), and most that the pool keeps, for such calls on four streams, and all
+// plans together hold.  Memory beyond what is kept would be mapped anew by each call
+// that is waited for: 20000 x 512 x 20000 takes 7.1 ms, and 45 ms so.
+constexpr size_t kScratchPerCall = size_t(1) << 30;
+constexpr size_t kScratchKept = size_t(4) << 30;
 
 // Shape checks common to every entry point.  Returns SGEMM_B200_OK or
 // SGEMM_B200_ERR_INVALID_ARG.

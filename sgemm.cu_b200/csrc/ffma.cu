@@ -216,6 +216,14 @@ int plain_select(int m, int n, int k, const float* A, int lda, const float* B, i
     return select_for_loader(m, n, k, loader, reads_c);
 }
 
+// Slots of a row of A transposed for configuration cfg, and the copy's bytes.
+static int km_pitch(int cfg, int m) {
+    return ffma::kConfigs[cfg].bm == 28 ? div_up(m, 28) * 32 : (m + 3) / 4 * 4;
+}
+static size_t km_bytes(int cfg, int m, int k) {
+    return sizeof(float) * (size_t)k * km_pitch(cfg, m);
+}
+
 // Whether a call may take scratch.  In a stream capture scratch becomes memory nodes,
 // and a graph that has some cannot be a child graph, nor be instantiated twice: a
 // captured call reads its operands in place, with the same result.  Only unaligned
@@ -404,8 +412,11 @@ int plain_launch_acc(int cfg, int m, int n, int k, float alpha, const float* A, 
         mask = 0;
         cfg = select_in_place(m, n, k, A, lda, B, ldb, beta != 0.0f);
     }
+    // a transposed A larger than kScratchPerCall only in the place of a copy
+    if (kConfigs[cfg].km && k > 0 && !(mask & 1) && km_bytes(cfg, m, k) > kScratchPerCall)
+        cfg = select_for_loader(m, n, k, kLoaderTma, beta != 0.0f, false);
 
-    // Scratch from the library pool, stream-ordered: A transposed for a
+    // Scratch, stream-ordered: A transposed for a
     // configuration that reads it so, or operands with strides TMA cannot
     // describe copied to aligned rows.  Same arithmetic, same bits.
     float *A2 = nullptr, *B2 = nullptr;
@@ -413,16 +424,16 @@ int plain_launch_acc(int cfg, int m, int n, int k, float alpha, const float* A, 
     if (km || mask) {
         const bool sevens = kConfigs[cfg].bm == 28;
         const bool pa = !km && (mask & 1) != 0, pb = (mask & 2) != 0;
-        const int lda2 = km ? (sevens ? div_up(m, 28) * 32 : (m + 3) / 4 * 4)
-                            : (k + 3) / 4 * 4;
+        const int lda2 = km ? km_pitch(cfg, m) : (k + 3) / 4 * 4;
         const int ldb2 = pb ? (n + 3) / 4 * 4 : ldb;
-        const size_t a_bytes = km ? sizeof(float) * (size_t)k * lda2
+        const size_t a_bytes = km ? km_bytes(cfg, m, k)
                                   : pa ? sizeof(float) * (size_t)m * lda2 : 0;
-        cudaMemPool_t pool = library_pool();
+        const size_t b_bytes = pb ? sizeof(float) * (size_t)k * ldb2 : 0;
+        // copies too large to keep in the scratch pool are kept by the library's
+        cudaMemPool_t pool = a_bytes + b_bytes <= kScratchPerCall ? scratch_pool() : library_pool();
         cudaError_t e = pool ? cudaSuccess : cudaErrorMemoryAllocation;
         if (e == cudaSuccess && a_bytes) e = cudaMallocFromPoolAsync(&A2, a_bytes, pool, stream);
-        if (e == cudaSuccess && pb)
-            e = cudaMallocFromPoolAsync(&B2, sizeof(float) * (size_t)k * ldb2, pool, stream);
+        if (e == cudaSuccess && b_bytes) e = cudaMallocFromPoolAsync(&B2, b_bytes, pool, stream);
         if (e != cudaSuccess) {
             // no scratch: the best configuration that reads the operands in place
             if (A2) cudaFreeAsync(A2, stream);

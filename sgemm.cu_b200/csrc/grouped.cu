@@ -498,6 +498,7 @@ struct sgemm_b200_grouped_plan {
     CUtensorMap* d_maps = nullptr;
     float* d_ws = nullptr;
     float* d_scratch = nullptr;  // transposed A (and copied B) of the problems that use them
+    size_t scratch_bytes = 0;    // of kScratchKept
     sgb::grouped::GPrep* d_preps = nullptr;
     int n_preps = 0, prep_tiles = 0;
     int* d_counters = nullptr;
@@ -509,6 +510,16 @@ struct sgemm_b200_grouped_plan {
 namespace sgb {
 namespace grouped {
 
+// Bytes of scratch that a device's plans hold together: at most kScratchKept.
+static size_t g_plan_scratch[64];
+static std::mutex g_plan_scratch_mu;
+
+static void give_plan_scratch(sgemm_b200_grouped_plan* p) {
+    std::lock_guard<std::mutex> lock(g_plan_scratch_mu);
+    if (p->scratch_bytes) g_plan_scratch[p->device] -= p->scratch_bytes;
+    p->scratch_bytes = 0;
+}
+
 static void free_plan(sgemm_b200_grouped_plan* p) {
     if (!p) return;
     if (p->exec) cudaGraphExecDestroy(p->exec);
@@ -516,7 +527,8 @@ static void free_plan(sgemm_b200_grouped_plan* p) {
     if (p->cap_stream) cudaStreamDestroy(p->cap_stream);
     cudaFree(p->d_block);
     cudaFree(p->d_ws);
-    cudaFree(p->d_scratch);  // back to the library pool, after the frees that wait for the device
+    give_plan_scratch(p);
+    pool_free(p->d_scratch);  // after the frees that wait for the device
     delete p;
 }
 
@@ -721,6 +733,16 @@ static void limit_scratch(Schedule* sc, size_t floats) {
     sc->scratch_floats = used;
 }
 
+// Scratch for a new plan beside those of the device's other plans.
+static void take_plan_scratch(sgemm_b200_grouped_plan* plan, Schedule* sc) {
+    if (plan->device < 0 || plan->device >= 64) return limit_scratch(sc, 0);
+    std::lock_guard<std::mutex> lock(g_plan_scratch_mu);
+    size_t& held = g_plan_scratch[plan->device];
+    limit_scratch(sc, (kScratchKept - held) / sizeof(float));
+    plan->scratch_bytes = sizeof(float) * sc->scratch_floats;
+    held += plan->scratch_bytes;
+}
+
 // The tensor maps of one problem: an (A, B) pair for each tile shape it uses,
 // at maps[2 * shape] and maps[2 * shape + 1] (six slots per problem).  `prep`:
 // the problem's prepared matrices (A, then B if it is copied), or null.
@@ -801,17 +823,19 @@ static int build_plan(const sgemm_b200_problem* probs, int count, const Table& t
     plan->ws_floats = (size_t)sc.ws_floats;
     plan->n_counters = 1 + sc.tickets;
 
-    // Scratch from the library pool: a plan made for one launch does not pay a
+    // Scratch from the scratch pool: a plan made for one launch does not pay a
     // cudaMalloc of its operands' size.  On the null stream, whose copies below
-    // end before this call does.
+    // end before this call does.  Within what the other plans leave of kScratchKept.
+    take_plan_scratch(plan, &sc);
     if (sc.scratch_floats) {
-        cudaMemPool_t pool = library_pool();
+        cudaMemPool_t pool = scratch_pool();
         if (!pool || cudaMallocFromPoolAsync(reinterpret_cast<void**>(&plan->d_scratch),
                                              sizeof(float) * sc.scratch_floats, pool,
                                              (cudaStream_t)0) != cudaSuccess) {
             cudaGetLastError();
             plan->d_scratch = nullptr;
             limit_scratch(&sc, 0);
+            give_plan_scratch(plan);
         }
     }
     std::vector<GPrep> preps;
@@ -931,7 +955,7 @@ static int launch(sgemm_b200_grouped_plan* plan, cudaStream_t stream, int use_gr
 
 template <class T>
 static cudaError_t grow(T** d, T** h, size_t* cap, size_t need, cudaStream_t s,
-                        size_t min_cap, size_t max_cap = SIZE_MAX) {
+                        size_t min_cap, cudaMemPool_t pool, size_t max_cap = SIZE_MAX) {
     if (need <= *cap) return cudaSuccess;
     const size_t n = std::min(std::max({need, *cap * 2, min_cap}), max_cap);
     if (*d) cudaFreeAsync(*d, s);
@@ -941,7 +965,6 @@ static cudaError_t grow(T** d, T** h, size_t* cap, size_t need, cudaStream_t s,
         cudaFreeHost(*h);
         *h = nullptr;
     }
-    cudaMemPool_t pool = library_pool();
     if (!pool) return cudaErrorMemoryAllocation;
     cudaError_t e = cudaMallocFromPoolAsync(reinterpret_cast<void**>(d), n * sizeof(T), pool, s);
     if (e == cudaSuccess && h) e = cudaMallocHost(reinterpret_cast<void**>(h), n * sizeof(T));
@@ -961,26 +984,28 @@ int arena_launch(Arena* a, const sgemm_b200_problem* probs, int count, cudaStrea
         if (e == cudaSuccess) e = x;
     };
     const size_t n_counters = 1 + (size_t)sc.tickets;
+    cudaMemPool_t pool = library_pool();
     // first capacities: 256 problems, 64 Ki work items (~1 MB pinned in all)
-    chk(grow(&a->d_probs, &a->h_probs, &a->cap_probs, (size_t)count, stream, 256));
-    chk(grow(&a->d_items, &a->h_items, &a->cap_items, sc.items.size(), stream, 1 << 16));
-    chk(grow(&a->d_maps, &a->h_maps, &a->cap_maps, 6 * (size_t)count, stream, 1536));
-    chk(grow<int>(&a->d_counters, nullptr, &a->cap_counters, n_counters, stream, 1024));
+    chk(grow(&a->d_probs, &a->h_probs, &a->cap_probs, (size_t)count, stream, 256, pool));
+    chk(grow(&a->d_items, &a->h_items, &a->cap_items, sc.items.size(), stream, 1 << 16,
+             pool));
+    chk(grow(&a->d_maps, &a->h_maps, &a->cap_maps, 6 * (size_t)count, stream, 1536, pool));
+    chk(grow<int>(&a->d_counters, nullptr, &a->cap_counters, n_counters, stream, 1024, pool));
     chk(grow<float>(&a->d_ws, nullptr, &a->cap_ws, std::max<size_t>(sc.ws_floats, 1), stream,
-                    1));
+                    1, pool));
     if (e != cudaSuccess) return cuda_status(e);
     const size_t limit = a->scratch_limit / sizeof(float);
     limit_scratch(&sc, limit);
     if (sc.scratch_floats &&
         grow<float>(&a->d_scratch, nullptr, &a->cap_scratch, sc.scratch_floats, stream,
-                    (size_t)1 << 22, limit) != cudaSuccess) {
+                    (size_t)1 << 22, scratch_pool(), limit) != cudaSuccess) {
         cudaGetLastError();
         limit_scratch(&sc, 0);
     }
     std::vector<GPrep> preps;
     const int prep_tiles = make_preps(sc, a->d_scratch, &preps);
     chk(grow(&a->d_preps, &a->h_preps, &a->cap_preps, std::max<size_t>(preps.size(), 1), stream,
-             512));
+             512, pool));
     if (e != cudaSuccess) return cuda_status(e);
     std::memcpy(a->h_probs, sc.probs.data(), sizeof(GProblem) * count);
     std::memcpy(a->h_items, sc.items.data(), sizeof(GItem) * sc.items.size());
@@ -1015,13 +1040,13 @@ int arena_launch(Arena* a, const sgemm_b200_problem* probs, int count, cudaStrea
 }
 
 void arena_release(Arena* a) {
-    cudaFree(a->d_probs);
-    cudaFree(a->d_items);
-    cudaFree(a->d_maps);
-    cudaFree(a->d_counters);
-    cudaFree(a->d_ws);
-    cudaFree(a->d_scratch);
-    cudaFree(a->d_preps);
+    pool_free(a->d_probs);
+    pool_free(a->d_items);
+    pool_free(a->d_maps);
+    pool_free(a->d_counters);
+    pool_free(a->d_ws);
+    pool_free(a->d_scratch);
+    pool_free(a->d_preps);
     cudaFreeHost(a->h_preps);
     cudaFreeHost(a->h_probs);
     cudaFreeHost(a->h_items);

@@ -1533,8 +1533,8 @@ int grouped_launch(Arena* a, int path, const sgemm_b200_problem* probs, void* co
 }
 
 void arena_release(Arena* a) {
-    cudaFree(a->d);
-    cudaFree(a->sums);
+    pool_free(a->d);
+    pool_free(a->sums);
     cudaFreeHost(a->h);
     *a = Arena();
 }
