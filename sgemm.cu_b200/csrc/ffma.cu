@@ -84,6 +84,7 @@ struct ConfigDesc {
     int bm, bn, threads, smem, loader;
     bool km;    // reads A transposed
     int a_box;  // rows of an A box (slots when transposed)
+    int ctas;   // that an SM's shared memory holds
     Cost cost;
     bool spare;  // only for calls without scratch: its twin on transposed A is faster
     void (*kernel)(const CUtensorMap, const CUtensorMap, const Params);
@@ -92,7 +93,8 @@ struct ConfigDesc {
 template <class C>
 constexpr ConfigDesc describe(const char* name, float u, float v, float w, bool spare = false) {
     return ConfigDesc{name, C::BM, C::BN, C::THREADS, C::SMEM_BYTES, C::LOADER, C::KM,
-                      C::A_BOX, Cost{u, v, w}, spare, &ffma_gemm_kernel<C>};
+                      C::A_BOX, 227 * 1024 / (C::SMEM_BYTES + 1024), Cost{u, v, w}, spare,
+                      &ffma_gemm_kernel<C>};
 }
 
 // u, v, w fitted per configuration to B200 timings of grids of 148 c CTAs,
@@ -150,6 +152,14 @@ static cudaError_t set_smem_attribute(int cfg) {
     return cudaSuccess;
 }
 
+// Unaligned operands are copied to aligned rows (one more launch) for the TMA
+// kernels from 512^3 multiply-adds on, and below that, from 317^3 on, where the cost
+// model finds it faster than the 4-byte cp.async loader on the operands in place: on a
+// B200 317^3 takes 10.0 us in place and 321^3 9.4 us copied, 401^3 37.6 and 10.1.  A
+// block copies a row per 0.6 us, however short: 36912 x 48 x 36 takes 14.5 us in place
+// and 35.9 copied.
+constexpr double kPackMinWork = 32.0e6, kPackWork = 134217728.0;  // 317^3, 512^3
+
 static bool tma_ok(const float* A, int lda, const float* B, int ldb) {
     return (lda % 4 == 0) && (ldb % 4 == 0) && (reinterpret_cast<uintptr_t>(A) % 16 == 0) &&
            (reinterpret_cast<uintptr_t>(B) % 16 == 0);
@@ -170,20 +180,31 @@ int plain_config_tile(int cfg, int* bm, int* bn) {
 
 // Modelled time of a problem on a configuration, in microseconds.  Tiles go to
 // whichever SM is free, so the busiest SM runs ceil(tiles / SMs) of them, and
-// once there are many the ends no longer line up.  A configuration that reads A
-// transposed also pays for the transpose (its launch, and its bytes at the rate
-// it runs at).
+// once there are many the ends no longer line up.  With few k steps the other CTAs of
+// an SM do not hide a CTA's fill (2.6 us) and epilogue (0.4 us per 8192 outputs, twice
+// when C is read), and each generation of resident CTAs pays what is left of them.
+// Over 286 problems of 4 to 2000 k steps the pick took 1.5% longer than the fastest
+// configuration so and 3.1% without that (33884 x 4 x 128 29.4 us from 20.7 before the
+// small-thread tiles).  A configuration that reads A transposed also pays for the
+// transpose (its launch, and its bytes at the rate it runs at).
 static double modelled_us(const ffma::ConfigDesc& cd, int m, int n, int k, int sms, bool reads_c) {
     const double per_sm = double(div_up(m, cd.bm)) * div_up(n, cd.bn) / sms;
     const double c = per_sm > 8 ? per_sm + 0.5 : std::ceil(per_sm);
-    const double t = c * cd.cost.w * (reads_c ? 1.6 : 1.0) +
-                     double(k) * (cd.cost.u * c + cd.cost.v) / 1965.0;
+    const double step = double(k) * cd.cost.u / 1965.0;  // a CTA's k steps beside others
+    double ends = c * cd.cost.w * (reads_c ? 1.6 : 1.0);
+    if (cd.ctas > 1 && c > 1) {
+        const double latency = 2.6 + 0.4 * (reads_c ? 2.0 : 1.0) * cd.bm * cd.bn / 8192.0;
+        const double others = std::min<double>(c, cd.ctas) - 1;
+        ends = std::max(ends, std::max(1.0, c / cd.ctas) * (latency - others * step));
+    }
+    const double t = ends + step * c + double(k) * cd.cost.v / 1965.0;
     return cd.km ? t + 3.0 + 8.0 * double(m) * k / 4.5e6 : t;
 }
 
 // The configuration with the smallest modelled time (the first of equals).
 // `scratch`: configurations that read A transposed may be taken.
-static int select_for_loader(int m, int n, int k, int loader, bool reads_c, bool scratch = true) {
+static int select_for_loader(int m, int n, int k, int loader, bool reads_c, bool scratch = true,
+                             double* us = nullptr) {
     using namespace ffma;
     const DeviceInfo& d = device_info();
     const int sms = d.sm_count > 0 ? d.sm_count : 148;
@@ -198,6 +219,7 @@ static int select_for_loader(int m, int n, int k, int loader, bool reads_c, bool
             best = c;
         }
     }
+    if (us) *us = best_t;
     return best;
 }
 
@@ -233,7 +255,7 @@ static bool scratch_allowed(int mask, int m, int n, int k, cudaStream_t stream) 
     const cudaError_t e = cudaStreamIsCapturing(stream, &st);
     if (e != cudaSuccess) cudaGetLastError();
     if (e == cudaSuccess && st == cudaStreamCaptureStatusNone) return true;
-    return mask && double(m) * n * k >= 134217728.0;
+    return mask && double(m) * n * k >= ffma::kPackWork;
 }
 
 namespace ffma {
@@ -292,18 +314,26 @@ __global__ void __launch_bounds__(kPackThreads)
     }
 }
 
-// Work (m*n*k) above which copying unaligned operands to aligned rows (one
-// more launch, about 3 us) and running the TMA kernel beats the 4-byte
-// cp.async loader: on a B200 317^3 takes 10.0 us on the small cp.async tiles
-// and 321^3 9.4 us copied; 401^3 37.6 us on the large ones, 10.1 us copied.
-constexpr double kPackMinWork = 32.0e6;  // 317^3
+static double pack_us(double rows, double elements) {
+    return 3.0 + 0.6 * std::ceil(rows / (8 * 148)) + 8.0 * elements / 4.5e6;
+}
 
 // Operands the plain path copies to aligned rows before its TMA kernel:
 // bit 0 A, bit 1 B; 0 when the kernel reads them in place.
 static int pack_mask(int m, int n, int k, const float* A, int lda, const float* B, int ldb) {
-    if (k <= 0 || tma_ok(A, lda, B, ldb) || double(m) * n * k < kPackMinWork) return 0;
+    const double work = double(m) * n * k;
+    if (k <= 0 || tma_ok(A, lda, B, ldb) || work < kPackMinWork) return 0;
     const bool pa = (lda % 4 != 0) || (reinterpret_cast<uintptr_t>(A) % 16 != 0);
     const bool pb = (ldb % 4 != 0) || (reinterpret_cast<uintptr_t>(B) % 16 != 0);
+    if (work < kPackWork) {
+        double copied = 0, in_place = 0;
+        select_for_loader(m, n, k, kLoaderTma, false, true, &copied);
+        select_for_loader(m, n, k, kLoaderAsync4, false, true, &in_place);
+        copied += pack_us((pa ? double(m) : 0.0) + (pb ? k : 0),
+                          (pa ? double(m) * k : 0.0) + (pb ? double(k) * n : 0.0));
+        // with few k steps the 4-byte loader takes about 1.25 times what the model says
+        if (copied >= 1.25 * in_place) return 0;
+    }
     return (pa ? 1 : 0) | (pb ? 2 : 0);
 }
 

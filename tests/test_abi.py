@@ -223,3 +223,25 @@ def test_split_workspace_is_the_planes_size(path, planes, esz):
         assert sg.split_workspace_size(sg.PATHS[path], m, n, k) == \
             a + planes * n * kp * esz + 1024
     assert sg.split_workspace_size(sg.PATHS["bf16x6"], 1, 1, 5_500_000) <= (64 << 20) + 1024
+
+
+@pytest.mark.parametrize("m,n,k", [(36912, 48, 36), (45212, 192, 4), (46812, 36, 56),
+                                   (58936, 64, 15), (57817, 18, 55), (64, 65536, 17)])
+def test_short_unaligned_rows_are_read_in_place(m, n, k):
+    # copies run at a row per 0.6 us and block: many short rows below 512^3 of work are
+    # up to 2.7 times faster in place
+    l = sg.lib()
+    assert l.sgemm_b200_packs(m, n, k, 16, k | 1, 16, n | 1) == 0
+    c = l.sgemm_b200_select_config_beta(m, n, k, 16, k | 1, 16, n | 1, None)
+    assert sg.config_names()[c].startswith("cpa_")
+    assert l.sgemm_b200_packs(401, 399, 403, 16, 403, 16, 399) == 3  # few rows: copied
+
+
+@pytest.mark.parametrize("m,n,k,slow", [(33884, 4, 128, "tma_32x32_w4_t4x2"),
+                                        (38260, 12, 80, "tma_32x32_w4_t4x2"),
+                                        (29408, 12, 60, "tma_32x32_w4_t4x2"),
+                                        (596, 19928, 4, "tma_64x64_w4_t8x4_s4")])
+def test_dispatch_counts_the_fill_of_few_k_steps(m, n, k, slow):
+    # tiles that were picked and are 13 to 43% slower than the one before them
+    c = sg.lib().sgemm_b200_select_config_beta(m, n, k, 16, k, 16, n, None)
+    assert sg.config_names()[c] != slow
