@@ -181,19 +181,20 @@ int plain_config_tile(int cfg, int* bm, int* bn) {
 // Modelled time of a problem on a configuration, in microseconds.  Tiles go to
 // whichever SM is free, so the busiest SM runs ceil(tiles / SMs) of them, and
 // once there are many the ends no longer line up.  With few k steps the other CTAs of
-// an SM do not hide a CTA's fill (2.6 us) and epilogue (0.4 us per 8192 outputs, twice
-// when C is read), and each generation of resident CTAs pays what is left of them.
-// Over 286 problems of 4 to 2000 k steps the pick took 1.5% longer than the fastest
-// configuration so and 3.1% without that (33884 x 4 x 128 29.4 us from 20.7 before the
-// small-thread tiles).  A configuration that reads A transposed also pays for the
-// transpose (its launch, and its bytes at the rate it runs at).
+// an SM do not hide a CTA's fill (2 us) and epilogue (1 us per 8192 outputs, twice when
+// C is read), and each generation of resident CTAs pays what is left of them.
+// Against the fastest configuration the pick took 1.8% longer over 286 problems
+// of 4 to 2000 k steps, of which 7 were slower than on the tiles of before (2.9% and
+// 15 without that: 596 x 19928 x 4 30.5 us from 27.0), and 1.1% over 278 of 64 to 500.
+// A configuration that reads A transposed also pays for the transpose (its launch,
+// and its bytes at the rate it runs at).
 static double modelled_us(const ffma::ConfigDesc& cd, int m, int n, int k, int sms, bool reads_c) {
     const double per_sm = double(div_up(m, cd.bm)) * div_up(n, cd.bn) / sms;
     const double c = per_sm > 8 ? per_sm + 0.5 : std::ceil(per_sm);
     const double step = double(k) * cd.cost.u / 1965.0;  // a CTA's k steps beside others
     double ends = c * cd.cost.w * (reads_c ? 1.6 : 1.0);
     if (cd.ctas > 1 && c > 1) {
-        const double latency = 2.6 + 0.4 * (reads_c ? 2.0 : 1.0) * cd.bm * cd.bn / 8192.0;
+        const double latency = 2.0 + 1.0 * (reads_c ? 2.0 : 1.0) * cd.bm * cd.bn / 8192.0;
         const double others = std::min<double>(c, cd.ctas) - 1;
         ends = std::max(ends, std::max(1.0, c / cd.ctas) * (latency - others * step));
     }

@@ -237,11 +237,11 @@ def test_short_unaligned_rows_are_read_in_place(m, n, k):
     assert l.sgemm_b200_packs(401, 399, 403, 16, 403, 16, 399) == 3  # few rows: copied
 
 
-@pytest.mark.parametrize("m,n,k,slow", [(33884, 4, 128, "tma_32x32_w4_t4x2"),
+@pytest.mark.parametrize("m,n,k,slow", [(54636, 8, 52, "tma_32x32_w4_t4x2"),
                                         (38260, 12, 80, "tma_32x32_w4_t4x2"),
                                         (29408, 12, 60, "tma_32x32_w4_t4x2"),
                                         (596, 19928, 4, "tma_64x64_w4_t8x4_s4")])
 def test_dispatch_counts_the_fill_of_few_k_steps(m, n, k, slow):
-    # tiles that were picked and are 13 to 43% slower than the one before them
+    # tiles that were picked and are 13 to 38% slower than the ones of before
     c = sg.lib().sgemm_b200_select_config_beta(m, n, k, 16, k, 16, n, None)
     assert sg.config_names()[c] != slow
