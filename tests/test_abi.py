@@ -238,7 +238,6 @@ def test_short_unaligned_rows_are_read_in_place(m, n, k):
 
 
 @pytest.mark.parametrize("m,n,k,slow", [(54636, 8, 52, "tma_32x32_w4_t4x2"),
-                                        (38260, 12, 80, "tma_32x32_w4_t4x2"),
                                         (29408, 12, 60, "tma_32x32_w4_t4x2"),
                                         (596, 19928, 4, "tma_64x64_w4_t8x4_s4")])
 def test_dispatch_counts_the_fill_of_few_k_steps(m, n, k, slow):
