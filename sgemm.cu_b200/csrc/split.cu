@@ -131,7 +131,11 @@ __device__ __forceinline__ void tile_coords(int bid, int tiles_m, int tiles_n, i
     tn = r / gsz;
 }
 
-template <int PATH>
+// SLABS: with the code that adds several slabs.  It costs TF32X3 registers and 3%
+// where there is one slab (B200: 3584^3 513 us without it, 525 with; 4096^3 741, 767;
+// 2048 x 2048 x 16384 803, 827), and BF16X6 nothing (4096^3 706, 697; 8192^3 5017,
+// 4953), which has the one form.
+template <int PATH, bool SLABS>
 __global__ void __launch_bounds__(THREADS, 1)
     split_gemm_kernel(const __grid_constant__ CUtensorMap tmA,
                       const __grid_constant__ CUtensorMap tmB, const Params p) {
@@ -149,11 +153,12 @@ __global__ void __launch_bounds__(THREADS, 1)
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     int tm, tn;
-    const int slab = blockIdx.x % p.splits;
-    tile_coords(blockIdx.x / p.splits, p.tiles_m, p.tiles_n, tm, tn);
+    const int slab = SLABS ? blockIdx.x % p.splits : 0;
+    tile_coords(SLABS ? blockIdx.x / p.splits : blockIdx.x, p.tiles_m, p.tiles_n, tm, tn);
     const int m0 = tm * BM, n0 = tn * BN;
-    const int kb0 = slab * p.blocks;
-    const int nk = min(p.blocks, (p.k + T::BK - 1) / T::BK - kb0);  // k blocks of this slab
+    const int kb0 = SLABS ? slab * p.blocks : 0;
+    const int kb_all = (p.k + T::BK - 1) / T::BK;
+    const int nk = SLABS ? min(p.blocks, kb_all - kb0) : kb_all;  // k blocks of this slab
     const int nsteps = nk * L::STEPS;
     const int nchunks = (nsteps + L::CHUNK_STEPS - 1) / L::CHUNK_STEPS;
 
@@ -293,7 +298,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         if (!ok) {
             abort_s = 1;
             atomicExch(p.status, SGEMM_B200_ERR_TIMEOUT);
-        } else if (!abort_s && p.splits > 1) {
+        } else if (SLABS && !abort_s && p.splits > 1) {
             // The slab's sums, to meet the other slabs' in shared memory (the stage
             // ring, every MMA being done): [row][PART_LD].
             float* part = reinterpret_cast<float*>(smem) + (q * 32 + lane) * PART_LD + h * 128;
@@ -352,7 +357,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         }
     }
 
-    if (p.splits > 1) {
+    if (SLABS && p.splits > 1) {
         // Every CTA of the cluster adds its share of the rows over the slabs, in
         // slab order, as split_fused_kernel does.
         cluster_sync_all();
@@ -580,6 +585,8 @@ static int launch(int m, int n, int k, float alpha, const float* A, int lda, con
 
     // The kernel's shared-memory attribute, once per device; a thread that
     // sees the flag also sees the attribute set.
+    auto one_slab = split_gemm_kernel<PATH, PATH == SGEMM_B200_PATH_BF16X6>;
+    auto kernel = splits > 1 ? split_gemm_kernel<PATH, true> : one_slab;
     static std::atomic<bool> attr_set[64];
     static std::mutex attr_mu;
     const int dev = device_info().device;
@@ -587,18 +594,18 @@ static int launch(int m, int n, int k, float alpha, const float* A, int lda, con
     if (!attr_set[dev].load(std::memory_order_acquire)) {
         std::lock_guard<std::mutex> lock(attr_mu);
         if (!attr_set[dev].load(std::memory_order_relaxed)) {
-            const cudaError_t e = cudaFuncSetAttribute(
-                split_gemm_kernel<PATH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                L::SMEM_BYTES);
-            if (e != cudaSuccess) return cuda_status(e);
+            for (auto f : {one_slab, split_gemm_kernel<PATH, true>}) {
+                const cudaError_t e = cudaFuncSetAttribute(
+                    f, cudaFuncAttributeMaxDynamicSharedMemorySize, L::SMEM_BYTES);
+                if (e != cudaSuccess) return cuda_status(e);
+            }
             attr_set[dev].store(true, std::memory_order_release);
         }
     }
     p.splits = splits;
     p.blocks = div_up(div_up(k, KCHUNK), splits) * (KCHUNK / T::BK);
-    return cuda_status(launch_chained_cluster(splits, split_gemm_kernel<PATH>,
-                                              p.tiles_m * p.tiles_n * splits, THREADS,
-                                              L::SMEM_BYTES, stream, tmA, tmB, p));
+    return cuda_status(launch_chained_cluster(splits, kernel, p.tiles_m * p.tiles_n * splits,
+                                              THREADS, L::SMEM_BYTES, stream, tmA, tmB, p));
 }
 
 // How a problem is computed: `splits` k slabs whose sums are added in slab order,
