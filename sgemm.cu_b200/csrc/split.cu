@@ -277,10 +277,10 @@ __global__ void __launch_bounds__(THREADS, 1)
         for (int j = 0; j < 128; ++j) acc[j] = 0.0f;
         bool ok = true;
         for (int c = 0; c < nchunks; ++c) {
-            if (!mbar_wait(&d1_full_bar, c & 1) || abort_s) {
-                ok = false;
-                break;
-            }
+            // (the warp leaves as a whole: tensor-memory loads take all its lanes)
+            ok = mbar_wait(&d1_full_bar, c & 1) && !abort_s;
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
             tc_fence_after();
 #pragma unroll
             for (int g = 0; g < 4; ++g) {
@@ -298,7 +298,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         if (!ok) {
             abort_s = 1;
             atomicExch(p.status, SGEMM_B200_ERR_TIMEOUT);
-        } else if (SLABS && !abort_s && p.splits > 1) {
+        } else if (SLABS && p.splits > 1) {
             // The slab's sums, to meet the other slabs' in shared memory (the stage
             // ring, every MMA being done): [row][PART_LD].
             float* part = reinterpret_cast<float*>(smem) + (q * 32 + lane) * PART_LD + h * 128;
@@ -311,7 +311,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                 for (int j = 0; j < 32; ++j)
                     part[g * 32 + j] = __fadd_rn(acc[g * 32 + j], __uint_as_float(r[j]));
             }
-        } else if (!abort_s) {
+        } else {
             // D2 is complete: the last D1 commit came after every MMA.
             const int row = m0 + q * 32 + lane;
 #pragma unroll
@@ -949,10 +949,9 @@ __global__ void __launch_bounds__(THREADS, 1) split_grouped_kernel(const GSParam
 #pragma unroll
             for (int j = 0; j < 128; ++j) acc[j] = 0.0f;
             for (int c = 0; c < nchunks; ++c, ++cg) {
-                if (!mbar_wait(&d1_full_bar, cg & 1) || abort_s) {
-                    ok = false;
-                    break;
-                }
+                ok = mbar_wait(&d1_full_bar, cg & 1) && !abort_s;
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
                 tc_fence_after();
 #pragma unroll
                 for (int gq = 0; gq < 4; ++gq) {
@@ -967,7 +966,7 @@ __global__ void __launch_bounds__(THREADS, 1) split_grouped_kernel(const GSParam
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&d1_empty_bar);
             }
-            if (!ok || abort_s) break;
+            if (!ok) break;
             // D2 is complete (the tile's last D1 commit came after its MMAs):
             // read it all, release it to the MMA warp, then store C.  The
             // outputs replace the running sums in place (acc doubles as v).

@@ -80,3 +80,17 @@ def test_fused_split_producer_arms_no_barrier_twice():
     assert re.match(r"raw_empty[^;]*\|\| b\.gone\) return false;", produce[wait:])
     assert wait < produce.index("mbar_arrive_expect_tx")
     assert "b.gone = 1" in _body(code, r"void wait_or_gone\(")
+
+
+@pytest.mark.parametrize("kernel", ["split_gemm_kernel", "split_grouped_kernel"])
+def test_planes_drain_warps_leave_as_whole_warps(kernel):
+    """The drain warps of the kernels on planes read tensor memory with all their lanes:
+    each wait, and the flag another role sets, goes into a vote before they leave."""
+    body = _body(_code("split.cu"), kernel + r"\(")
+    drain = body[body.index("float acc[128];"):body.index("tmem_dealloc")]
+    loads = drain[:drain.rindex("tmem_ld_32x32b_x32")]
+    waits = [w.start() for w in re.finditer(r"mbar_wait\(", loads)]
+    assert len(waits) == 1
+    after = loads[waits[0]:]
+    assert re.match(r"mbar_wait\([^;]*\) && !abort_s;\s*ok = __all_sync\(0xffffffffu, ok\);", after)
+    assert not re.search(r"if \([^;{]*abort_s", loads)
