@@ -170,13 +170,6 @@ def _peaks():
                 "sm_max_mhz": 1965.0}, "fallback"
 
 
-def _transposes(cfg_name: str) -> bool:
-    """Whether the plain path transposes A, one more launch, for a configuration."""
-    in_place = ("tma_64x64_w4_t8x4_s4", "tma_32x64_w2_t8x4_s4", "tma_28x256_w4p_t7x8_s4")
-    small = ("t4x2" in cfg_name or "t4x4" in cfg_name) and not cfg_name.endswith("_at")
-    return cfg_name.startswith("tma_") and cfg_name not in in_place and not small
-
-
 def _traffic(kernel_key: str):
     """DRAM bytes per launch of the dominant kernel from the committed ncu summary."""
     try:
@@ -843,7 +836,8 @@ def run(args):
     flush = torch.empty(int(peaks.get("l2_bytes", 256 << 20)) // 4, device="cuda")
     cfg = sg.select_config(SIZE, SIZE, SIZE, A, SIZE, B, SIZE, beta=BETA)
     cfg_name = sg.config_names()[cfg]
-    packed = sg.packs(SIZE, SIZE, SIZE, A, SIZE, B, SIZE)  # pack step: one more launch
+    packed = sg.packs(SIZE, SIZE, SIZE, A, SIZE, B, SIZE)
+    launches = sg.launches(SIZE, SIZE, SIZE, A, SIZE, B, SIZE, beta=BETA)
 
     # parity sample: C after one GEMM from C0 (checked by the cpu_baseline leg)
     C0_host = C0.cpu().numpy()
@@ -900,7 +894,7 @@ def run(args):
         "p99_ms": round(sorted(ms)[min(len(ms) - 1, int(0.99 * len(ms)))], 4),
         "roofline": roofline,
         "clocks": clk,
-        "gpu_launches": args.steps * (2 if packed or _transposes(cfg_name) else 1),
+        "gpu_launches": args.steps * launches,
         "peaks_source": peak_src,
     }
 

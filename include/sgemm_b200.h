@@ -100,9 +100,9 @@ const char* sgemm_b200_config_name(int cfg);
  * pointers when C is read (beta != 0); host-only.  C and ldc are not used
  * (kept for callers of the first form of this query).  Strides that TMA
  * cannot describe (not a multiple of 4 floats, or a base not 16-byte aligned)
- * on problems of at least 32e6 multiply-adds (317^3) are first copied to
- * aligned rows (see sgemm_b200_packs), so the answer is then a TMA
- * configuration; smaller such problems use a cp.async configuration. */
+ * are first copied to aligned rows where that pays (see sgemm_b200_packs), so
+ * the answer is then a TMA configuration; other such problems use a cp.async
+ * configuration. */
 int sgemm_b200_select_config(int m, int n, int k,
                              const float* A, int lda,
                              const float* B, int ldb,
@@ -118,10 +118,19 @@ int sgemm_b200_select_config_beta(int m, int n, int k,
 
 /* Operands sgemm_b200 copies to aligned rows before its kernel (host-only):
  * bit 0 for A, bit 1 for B, 0 when both are read in place.  The copy is one
- * extra kernel launch for both operands. */
+ * extra kernel launch for both operands.  Always from 512^3 multiply-adds on, and
+ * where it is faster from 317^3 on. */
 int sgemm_b200_packs(int m, int n, int k,
                      const float* A, int lda,
                      const float* B, int ldb);
+
+/* Kernels sgemm_b200 launches for this shape, these pointers and this beta (as in
+ * sgemm_b200_select_config_beta) outside stream capture; host-only.  2 when one
+ * prepares operands first: copies, or A transposed. */
+int sgemm_b200_launches(int m, int n, int k,
+                        const float* A, int lda,
+                        const float* B, int ldb,
+                        const float* beta);
 
 /* Replaces the reference's pre-Ampere texture path (src/sgemm.cuh:49-89,
  * sgemm_texld_128x128x8 in src/kernels/128x128x8_texld.cuh): when lda and ldb

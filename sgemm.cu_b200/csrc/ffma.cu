@@ -247,6 +247,21 @@ static size_t km_bytes(int cfg, int m, int k) {
     return sizeof(float) * (size_t)k * km_pitch(cfg, m);
 }
 
+// A transposed A larger than kScratchPerCall is made only in the place of a copy.
+static bool too_large(int cfg, int mask, int m, int k) {
+    return ffma::kConfigs[cfg].km && k > 0 && !(mask & 1) && km_bytes(cfg, m, k) > kScratchPerCall;
+}
+
+// The configuration that runs, given the operands copied first (pack_mask).
+static int choose(int mask, int m, int n, int k, const float* A, int lda, const float* B, int ldb,
+                  bool reads_c) {
+    const int cfg = mask ? select_for_loader(m, n, k, ffma::kLoaderTma, reads_c)
+                         : plain_select(m, n, k, A, lda, B, ldb, reads_c);
+    return too_large(cfg, mask, m, k)
+               ? select_for_loader(m, n, k, ffma::kLoaderTma, reads_c, false)
+               : cfg;
+}
+
 // Whether a call may take scratch.  In a stream capture scratch becomes memory nodes,
 // and a graph that has some cannot be a child graph, nor be instantiated twice: a
 // captured call reads its operands in place, with the same result.  Only unaligned
@@ -433,9 +448,7 @@ int plain_launch_acc(int cfg, int m, int n, int k, float alpha, const float* A, 
         return SGEMM_B200_ERR_INVALID_ARG;
     // carried accumulators: the caller keeps its operands TMA-aligned (no pack step)
     int mask = (cfg < 0 && !acc_in && !acc_out) ? pack_mask(m, n, k, A, lda, B, ldb) : 0;
-    if (cfg < 0)
-        cfg = mask ? select_for_loader(m, n, k, kLoaderTma, beta != 0.0f)
-                   : plain_select(m, n, k, A, lda, B, ldb, beta != 0.0f);
+    if (cfg < 0) cfg = choose(mask, m, n, k, A, lda, B, ldb, beta != 0.0f);
     if (cfg >= kNumConfigs) return SGEMM_B200_ERR_INVALID_ARG;
     if (!mask && kConfigs[cfg].loader == kLoaderTma && k > 0 && !tma_ok(A, lda, B, ldb))
         return SGEMM_B200_ERR_INVALID_ARG;
@@ -443,8 +456,7 @@ int plain_launch_acc(int cfg, int m, int n, int k, float alpha, const float* A, 
         mask = 0;
         cfg = select_in_place(m, n, k, A, lda, B, ldb, beta != 0.0f);
     }
-    // a transposed A larger than kScratchPerCall only in the place of a copy
-    if (kConfigs[cfg].km && k > 0 && !(mask & 1) && km_bytes(cfg, m, k) > kScratchPerCall)
+    if (too_large(cfg, mask, m, k))
         cfg = select_for_loader(m, n, k, kLoaderTma, beta != 0.0f, false);
 
     // Scratch, stream-ordered: A transposed for a
@@ -538,10 +550,17 @@ extern "C" int sgemm_b200_select_config_beta(int m, int n, int k, const float* A
                                              const float* B, int ldb, const float* beta) {
     if (m <= 0 || n <= 0 || k < 0) return -1;
     const bool reads_c = beta == nullptr || *beta != 0.0f;
-    // the kernel that runs: after a pack step the operands are TMA-aligned
-    if (sgb::ffma::pack_mask(m, n, k, A, lda, B, ldb))
-        return sgb::select_for_loader(m, n, k, sgb::ffma::kLoaderTma, reads_c);
-    return sgb::plain_select(m, n, k, A, lda, B, ldb, reads_c);
+    const int mask = sgb::ffma::pack_mask(m, n, k, A, lda, B, ldb);
+    return sgb::choose(mask, m, n, k, A, lda, B, ldb, reads_c);
+}
+
+extern "C" int sgemm_b200_launches(int m, int n, int k, const float* A, int lda, const float* B,
+                                   int ldb, const float* beta) {
+    if (m <= 0 || n <= 0 || k < 0) return 0;
+    const int cfg = sgemm_b200_select_config_beta(m, n, k, A, lda, B, ldb, beta);
+    const bool prepares = sgb::ffma::pack_mask(m, n, k, A, lda, B, ldb) != 0 ||
+                          (sgb::ffma::kConfigs[cfg].km && k > 0);
+    return prepares ? 2 : 1;
 }
 
 extern "C" int sgemm_b200_select_config(int m, int n, int k, const float* A, int lda,

@@ -124,6 +124,7 @@ def _declare(lib: ctypes.CDLL) -> None:
     d("sgemm_b200_select_config_beta", _I, [_I, _I, _I, _P, _I, _P, _I, _FP])
     d("sgemm_b200_abi_version", _I, [])
     d("sgemm_b200_packs", _I, [_I, _I, _I, _P, _I, _P, _I])
+    d("sgemm_b200_launches", _I, [_I, _I, _I, _P, _I, _P, _I, _FP])
     d("sgemm_b200_basic", _I, _GEMM_ARGS + [_P])
     d("sgemm_b200_texld", _I, _GEMM_ARGS + [_P])
     d("sgemm_b200_split_workspace_size", ctypes.c_size_t, [_I, _I, _I, _I])
@@ -398,6 +399,16 @@ def packs(m: int, n: int, k: int, A=None, lda: int = 0, B=None, ldb: int = 0) ->
     pa = A.data_ptr() if A is not None else 16
     pb = B.data_ptr() if B is not None else 16
     return lib().sgemm_b200_packs(m, n, k, pa, lda or k, pb, ldb or n)
+
+
+def launches(m: int, n: int, k: int, A=None, lda: int = 0, B=None, ldb: int = 0,
+             beta: Optional[float] = None) -> int:
+    """Kernels sgemm() launches outside stream capture: 2 when operands are copied or
+    A is transposed first."""
+    pa = A.data_ptr() if A is not None else 16
+    pb = B.data_ptr() if B is not None else 16
+    return lib().sgemm_b200_launches(m, n, k, pa, lda or k, pb, ldb or n,
+                                     None if beta is None else _f(beta))
 
 
 def selftest_wait_timeout(limit_us: int, stream=None) -> None:

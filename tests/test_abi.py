@@ -244,3 +244,17 @@ def test_dispatch_counts_the_fill_of_few_k_steps(m, n, k, slow):
     # tiles that were picked and are 13 to 38% slower than the ones of before
     c = sg.lib().sgemm_b200_select_config_beta(m, n, k, 16, k, 16, n, None)
     assert sg.config_names()[c] != slow
+
+
+def test_launch_counts():
+    # A transposed or rows copied are a launch more; tiles that read A in place are not,
+    # and neither is an A whose transposed copy would take more than a call's scratch
+    assert sg.launches(8192, 8192, 8192, beta=0.5) == 2
+    assert sg.launches(256, 256, 256) == sg.launches(1024, 1024, 1024) == 1
+    assert sg.launches(3001, 3001, 3001) == 2 and sg.launches(300, 301, 299) == 1
+    assert sg.launches(0, 5, 5) == 0 and sg.launches(5, 5, 0) == 1
+    assert sg.launches(20000, 2048, 20000) == 1 and sg.launches(16384, 2048, 16384) == 2
+    names = sg.config_names()
+    for shape in ((24, 4096, 4096), (768, 768, 768), (8192, 512, 8192), (2048, 2048, 2048)):
+        in_place = names[sg.select_config(*shape, beta=0.0)]
+        assert sg.launches(*shape, beta=0.0) == (2 if in_place == "tma_28x256_w4p_t7x8_s3" else 1)
