@@ -172,12 +172,13 @@ size_t sgemm_b200_split_workspace_size(int path, int m, int n, int k);
  * accumulation in tensor memory.  Same argument meaning as sgemm_b200.
  * A workspace receives the operands' split planes.  It may be NULL, in which
  * case the call takes what it needs stream-ordered on `stream` from a memory pool
- * the library keeps per device (freed blocks are reused by later calls): nothing
- * for outputs of up to about 2000 x 2000 with aligned strides, whose kernel splits
- * the operands itself, else the planes or aligned copies.  Small outputs are also
- * computed in several slabs of k whose sums are added in order; how many depends
- * on path, m, n and k alone, so a problem's result does not depend on the
- * workspace, the strides or the entry point. */
+ * the library keeps per device (freed blocks are reused by later calls), and may run
+ * a kernel that splits the operands itself and needs no planes: which kernel, and
+ * so what it allocates, is the faster one by path, m, n and k, and no bound on one
+ * size tells (sgemm_b200_split_query does).  Small outputs are also computed in
+ * several slabs of k whose sums are added in order; how many depends on path, m, n
+ * and k alone, so a problem's result does not depend on the workspace, the strides
+ * or the entry point. */
 int sgemm_b200_split(int path, int m, int n, int k,
                      const float* alpha,
                      const float* A, int lda,
@@ -186,6 +187,16 @@ int sgemm_b200_split(int path, int m, int n, int k,
                      float* C, int ldc,
                      void* workspace, size_t workspace_bytes,
                      sgemm_b200_stream_t stream);
+
+/* What sgemm_b200_split does with a NULL workspace (host-only): *inside is 1 when its
+ * kernel splits the operands itself and 0 when it runs on planes from a pre-pass,
+ * *slabs the k slabs, *bytes the device memory the call allocates (the planes, or
+ * copies of operands whose strides or bases TMA cannot describe).  All 0 when there
+ * are no products (m, n or k 0). */
+int sgemm_b200_split_query(int path, int m, int n, int k,
+                           const float* A, int lda,
+                           const float* B, int ldb,
+                           int* inside, int* slabs, size_t* bytes);
 
 /* Allocation-free split-precision GEMM.  No counterpart in the reference
  * (which never allocates, and has no split path).
@@ -360,6 +371,12 @@ int sgemm_b200_grouped_schedule(const sgemm_b200_problem* problems, int count,
  * path (C := beta*C).  Stream-ordered; returns without synchronising. */
 int sgemm_b200_grouped_split(int path, const sgemm_b200_problem* problems, int count,
                              sgemm_b200_stream_t stream);
+
+/* Which of the two kernels computes each problem of that launch (host-only):
+ * inside[i] is 1 for the one that splits the operands itself, 0 for the one on planes
+ * (and for a problem without products). */
+int sgemm_b200_grouped_split_query(int path, const sgemm_b200_problem* problems, int count,
+                                   int* inside);
 
 /* The baseline that launch replaces: one sgemm_b200_split call per problem,
  * in order, on `stream`. */

@@ -1733,6 +1733,33 @@ extern "C" int sgemm_b200_grouped_split(int path, const sgemm_b200_problem* prob
     return s;
 }
 
+extern "C" int sgemm_b200_split_query(int path, int m, int n, int k, const float* A, int lda,
+                                      const float* B, int ldb, int* inside, int* slabs,
+                                      size_t* bytes) {
+    if (m < 0 || n < 0 || k < 0 || !inside || !slabs || !bytes ||
+        (path != SGEMM_B200_PATH_BF16X6 && path != SGEMM_B200_PATH_TF32X3))
+        return SGEMM_B200_ERR_INVALID_ARG;
+    *inside = *slabs = 0;
+    *bytes = 0;
+    if (m == 0 || n == 0 || k == 0) return SGEMM_B200_OK;
+    const sgb::split::Route r = sgb::split::route(path, m, n, k);
+    *inside = r.fused;
+    *slabs = r.splits;
+    *bytes = r.fused ? sgb::split::packed(m, n, k, A, lda, B, ldb, nullptr).bytes
+                     : sgemm_b200_split_workspace_size(path, m, n, k);
+    return SGEMM_B200_OK;
+}
+
+extern "C" int sgemm_b200_grouped_split_query(int path, const sgemm_b200_problem* problems,
+                                              int count, int* inside) {
+    if (count < 0 || (count > 0 && (!problems || !inside)) ||
+        (path != SGEMM_B200_PATH_BF16X6 && path != SGEMM_B200_PATH_TF32X3))
+        return SGEMM_B200_ERR_INVALID_ARG;
+    const std::vector<char> fused = sgb::split::grouped_classes(path, problems, count);
+    for (int i = 0; i < count; ++i) inside[i] = fused[i];
+    return SGEMM_B200_OK;
+}
+
 extern "C" int sgemm_b200_grouped_split_sequential(int path, const sgemm_b200_problem* problems,
                                                    int count, sgemm_b200_stream_t stream) {
     if (count < 0 || (count > 0 && !problems)) return SGEMM_B200_ERR_INVALID_ARG;

@@ -128,6 +128,9 @@ def _declare(lib: ctypes.CDLL) -> None:
     d("sgemm_b200_basic", _I, _GEMM_ARGS + [_P])
     d("sgemm_b200_texld", _I, _GEMM_ARGS + [_P])
     d("sgemm_b200_split_workspace_size", ctypes.c_size_t, [_I, _I, _I, _I])
+    d("sgemm_b200_split_query", _I, [_I, _I, _I, _I, _P, _I, _P, _I, ctypes.POINTER(_I),
+                                     ctypes.POINTER(_I), ctypes.POINTER(ctypes.c_size_t)])
+    d("sgemm_b200_grouped_split_query", _I, [_I, _P, _I, ctypes.POINTER(_I)])
     d("sgemm_b200_split", _I, [_I] + _GEMM_ARGS + [_P, ctypes.c_size_t, _P])
     d("sgemm_b200_gemm", _I, [_I] + _GEMM_ARGS + [_P])
     d("sgemm_b200_host", _I, [_I] + _GEMM_ARGS + [_P])
@@ -298,6 +301,17 @@ def split_workspace_size(path: int, m: int, n: int, k: int) -> int:
     return int(lib().sgemm_b200_split_workspace_size(path, m, n, k))
 
 
+def split_query(path, m: int, n: int, k: int, lda: int = 0, ldb: int = 0):
+    """(operands split inside the kernel?, k slabs, bytes allocated) of a split GEMM
+    without a workspace, on 16-byte-aligned bases."""
+    p = PATHS[path] if isinstance(path, str) else int(path)
+    inside, slabs, nbytes = ctypes.c_int(), ctypes.c_int(), ctypes.c_size_t()
+    _check(lib().sgemm_b200_split_query(p, m, n, k, 16, lda or k, 16, ldb or n,
+                                        ctypes.byref(inside), ctypes.byref(slabs),
+                                        ctypes.byref(nbytes)), "split_query")
+    return bool(inside.value), slabs.value, int(nbytes.value)
+
+
 def sgemm_split(path, A, B, C, alpha: float = 1.0, beta: float = 0.0, workspace=None,
                 stream=None) -> None:
     """Split-precision tensor-core GEMM; path is 'bf16x6', 'tf32x3' or the enum."""
@@ -445,6 +459,16 @@ def grouped_sequential(problems, stream=None) -> None:
     """The baseline: one plain sgemm_b200 launch per problem, in order."""
     _check(lib().sgemm_b200_grouped_sequential(problems, len(problems), _stream_ptr(stream)),
            "grouped_sequential")
+
+
+def grouped_split_query(path, problems):
+    """Per problem of grouped_split: whether its operands are split inside the kernel
+    (else by the pre-pass)."""
+    p = PATHS[path] if isinstance(path, str) else int(path)
+    inside = (ctypes.c_int * max(len(problems), 1))()
+    _check(lib().sgemm_b200_grouped_split_query(p, problems, len(problems), inside),
+           "grouped_split_query")
+    return [bool(x) for x in inside[:len(problems)]]
 
 
 def grouped_split(path, problems, stream=None) -> None:

@@ -258,3 +258,20 @@ def test_launch_counts():
     for shape in ((24, 4096, 4096), (768, 768, 768), (8192, 512, 8192), (2048, 2048, 2048)):
         in_place = names[sg.select_config(*shape, beta=0.0)]
         assert sg.launches(*shape, beta=0.0) == (2 if in_place == "tma_28x256_w4p_t7x8_s3" else 1)
+
+
+def test_split_queries():
+    for path in ("bf16x6", "tf32x3"):
+        # few tiles: split inside, in slabs; nothing allocated unless rows are copied
+        assert sg.split_query(path, 64, 64, 4096) == (True, 8, 0)
+        inside, slabs, nbytes = sg.split_query(path, 64, 64, 4096, lda=4097)
+        assert (inside, slabs) == (True, 8) and 64 * 4096 * 4 <= nbytes <= 64 * 4096 * 4 + 1024
+        # many tiles: from planes, in one slab
+        assert sg.split_query(path, 8192, 8192, 8192) == \
+            (False, 1, sg.split_workspace_size(sg.PATHS[path], 8192, 8192, 8192))
+        assert sg.split_query(path, 0, 5, 5) == sg.split_query(path, 5, 5, 0) == (False, 0, 0)
+    with pytest.raises(sg.SgemmError):
+        sg.split_query(sg.PATHS["plain"], 64, 64, 64)
+    table = (sg.Problem * 2)(sg.Problem(64, 64, 4096, 4096, 64, 64, 1.0, 0.0, 16, 16, 16),
+                             sg.Problem(0, 64, 64, 64, 64, 64, 1.0, 0.0, 16, 16, 16))
+    assert sg.grouped_split_query("bf16x6", table) == [True, False]

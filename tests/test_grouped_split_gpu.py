@@ -139,3 +139,32 @@ def test_grouped_split_thin_unaligned_problems(path):
         sg.gemm(path, A, B, want, alpha, beta)
         torch.cuda.synchronize()
         assert torch.equal(C, want), (A.shape, B.shape)
+
+
+@pytest.mark.parametrize("path", PATHS)
+@pytest.mark.parametrize("pad", [0, 3])
+def test_grouped_split_both_kernels_in_one_launch(path, pad):
+    """A table that the rule divides between the kernel on planes and the one that
+    splits inside, so that one launch chains the pre-pass (planes of A and B, and with
+    odd strides row copies), the fused kernel and the planes kernel: each problem's own
+    bits, at tile edges and k remainders of the planes kernel, and over several tiles
+    per CTA."""
+    torch = _torch()
+    shapes = [(3072, 3072, 768), (3070, 3075, 770), (64, 64, 4096), (3072, 3072, 768),
+              (24, 4096, 4096), (200, 700, 1284), (2945, 3073, 1001), (16, 128, 256),
+              (3072, 3072, 768), (3200, 2816, 896), (300, 130, 2100), (64, 0, 32), (50, 70, 0)]
+    specs, c0 = _make(shapes, 1500, pad=pad)
+    probs = sg.make_problems(specs)
+    inside = sg.grouped_split_query(path, probs)
+    assert any(inside) and not all(inside[i] for i, s in enumerate(shapes) if min(s) > 0)
+    sg.grouped_split(path, probs)
+    torch.cuda.synchronize()
+    assert sg.device_status() == sg.OK
+    for (A, B, C, alpha, beta), C0 in zip(specs, c0):
+        want = C0.clone()
+        if A.shape[1]:
+            sg.gemm(path, A, B, want, alpha, beta)
+        else:
+            sg.sgemm(A, B, want, alpha, beta)
+        torch.cuda.synchronize()
+        assert torch.equal(C, want), (A.shape, B.shape)
