@@ -39,9 +39,9 @@
 // A split pre-pass writes the operand planes (A as [split][M][Kp], B
 // transposed to [split][N][Kp], both K-major) into a workspace.
 //
-// Outputs of fewer tiles than about 2000 x 2000 are faster on split_fused.cuh's
-// kernel, which reads FP32 and splits in the SM; route() chooses, and cuts k into
-// slabs where tiles alone would leave SMs idle.
+// Outputs of few tiles, and shapes whose planes are dear, are faster on
+// split_fused.cuh's kernel, which reads FP32 and splits in the SM; route() chooses, and
+// cuts k into slabs where tiles alone would leave SMs idle.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -618,38 +618,71 @@ struct Route {
     int splits;
 };
 
-// Modelled times in microseconds, from B200 timings.  Fused kernel: a block of 32
-// k takes a + b NT per CTA (NT rows of the tile), SMs take whole rounds of CTAs (1%
-// more per round: the power cap).  Pre-pass and 128 x 256 tiles: the planes' bytes,
-// and 0.93 us (BF16X6; 1.16 where the planes' rows do not start on 128 bytes) or 1.0
-// us (TF32X3) per block of 32 k and round.  Both sides measured (fused, planes):
-// BF16X6 1536^3 36, 66; 1800^3 80, 103; 2048^3 99, 95; 2500^3 198, 282; 3000^3 281,
-// 367; 3500^3 534, 464; 4096^3 795, 767.  TF32X3 1536^3 39, 77; 2048^3 99, 107 to
-// 104; 2300^3 166, 202; 3000^3 352, 311.
-static Route route(int path, int m, int n, int k) {
+// The slabs, by a model of the fused kernel in microseconds: a block of 32 k takes
+// a + b NT per CTA (NT rows of the tile), SMs take whole rounds of CTAs (1% more per
+// round: the power cap).
+static int route_slabs(int path, int m, int n, int k) {
     const bool bf = path == SGEMM_B200_PATH_BF16X6;
-    const double sms = 148;
     const int tiles_m = div_up(m, fused::NT_MAX), nt = div_up(div_up(m, tiles_m), 16) * 16;
     const int tiles = tiles_m * div_up(n, fused::TN), chunks = div_up(k, KCHUNK);
     const double block = bf ? 0.235 + 0.0033 * nt : 0.33 + 0.0034 * nt;
-    Route best{true, 1};
+    int best = 1;
     double best_t = 1e300;
     for (int s = 1; s <= 8; s *= 2) {
         if (s > 1 && (div_up(chunks, s) * (s - 1) >= chunks || tiles * s > 148)) break;
-        const double rounds = std::ceil(tiles * s / sms);
+        const double rounds = std::ceil(tiles * s / 148.0);
         const double t = 4.0 + (s > 1 ? 2.5 : 0.0) + rounds * (0.99 + 0.01 * rounds) *
                                                          div_up(chunks, s) * (KCHUNK / 32) * block;
         if (t < best_t * 0.95) {
             best_t = t;
-            best.splits = s;
+            best = s;
         }
     }
-    const double planes = (double(m) + n) * k * (bf ? 10.0 : 12.0) / 4.5e6;
-    const double tiles256 = std::ceil(double(div_up(m, BM)) * div_up(n, BN) / sms);
-    const double t_planes = 10.0 + planes +
-                            tiles256 * div_up(k, 32) * (!bf ? 1.0 : k % 64 == 0 ? 0.93 : 1.16);
-    if (t_planes < best_t) best = Route{false, 1};
     return best;
+}
+
+// Which kernel: both sides modelled, in microseconds, and fitted together to 500 shapes
+// a path of 200 to 10000 rows, columns and k, timed on both on a B200 (8% rms).  On
+// 170 other shapes the pick takes 0.1% (BF16X6) and 0.2% (TF32X3) longer than the
+// faster kernel.  Fused: blocks of 32 k and the epilogue per round of CTAs, 4.4 us
+// for slabs, and copies where the rows of A or B are not whole 16-byte units (here by
+// k and n, so that the choice depends on the sizes alone).  Planes: their bytes, blocks
+// of 32 k, half dearer for BF16X6 where the planes' rows start on odd 16 bytes (a
+// 64-byte row of a box then touches three 32-byte sectors), and an epilogue that
+// without whole 16-byte units stores four bytes at a time.  Ties go to planes.
+// Measured (fused, planes): BF16X6 1800^3 79, 100; 2048^3 96, 91; 2500^3 163, 259;
+// 3072^3 302, 270; 2494 x 1389 x 5754 278, 232; 4096 x 2048 x 10000 1081, 931; TF32X3
+// 2048^3 102, 98; 2304^3 164, 192; 3072^3 337, 303.
+static Route route(int path, int m, int n, int k) {
+    struct Fit {
+        double fixed, slabs, block, block_nt, epilogue, more, copies;            // fused
+        double p_fixed, bytes, p_block, p_odd, p_epilogue, p_scalar, p_more, ties;  // planes
+    };
+    static const Fit fits[2] = {
+        {0.75, 4.4, 0.197, 0.0036, 0.92, 0.017, 0.47,
+         7.7, 1.08, 0.875, 1.29, 6.0, 19.7, 0.046, 1.04},
+        {1.3, 4.7, 0.375, 0.0028, 0.13, 0.020, 0.51,
+         9.0, 1.25, 0.98, 0.98, 3.4, 17.2, 0.065, 1.06}};
+    const bool bf = path == SGEMM_B200_PATH_BF16X6;
+    const Fit& f = fits[bf ? 0 : 1];
+    const int slabs = route_slabs(path, m, n, k);
+    const int tiles_m = div_up(m, fused::NT_MAX), nt = div_up(div_up(m, tiles_m), 16) * 16;
+    const double ctas = double(tiles_m) * div_up(n, fused::TN) * slabs;
+    const double rounds = std::ceil(ctas / 148.0);
+    const double copied = (k % 4 ? double(m) * k : 0.0) + (n % 4 ? double(k) * n : 0.0);
+    const double inside =
+        f.fixed + (slabs > 1 ? f.slabs : 0.0) +
+        rounds * (1.0 + f.more * (rounds - 1.0)) *
+            (div_up(div_up(k, KCHUNK), slabs) * (KCHUNK / 32) * (f.block + f.block_nt * nt) +
+             f.epilogue * nt / 128.0) +
+        (copied > 0 ? 3.0 + f.copies * copied * 8.0 / 4.5e6 : 0.0);
+    const double rounds256 = std::ceil(double(div_up(m, BM)) * div_up(n, BN) / 148.0);
+    const double planes =
+        f.p_fixed + f.bytes * (double(m) + n) * k * (bf ? 10.0 : 12.0) / 4.5e6 +
+        rounds256 * (1.0 + f.p_more * (rounds256 - 1.0)) *
+            (div_up(k, 32) * (div_up(k, 8) % 2 ? f.p_odd : f.p_block) +
+             (n % 4 ? f.p_scalar : f.p_epilogue));
+    return planes < inside * f.ties ? Route{false, 1} : Route{true, slabs};
 }
 
 // Whether split_fused_kernel's TMA boxes can describe the operands.

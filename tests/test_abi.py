@@ -275,3 +275,16 @@ def test_split_queries():
     table = (sg.Problem * 2)(sg.Problem(64, 64, 4096, 4096, 64, 64, 1.0, 0.0, 16, 16, 16),
                              sg.Problem(0, 64, 64, 64, 64, 64, 1.0, 0.0, 16, 16, 16))
     assert sg.grouped_split_query("bf16x6", table) == [True, False]
+
+
+@pytest.mark.parametrize("path,m,n,k,inside", [
+    ("bf16x6", 1624, 2496, 4176, False), ("bf16x6", 2494, 1389, 5754, False),
+    ("bf16x6", 4096, 2048, 10000, False), ("bf16x6", 1648, 2168, 3920, False),
+    ("bf16x6", 2500, 2500, 2500, True), ("bf16x6", 2100, 5932, 5942, True),
+    ("bf16x6", 136, 4096, 4096, True), ("bf16x6", 8192, 8192, 8192, False),
+    ("tf32x3", 2048, 2048, 2048, False), ("tf32x3", 2304, 2304, 2304, True),
+    ("tf32x3", 3072, 3072, 3072, False), ("tf32x3", 24, 4096, 4096, True)])
+def test_split_kernel_is_the_measured_faster_one(path, m, n, k, inside):
+    # each at least 4% faster on this kernel; the first four ran on the other one and
+    # were slower than before there were two
+    assert sg.split_query(path, m, n, k)[0] == inside
