@@ -48,8 +48,12 @@ extern "C" {
 typedef struct sgemm_b200_server sgemm_b200_server;
 
 typedef struct {
-    size_t hbm_budget_bytes;  /* device pool size (launches may hold up to an eighth of it more,
-                                 for operands they prepare) */
+    /* Device pool size.  Beside it, and until the server is destroyed, its launches
+     * hold on the plain path up to an eighth of it for operands they prepare, on the
+     * split paths up to 9.5 MiB per slot for the sums of k slabs (64 KiB per SM), and
+     * on every path the tables of their launches (below 4 MiB per slot for batches of
+     * up to 256 requests). */
+    size_t hbm_budget_bytes;
     int slots;                /* batches that may be in flight at once (streams) */
     int max_batch;            /* most requests in one batch */
     int path;                 /* sgemm_b200_path */

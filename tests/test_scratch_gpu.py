@@ -77,3 +77,23 @@ def test_a_server_gives_its_launch_memory_back(path):
     srv.close()
     _reserved()
     assert sg.pool_usage()[0] == used0
+
+
+@pytest.mark.parametrize("path", ["plain", "bf16x6", "tf32x3"])
+def test_a_server_holds_what_its_header_says_beside_the_budget(path):
+    """A small budget and several slots: operands that a plain batch prepares within an
+    eighth of the budget, the slab sums of a split batch per slot, and tables."""
+    import torch
+
+    _reserved()
+    used0 = sg.pool_usage()[0]
+    budget, slots = 64 << 20, 3
+    srv = sg.Server(budget, slots=slots, max_batch=4, path=path)
+    for seed in range(24):
+        srv.submit(96 + seed, 768, 4096, seed=seed)
+    srv.drain()
+    held = sg.pool_usage()[0] - used0
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    share = budget // 8 if path == "plain" else slots * sms * (64 << 10)
+    assert held <= share + slots * (4 << 20)
+    srv.close()
