@@ -66,13 +66,16 @@ typedef enum {
  * status return.  Each C element is accumulated over k in increasing order
  * with one fused multiply-add per term, then acc *= alpha and
  * C = fmaf(C_old, beta, acc), so results equal the reference kernels' bit for
- * bit on the same inputs.  After one call on the device outside stream
- * capture (which caches the device's properties and the library pool), calls
- * can be captured into a CUDA graph, including ones that prepare operands
- * first: large problems read a transposed copy of A, and unaligned strides are
- * copied to aligned rows (the scratch, 4 m k bytes and the copies', is
- * stream-ordered from the library's pool; without it a call reads its operands
- * in place, with the same result). */
+ * bit on the same inputs.
+ *
+ * Large problems read a transposed copy of A and unaligned strides may be copied to
+ * aligned rows first (sgemm_b200_launches): stream-ordered scratch of the library's,
+ * at most 1 GiB for a transposed A.  Without it a call reads its operands in place,
+ * with the same result.  After one call on the device outside stream capture (which
+ * caches the device's properties), calls can be captured into a CUDA graph.  A
+ * captured call takes no scratch, so its graph has kernel nodes only, except on
+ * unaligned strides from 512^3 multiply-adds on: their copies become memory nodes,
+ * and such a graph cannot be a child graph or have two instantiations at a time. */
 int sgemm_b200(int m, int n, int k,
                const float* alpha,
                const float* A, int lda,
@@ -410,13 +413,15 @@ int sgemm_b200_fill_random(float* X, int rows, int cols, int ld,
                            uint64_t seed, uint32_t tag, int dist,
                            sgemm_b200_stream_t stream);
 
-/* Bytes the library's own stream-ordered memory pool on the current device
- * holds for live allocations (*used_bytes) and keeps reserved from the driver
- * (*reserved_bytes).  The pool backs the scratch the library allocates itself:
- * split workspaces when the caller passes none, operands prepared for a kernel
- * (transposed copies of A, aligned copies; a grouped plan holds its own until it is
- * destroyed), and the host-operand path's staging.  Both are 0 before any call
- * on the device has created the pool; the query never creates it. */
+/* Bytes the library's own stream-ordered memory pools on the current device
+ * hold for live allocations (*used_bytes) and keep reserved from the driver
+ * (*reserved_bytes).  They back the memory the library allocates itself: split
+ * workspaces when the caller passes none, launch tables, the host-operand path's
+ * staging, and operands prepared for a kernel (transposed copies of A, aligned
+ * copies).  Prepared operands come from a pool that keeps at most 4 GiB unused; all
+ * grouped plans of a device together hold at most 4 GiB of them, each its own until
+ * it is destroyed, and read further operands in place.  Both counts are 0 before any
+ * call on the device has created a pool; the query never creates one. */
 int sgemm_b200_pool_usage(size_t* used_bytes, size_t* reserved_bytes);
 
 /* Reads and clears the device-side status word that bounded waits set on

@@ -195,9 +195,10 @@ __device__ __forceinline__ void compute_stage(const uint8_t* __restrict__ As,
     }
 }
 
-// Accumulate one k block with A kept [k][slot]: per k the thread's rows come
-// in two 128-bit loads and its columns in TN / 4, and one packed FMA (fma.rn.f32x2) updates two neighbouring columns
-// of a row with one rounding per element.
+// Accumulate one k block with A kept [k][slot]: per k the thread's rows come in
+// two 128-bit loads (one for 4-row threads) and its columns in TN / V, and one
+// packed FMA (fma.rn.f32x2) updates two neighbouring columns of a row with one
+// rounding per element.
 //
 // Why this layout: with A [row][k], a thread's 128-bit load holds 4 k of one
 // row, so the TM values a k step multiplies sit in registers whose numbers
@@ -280,8 +281,8 @@ __device__ __forceinline__ void load_stage_async4(const Operands& p, uint8_t* As
     }
 }
 
-// Thread (wm, wn, lm, ln) owns rows m0 + WROWS wm + lm + 4i (i < TM) and the
-// float4 column groups n0 + wn*8*TN + 4ln + 32g (g < TN/4).  One row at a
+// Thread (wm, wn, lm, ln) owns rows m0 + WROWS wm + C::row(lm, i) (i < TM) and the
+// column groups of V at n0 + 8 TN wn + V ln + 8 V g (g < TN / V).  One row at a
 // time, each C load right before its store.
 template <class C>
 __device__ __forceinline__ void epilogue_rows(const Operands& p, int m0, int n0, int wm, int wn,
@@ -509,8 +510,8 @@ struct Params {
 };
 
 // Thread (wm, wn, lm, ln) moves its accumulators between registers and an
-// m x n row-major buffer: acc[i][4g+e] is element (m0 + WROWS wm + lm + 4i,
-// n0 + 8 TN wn + 4 ln + 32 g + e).  A sum resumed from the buffer continues
+// m x n row-major buffer: acc[i][V g + e] is element (m0 + WROWS wm + C::row(lm, i),
+// n0 + 8 TN wn + V ln + 8 V g + e).  A sum resumed from the buffer continues
 // the same k-ordered FMA chain, so a product computed over k ranges that
 // start on whole 32-deep k blocks has the bits of the product in one launch.
 template <class C, bool STORE>
