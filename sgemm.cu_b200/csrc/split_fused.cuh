@@ -28,9 +28,10 @@
 // and ~1230 at NT = 128, whose MMAs take 200-770; the rest is the split itself
 // (ALU issue and the chain load, convert, store) and, at NT = 128, shared memory
 // (each element is landed and read, A's planes written and read by every MMA).
-// Measured per call, BF16X6, against pre-pass and 128 x 256 tiles: 24 x 4096 x 4096
-// 18.5 us from 161, 136 x 4096 x 4096 38.6 from 164, 1000^3 17.3 from 68, 512^3 11.5
-// from 33, 64 x 64 x 4096 13.3 from 128; at 2048^3 the two meet (95 us).
+// Measured per call, back to back on three inputs in rotation, BF16X6, against pre-pass
+// and 128 x 256 tiles: 24 x 4096 x 4096 18.6 us from 161, 136 x 4096 x 4096 42.0 from 164,
+// 1000^3 18.2 from 74, 512^3 11.3 from 33, 64 x 64 x 4096 13.4 from 128; at 2048^3 the
+// two meet (96 us here, 91 there).
 #pragma once
 
 namespace fused {
@@ -332,8 +333,8 @@ __device__ __forceinline__ bool convert(const Place& pl, Barriers& b, int nt, in
             reinterpret_cast<const float*>(ra + nt * BK * 4) + 16 * h * TN + q * 32 + lane;
         // B: 16 k of one column, split and stored four words of each plane at a time.
         // All at once needs three times the registers, which the other roles' limit
-        // (96) does not leave: 136 rows BF16X6 41.0 us so, 38.6 in steps, TF32X3 48.7 and
-        // 44.7; a grouped table of 22 314 and 263 (it spilled).
+        // (96) does not leave: 136 rows of one input, B in L2, BF16X6 41.0 us so, 38.6 in
+        // steps, TF32X3 48.7 and 44.7; a grouped table of 22 314 and 263 (it spilled).
         const uint32_t bt = trow + 3 * pl.dcols + group * L::OPCOLS + h * (L::BCOLS / 2);
         constexpr int KS = 16 / T::ESZ;  // k per step
 #pragma unroll
