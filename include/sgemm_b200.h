@@ -194,8 +194,9 @@ int sgemm_b200_split(int path, int m, int n, int k,
 /* What sgemm_b200_split does with a NULL workspace (host-only): *inside is 1 when its
  * kernel splits the operands itself and 0 when it runs on planes from a pre-pass,
  * *slabs the k slabs, *bytes the device memory the call allocates (the planes, or
- * copies of operands whose strides or bases TMA cannot describe).  All 0 when there
- * are no products (m, n or k 0). */
+ * copies of operands whose strides or bases TMA cannot describe), for a C of 16-byte
+ * aligned rows if n is a multiple of 4.  All 0 when there are no products (m, n or k
+ * 0). */
 int sgemm_b200_split_query(int path, int m, int n, int k,
                            const float* A, int lda,
                            const float* B, int ldb,

@@ -641,19 +641,33 @@ static int route_slabs(int path, int m, int n, int k) {
     return best;
 }
 
-// Which kernel: both sides modelled, in microseconds, and fitted together to 500 shapes
-// a path of 200 to 10000 rows, columns and k, timed on both on a B200 (8% rms).  On
-// 170 other shapes the pick takes 0.1% (BF16X6) and 0.2% (TF32X3) longer than the
-// faster kernel.  Fused: blocks of 32 k and the epilogue per round of CTAs, 4.4 us
-// for slabs, and copies where the rows of A or B are not whole 16-byte units (here by
-// k and n, so that the choice depends on the sizes alone).  Planes: their bytes, blocks
-// of 32 k, half dearer for BF16X6 where the planes' rows start on odd 16 bytes (a
-// 64-byte row of a box then touches three 32-byte sectors), and an epilogue that
-// without whole 16-byte units stores four bytes at a time.  Ties go to planes.
+// What a call's strides add to its route: operands the fused kernel needs copied to
+// aligned rows, and C rows that are not whole 16-byte units.
+struct Strides {
+    bool copy_a, copy_b, scalar_c;
+};
+static Strides strides_of(const float* A, int lda, const float* B, int ldb, const float* C,
+                          int ldc) {
+    return Strides{lda % 4 != 0 || reinterpret_cast<uintptr_t>(A) % 16 != 0,
+                   ldb % 4 != 0 || reinterpret_cast<uintptr_t>(B) % 16 != 0,
+                   ldc % 4 != 0 || reinterpret_cast<uintptr_t>(C) % 16 != 0};
+}
+
+// Whether the fused kernel is the faster one: both sides modelled, in microseconds, and
+// fitted together to 500 shapes a path of 200 to 10000 rows, columns and k, timed on
+// both on a B200 (8% rms).  On 170 other shapes the pick takes 0.1% (BF16X6) and 0.2%
+// (TF32X3) longer than the faster kernel.  Fused: blocks of 32 k and the epilogue per
+// round of CTAs, 4.4 us for slabs, and copies of rows that are not whole 16-byte units
+// (a block copies a row per 0.6 us, however short).  Planes: their bytes, blocks of 32
+// k, half dearer for BF16X6 where the planes' rows start on odd 16 bytes (a 64-byte row
+// of a box then touches three 32-byte sectors), and an epilogue that without whole
+// 16-byte units stores four bytes at a time (35% of it is there for one column, too).
+// Ties go to planes.  Of 196 further shapes of 32 to 65536 rows, 1 to 8000 columns and 2
+// to 3000 k one was more than 4% slower than from planes before there were two kernels.
 // Measured (fused, planes): BF16X6 1800^3 79, 100; 2048^3 96, 91; 2500^3 163, 259;
-// 3072^3 302, 270; 2494 x 1389 x 5754 278, 232; 4096 x 2048 x 10000 1081, 931; TF32X3
-// 2048^3 102, 98; 2304^3 164, 192; 3072^3 337, 303.
-static Route route(int path, int m, int n, int k) {
+// 3072^3 302, 270; 2494 x 1389 x 5754 278, 232; 4096 x 2048 x 10000 1081, 931; 65536 x 3
+// x 8 65, 37; TF32X3 2048^3 102, 98; 2304^3 164, 192; 3072^3 337, 303.
+static bool fused_pays(int path, int m, int n, int k, int slabs, Strides st) {
     struct Fit {
         double fixed, slabs, block, block_nt, epilogue, more, copies;            // fused
         double p_fixed, bytes, p_block, p_odd, p_epilogue, p_scalar, p_more, ties;  // planes
@@ -665,24 +679,42 @@ static Route route(int path, int m, int n, int k) {
          9.0, 1.25, 0.98, 0.98, 3.4, 17.2, 0.065, 1.06}};
     const bool bf = path == SGEMM_B200_PATH_BF16X6;
     const Fit& f = fits[bf ? 0 : 1];
-    const int slabs = route_slabs(path, m, n, k);
     const int tiles_m = div_up(m, fused::NT_MAX), nt = div_up(div_up(m, tiles_m), 16) * 16;
     const double ctas = double(tiles_m) * div_up(n, fused::TN) * slabs;
     const double rounds = std::ceil(ctas / 148.0);
-    const double copied = (k % 4 ? double(m) * k : 0.0) + (n % 4 ? double(k) * n : 0.0);
+    const double copied = (st.copy_a ? double(m) * k : 0.0) + (st.copy_b ? double(k) * n : 0.0);
+    const double rows = (st.copy_a ? double(m) : 0.0) + (st.copy_b ? double(k) : 0.0);
+    // (whole chunks of k also below one: what is too much then is a round's fixed cost)
+    const int blocks = div_up(div_up(k, KCHUNK), slabs) * (KCHUNK / 32);
     const double inside =
         f.fixed + (slabs > 1 ? f.slabs : 0.0) +
         rounds * (1.0 + f.more * (rounds - 1.0)) *
-            (div_up(div_up(k, KCHUNK), slabs) * (KCHUNK / 32) * (f.block + f.block_nt * nt) +
-             f.epilogue * nt / 128.0) +
-        (copied > 0 ? 3.0 + f.copies * copied * 8.0 / 4.5e6 : 0.0);
+            (blocks * (f.block + f.block_nt * nt) + f.epilogue * nt / 128.0) +
+        (rows > 0 ? 3.0 + std::max(f.copies * copied * 8.0 / 4.5e6, 0.6 * rows / (8 * 148)) : 0.0);
     const double rounds256 = std::ceil(double(div_up(m, BM)) * div_up(n, BN) / 148.0);
     const double planes =
         f.p_fixed + f.bytes * (double(m) + n) * k * (bf ? 10.0 : 12.0) / 4.5e6 +
-        rounds256 * (1.0 + f.p_more * (rounds256 - 1.0)) *
+        rounds256 * (1.0 + f.p_more * (std::min(rounds256, 8.0) - 1.0)) *
             (div_up(k, 32) * (div_up(k, 8) % 2 ? f.p_odd : f.p_block) +
-             (n % 4 ? f.p_scalar : f.p_epilogue));
-    return planes < inside * f.ties ? Route{false, 1} : Route{true, slabs};
+             (st.scalar_c ? f.p_scalar * (0.35 + 0.65 * n / (BN * double(div_up(n, BN))))
+                          : f.p_epilogue));
+    return planes >= inside * f.ties;
+}
+
+// The route: a function of path and sizes alone, with the strides of matrices without
+// padding.  What depends on it are the slabs, and so the bits.
+static Route route(int path, int m, int n, int k) {
+    const int slabs = route_slabs(path, m, n, k);
+    return fused_pays(path, m, n, k, slabs, Strides{k % 4 != 0, n % 4 != 0, n % 4 != 0})
+               ? Route{true, slabs}
+               : Route{false, 1};
+}
+
+// The kernel of a call with these strides.  In one slab both have the same bits, so
+// padded or odd strides may change the choice; several slabs are the fused kernel's.
+static bool call_is_fused(int path, int m, int n, int k, Route r, Strides st) {
+    return r.splits > 1 || route_slabs(path, m, n, k) > 1 ? r.fused
+                                                          : fused_pays(path, m, n, k, 1, st);
 }
 
 // Whether split_fused_kernel's TMA boxes can describe the operands.
@@ -1594,8 +1626,10 @@ static int split_launch(int path, int m, int n, int k, float alpha, const float*
         return plain_launch(-1, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, stream);
     split::Route r = split::route(path, m, n, k);
     if (whole.m) r.splits = split::route(path, whole.m, whole.n, k).splits;
+    const bool fused = split::call_is_fused(path, m, n, k, r,
+                                            split::strides_of(A, lda, B, ldb, C, ldc));
     // (a workspace the caller passes receives the operand planes)
-    if ((!ws || ws_optional) && r.fused) {
+    if ((!ws || ws_optional) && fused) {
         split::Packed pk = split::packed(m, n, k, A, lda, B, ldb, nullptr);
         if (pk.bytes <= (ws_optional ? ws_bytes : SIZE_MAX)) {
             void* rows = ws;
@@ -1776,9 +1810,10 @@ extern "C" int sgemm_b200_split_query(int path, int m, int n, int k, const float
     *bytes = 0;
     if (m == 0 || n == 0 || k == 0) return SGEMM_B200_OK;
     const sgb::split::Route r = sgb::split::route(path, m, n, k);
-    *inside = r.fused;
+    sgb::split::Strides st = sgb::split::strides_of(A, lda, B, ldb, nullptr, n);
+    *inside = sgb::split::call_is_fused(path, m, n, k, r, st);
     *slabs = r.splits;
-    *bytes = r.fused ? sgb::split::packed(m, n, k, A, lda, B, ldb, nullptr).bytes
+    *bytes = *inside ? sgb::split::packed(m, n, k, A, lda, B, ldb, nullptr).bytes
                      : sgemm_b200_split_workspace_size(path, m, n, k);
     return SGEMM_B200_OK;
 }

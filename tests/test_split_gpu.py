@@ -288,3 +288,19 @@ def test_split_host_blocks_keep_the_whole_problems_slabs(path):
                   0.5, path=path, plan=(128, [128, 384]))
     torch.cuda.synchronize()
     assert np.array_equal(hC.numpy(), want)
+
+
+@pytest.mark.parametrize("path", PATHS)
+@pytest.mark.parametrize("m,n,k", [(2139, 1560, 54), (8192, 24, 16), (4381, 1380, 68),
+                                   (700, 701, 255)])
+def test_split_kernel_may_depend_on_strides_but_not_the_bits(path, m, n, k):
+    """In one k slab the strides choose between the two kernels (short rows are dear to
+    copy): aligned rows, odd rows of A and B, odd rows of C, the same bits."""
+    A = oracle.fill(m, k, 19, 1, 0)
+    B = oracle.fill(k, n, 19, 2, 0)
+    C = oracle.fill(m, n, 19, 3, 0)
+    want = _run(path, A, B, C, 1.5, 0.5, ws=True)
+    for lds in ((None, None, None), ((k + 7) // 4 * 4, (n + 7) // 4 * 4, (n + 7) // 4 * 4),
+                (k | 1, n | 1, None), (None, None, n | 1)):
+        got = _run(path, A, B, C, 1.5, 0.5, ws=False, lds=lds)
+        assert np.array_equal(got.view(np.uint32), want.view(np.uint32)), lds
