@@ -226,7 +226,8 @@ def test_split_workspace_is_the_planes_size(path, planes, esz):
 
 
 @pytest.mark.parametrize("m,n,k", [(36912, 48, 36), (45212, 192, 4), (46812, 36, 56),
-                                   (58936, 64, 15), (57817, 18, 55), (64, 65536, 17)])
+                                   (58936, 64, 15), (57817, 18, 55), (64, 65536, 17),
+                                   (1940, 3645, 16), (521, 9319, 11)])
 def test_short_unaligned_rows_are_read_in_place(m, n, k):
     # copies run at a row per 0.6 us and block: many short rows below 512^3 of work are
     # up to 2.7 times faster in place
@@ -288,3 +289,10 @@ def test_split_kernel_is_the_measured_faster_one(path, m, n, k, inside):
     # each at least 4% faster on this kernel; the first four ran on the other one and
     # were slower than before there were two
     assert sg.split_query(path, m, n, k)[0] == inside
+
+
+def test_one_block_of_k_steps_is_read_in_place():
+    # odd rows of A alone, which are few and cheap to copy, but nothing is gained by it
+    l = sg.lib()
+    assert l.sgemm_b200_packs(64, 65536, 17, 16, 17, 16, 65536) == 0
+    assert l.sgemm_b200_packs(64, 65536, 33, 16, 33, 16, 65536) == 1
