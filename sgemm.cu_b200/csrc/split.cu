@@ -616,6 +616,7 @@ static int launch(int m, int n, int k, float alpha, const float* A, int lda, con
 struct Route {
     bool fused;
     int splits;
+    int slabs;  // that the fused kernel would take
 };
 
 // The slabs, by a model of the fused kernel in microseconds: a block of 32 k takes
@@ -703,18 +704,20 @@ static bool fused_pays(int path, int m, int n, int k, int slabs, Strides st) {
 
 // The route: a function of path and sizes alone, with the strides of matrices without
 // padding.  What depends on it are the slabs, and so the bits.
+static Strides dense(int n, int k) { return Strides{k % 4 != 0, n % 4 != 0, n % 4 != 0}; }
 static Route route(int path, int m, int n, int k) {
     const int slabs = route_slabs(path, m, n, k);
-    return fused_pays(path, m, n, k, slabs, Strides{k % 4 != 0, n % 4 != 0, n % 4 != 0})
-               ? Route{true, slabs}
-               : Route{false, 1};
+    return fused_pays(path, m, n, k, slabs, dense(n, k)) ? Route{true, slabs, slabs}
+                                                         : Route{false, 1, slabs};
 }
 
 // The kernel of a call with these strides.  In one slab both have the same bits, so
 // padded or odd strides may change the choice; several slabs are the fused kernel's.
 static bool call_is_fused(int path, int m, int n, int k, Route r, Strides st) {
-    return r.splits > 1 || route_slabs(path, m, n, k) > 1 ? r.fused
-                                                          : fused_pays(path, m, n, k, 1, st);
+    const Strides d = dense(n, k);
+    const bool as_dense =
+        st.copy_a == d.copy_a && st.copy_b == d.copy_b && st.scalar_c == d.scalar_c;
+    return r.splits > 1 || r.slabs > 1 || as_dense ? r.fused : fused_pays(path, m, n, k, 1, st);
 }
 
 // Whether split_fused_kernel's TMA boxes can describe the operands.
