@@ -133,18 +133,19 @@ struct Barriers {
     volatile int gone;  // a wait has expired
 };
 
-// A split warp's wait.  A lane whose wait expires stays with its warp, which goes on
-// (in bounds, on what it finds) to the chunk's vote on `gone` (convert); waits that
-// come before that no longer last.  A vote per wait instead costs 1-2% of a call.
-__device__ __forceinline__ void wait_or_gone(Barriers& b, uint64_t* bar, uint32_t parity) {
-    if (mbar_try_wait(bar, parity)) return;
+// A split warp's wait.  A lane whose wait expires (false) stays with its warp, which
+// goes on (in bounds, on what it finds) to the chunk's vote on `gone` (convert); waits
+// that come before that no longer last.  A vote per wait instead costs 1-2% of a call.
+__device__ __forceinline__ bool wait_or_gone(Barriers& b, uint64_t* bar, uint32_t parity) {
+    if (mbar_try_wait(bar, parity)) return true;
     const uint64_t t0 = globaltimer_ns();
     while (!mbar_try_wait(bar, parity)) {
         if (b.gone || globaltimer_ns() - t0 > kWaitLimitNs) {
             b.gone = 1;
-            return;
+            return false;
         }
     }
+    return true;
 }
 
 // Where a CTA keeps things: operand buffers, landing stages (A [nt][32 k], then
@@ -235,12 +236,15 @@ __device__ __forceinline__ bool multiply(const Place& pl, Barriers& b, int nt, i
                                         : sw128_kmajor_desc(smem_u32(pl.ops));
     const uint32_t plane16 = static_cast<uint32_t>(nt * L::ROW) >> 4;
     const uint32_t d2 = pl.tmem + 2 * pl.dcols;
-    bool ok = true;  // of this lane's waits; the warp votes before it goes on
-    if (slab > 0) ok = mbar_wait(&b.d2_empty, (slab - 1) & 1);  // D2 of the slab before is read
+    if (slab > 0) {  // D2 of the slab before has been read
+        const bool ok = mbar_wait(&b.d2_empty, (slab - 1) & 1);
+        if (!__all_sync(0xffffffffu, ok)) return false;
+        tc_fence_after();
+    }
     for (int i = 0; i < nb; ++i, ++g) {
         const int s = g % G;
         const bool start = i % CHUNK_BLOCKS == 0;  // D1 restarts
-        if (ok) ok = mbar_wait(&b.op_full[s], (g / G) & 1);
+        bool ok = mbar_wait(&b.op_full[s], (g / G) & 1);
         if (ok && start && cg >= 2) ok = mbar_wait(&b.d1_empty[cg & 1], ((cg >> 1) - 1) & 1);
         if (!__all_sync(0xffffffffu, ok)) return false;
         tc_fence_after();
@@ -314,8 +318,9 @@ __device__ __forceinline__ bool convert(const Place& pl, Barriers& b, int nt, in
         }
     };
     auto drain_chunk = [&] {
-        wait_or_gone(b, &b.d1_full[cg & 1], (cg >> 1) & 1);
-        if (!__all_sync(0xffffffffu, !b.gone)) return false;
+        const int gone = b.gone;  // of the waits before; read behind this one it would take 0.5%
+        const bool ok = wait_or_gone(b, &b.d1_full[cg & 1], (cg >> 1) & 1) && !gone;
+        if (!__all_sync(0xffffffffu, ok)) return false;
         tc_fence_after();
         drain((cg & 1) * pl.dcols);
         tc_fence_before();

@@ -79,7 +79,7 @@ def test_fused_split_producer_arms_no_barrier_twice():
     wait = produce.index("raw_empty")
     assert re.match(r"raw_empty[^;]*\|\| b\.gone\) return false;", produce[wait:])
     assert wait < produce.index("mbar_arrive_expect_tx")
-    assert "b.gone = 1" in _body(code, r"void wait_or_gone\(")
+    assert "b.gone = 1" in _body(code, r"bool wait_or_gone\(")
 
 
 @pytest.mark.parametrize("kernel", ["split_gemm_kernel", "split_grouped_kernel"])
